@@ -17,6 +17,7 @@
 #include "gpumpi.h"
 #include "hostjob.h"
 #include "rt.cuh"
+#include "spread.cuh"
 
 extern __device__ MPI_Op_impl gm_builtin_ops[GPUMPI_NUM_BUILTIN_OPS];
 
@@ -183,6 +184,12 @@ struct gpumpi_plan_s {
     int independent = 0;                   // calls touch disjoint memory and include no barrier
     int sync_mode = 0;                     // 0 automatic, 1 flag rounds for every call
     std::vector<int> plain_op;             // collective of each plain launch
+    // spread form of the launch-ordered launches (spread.cuh); ntiles 0 in a
+    // launch it does not cover
+    bool batch_spread = false;
+    SpreadArgs batch_tiles;
+    std::vector<char> plain_spread;
+    std::vector<SpreadArgs> plain_tiles;
 };
 
 namespace {
@@ -213,6 +220,9 @@ int api_job() {
     // in shared memory: prefer the largest shared-memory carve-out
     CK(cudaFuncSetAttribute((const void*)gpumpi_plan_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                             (int)cudaSharedmemCarveoutMaxShared));
+    CK(cudaFuncSetAttribute((const void*)gpumpi_spread_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                            (int)cudaSharedmemCarveoutMaxShared));
+    CK(cudaFuncSetAttribute((const void*)gpumpi_spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM));
     Job hj;
     memset(&hj, 0, sizeof(hj));
     char* mem = nullptr;
@@ -327,6 +337,15 @@ int launch(const void* kern, int grid, int threads, size_t smem, PlanArgs* args,
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     CK(cudaLaunchKernelExC(&cfg, kern, params));
+    g_launches++;
+    return GPUMPI_OK;
+}
+
+// Tiles are independent: any number of blocks, no cooperative launch.
+int launch_spread(SpreadArgs* args, cudaStream_t st) {
+    void* params[] = {args};
+    const u32 grid = std::max(1u, std::min(args->ntiles, 1u << 30));
+    CK(cudaLaunchKernel((const void*)gpumpi_spread_kernel, dim3(grid), dim3(SP_T), params, SP_SMEM, st));
     g_launches++;
     return GPUMPI_OK;
 }
@@ -446,8 +465,33 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     size_t off_pc = (off_pp + sizeof(int) * 2 * ndesc + 15) & ~(size_t)15;
     size_t off_ptr = off_pc + sizeof(DevComm) * ndesc;
     size_t off_pubt = (off_ptr + sizeof(void*) * ptrs + 63) & ~(size_t)63;   // Pub tables, one entry per rank
-    size_t total = off_pubt + sizeof(Pub) * (ptrs / 2) + 16;
+    const size_t off_sp = off_pubt + sizeof(Pub) * (ptrs / 2);   // SpreadCalls, then their address tables
+    // the spread form: the whole batched launch, or each plain launch it covers
     gpumpi_plan_s* p = new gpumpi_plan_s();
+    p->independent = plan_independent(descs, ndesc) ? 1 : 0;
+    std::vector<SpreadBuilder> spread(batched ? 1 : ndesc);
+    p->plain_spread.assign(ndesc, 0);
+    p->plain_tiles.resize(ndesc);
+    auto covers = [&](int i) { return SpreadBuilder::covers(descs[i], descs[i].comm->n, esize_of(descs[i].dtype)); };
+    auto traffic = [&](int i) { return SpreadBuilder::traffic(descs[i], descs[i].comm->n, esize_of(descs[i].dtype)); };
+    if (batched) {
+        double bytes = 0;
+        p->batch_spread = p->independent != 0;
+        for (int i = 0; i < ndesc && p->batch_spread; i++) {
+            p->batch_spread = covers(i);
+            bytes += traffic(i);
+        }
+        for (int i = 0; i < ndesc && p->batch_spread; i++)
+            spread[0].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), bytes);
+    } else {
+        for (int k = 0; k < ndesc; k++) {
+            const int i = order[k];
+            p->plain_spread[k] = covers(i);
+            if (p->plain_spread[k]) spread[k].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), traffic(i));
+        }
+    }
+    size_t total = off_sp;
+    for (const SpreadBuilder& b : spread) total += sizeof(SpreadCall) * b.calls.size() + sizeof(void*) * b.ptrs.size() + 64;
     CK(cudaMalloc(&p->base, total));
     char* base = p->base;
     std::vector<char> h(total, 0);
@@ -507,6 +551,24 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
         pp[2 * k + 1] = 1;
         pc[k] = comms[hd[k].comm]->hcomm;
     }
+    size_t at = off_sp;
+    for (size_t k = 0; k < spread.size(); k++) {
+        SpreadBuilder& b = spread[k];
+        SpreadArgs& a = batched ? p->batch_tiles : p->plain_tiles[k];
+        memset(&a, 0, sizeof(a));
+        const size_t calls_at = (at + 63) & ~(size_t)63;
+        at = calls_at + sizeof(SpreadCall) * b.calls.size();
+        a.ntiles = b.finish(base + at);
+        if (!b.calls.empty()) {
+            memcpy(h.data() + calls_at, b.calls.data(), sizeof(SpreadCall) * b.calls.size());
+            memcpy(h.data() + at, b.ptrs.data(), sizeof(void*) * b.ptrs.size());
+            a.one = b.calls[0];
+        }
+        at += sizeof(void*) * b.ptrs.size();
+        a.calls = (const SpreadCall*)(base + calls_at);
+        a.ncalls = (u32)b.calls.size();
+        a.job = g_api.djob;
+    }
     CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));
     p->ndesc = ndesc;
     p->ncomm = ncomm;
@@ -520,7 +582,6 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     p->batch_args.slot_comm = (const int*)(base + off_sc);
     p->batch_args.slot_rank = (const int*)(base + off_sr);
     p->batch_args.comms = (const DevComm*)(base + off_cm);
-    p->independent = plan_independent(descs, ndesc) ? 1 : 0;
     p->batch_args.ordered = p->independent;
     p->batch_args.pad = 0;
     p->plain_args.resize(ndesc);
@@ -572,9 +633,14 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
 
 static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
     const void* k = (const void*)gpumpi_plan_kernel;
-    if (p->batched) return launch(k, p->total_slots, p->threads, p->smem, &p->batch_args, st);
+    if (p->batched) {
+        if (p->batch_spread && p->batch_args.ordered) return launch_spread(&p->batch_tiles, st);
+        return launch(k, p->total_slots, p->threads, p->smem, &p->batch_args, st);
+    }
     for (int i = 0; i < p->ndesc; i++) {
-        int rc = launch(k, p->plain_grid[i], p->plain_threads[i], p->plain_smem[i], &p->plain_args[i], st);
+        int rc = p->plain_spread[i] && p->plain_args[i].ordered
+                     ? launch_spread(&p->plain_tiles[i], st)
+                     : launch(k, p->plain_grid[i], p->plain_threads[i], p->plain_smem[i], &p->plain_args[i], st);
         if (rc) return rc;
     }
     return GPUMPI_OK;

@@ -11,6 +11,7 @@
 // `a != b` on 0/1 inputs.  Complex products use round-to-nearest intrinsics
 // so that no multiply-add is contracted and results match a host fold bit
 // for bit.
+#include "redop.cuh"
 #include "rt.cuh"
 
 #define GPUMPI_OP_OBJ_F(name, idx) {idx, 1, nullptr}
@@ -138,21 +139,12 @@ __device__ int op_check(MPI_Op op, MPI_Datatype t) {
 }
 
 // ---------------------------------------------------------------- operators
-template <class T> struct OMax { __device__ static T f(T a, T b) { return a > b ? a : b; } };
-template <class T> struct OMin { __device__ static T f(T a, T b) { return a > b ? b : a; } };
-template <class T> struct OSum { __device__ static T f(T a, T b) { return (T)(a + b); } };
-template <class T> struct OProd { __device__ static T f(T a, T b) { return (T)(a * b); } };
 template <class T> struct OLAnd { __device__ static T f(T a, T b) { return (T)(a && b); } };
 template <class T> struct OLOr { __device__ static T f(T a, T b) { return (T)(a || b); } };
 template <class T> struct OLXor { __device__ static T f(T a, T b) { return (T)((!a) != (!b)); } };
 template <class T> struct OBAnd { __device__ static T f(T a, T b) { return (T)(a & b); } };
 template <class T> struct OBOr { __device__ static T f(T a, T b) { return (T)(a | b); } };
 template <class T> struct OBXor { __device__ static T f(T a, T b) { return (T)(a ^ b); } };
-
-template <> struct OSum<float> { __device__ static float f(float a, float b) { return __fadd_rn(a, b); } };
-template <> struct OSum<double> { __device__ static double f(double a, double b) { return __dadd_rn(a, b); } };
-template <> struct OProd<float> { __device__ static float f(float a, float b) { return __fmul_rn(a, b); } };
-template <> struct OProd<double> { __device__ static double f(double a, double b) { return __dmul_rn(a, b); } };
 
 template <> struct OSum<gpumpi_cfloat> {
     __device__ static gpumpi_cfloat f(gpumpi_cfloat a, gpumpi_cfloat b) {
@@ -209,15 +201,6 @@ static __device__ void fold_scalar(T* out, const Pub* pub, int nin, u64 in_off, 
         for (int q = 1; q < nin; q++) acc = O::f(ldcg(in_ptr<T>(pub, q, in_off, ptab) + i), acc);
         out[i - lo] = acc;
     }
-}
-
-template <class T, class O>
-static __device__ __forceinline__ void combine(uint4& acc, const uint4& x) {
-    constexpr int V = 16 / sizeof(T);
-    T* a = reinterpret_cast<T*>(&acc);
-    const T* xe = reinterpret_cast<const T*>(&x);
-#pragma unroll
-    for (int e = 0; e < V; e++) a[e] = O::f(xe[e], a[e]);
 }
 
 // 16-byte vector path for 4- and 8-byte element types when every input and

@@ -1,0 +1,703 @@
+// Kernel and tile lists of the spread form (spread.cuh).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "redop.cuh"
+#include "spread.cuh"
+
+namespace gm {
+
+// Element types of a fold; sums and products of unsigned types use the signed
+// type's code (the same bits).
+enum FoldType : int { FT_I8, FT_U8, FT_I16, FT_U16, FT_I32, FT_U32, FT_I64, FT_U64, FT_F32, FT_F64, FT_NONE };
+
+// ------------------------------------------------------------------ device
+
+// Entry i of a table of addresses (constant while a launch runs).
+template <class P>
+static __device__ __forceinline__ P ld_ptr(P const* t, u32 i) {
+    return reinterpret_cast<P>(__ldg(reinterpret_cast<const u64*>(t) + i));
+}
+
+template <class V>
+static __device__ __forceinline__ V ld_unit(const char* p) {
+    return __ldcg(reinterpret_cast<const V*>(p));
+}
+
+// Asynchronous copy of B bytes to shared memory; 16-byte copies bypass L1.
+template <int B>
+static __device__ __forceinline__ void cp_async(u32 dst, const char* src) {
+    if constexpr (B == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(B) : "memory");
+}
+static __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+static __device__ __forceinline__ void cp_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <class V>
+static __device__ __noinline__ void fan_tile(const SpreadCall& c, u32 tile) {
+    constexpr int U = 8;
+    const u32 pieces = (u32)((c.nu + c.per - 1) / c.per);
+    const u32 piece = tile % pieces;
+    const u32 rest = tile / pieces;
+    const u32 q = rest % c.nsrc, r0 = rest / c.nsrc * c.group;
+    const u32 r1 = min(r0 + c.group, c.ndst);
+    const u64 o0 = (u64)piece * c.per;
+    const u64 o1 = min(o0 + c.per, c.nu);
+    const char* s = ld_ptr(c.src, q) + c.rs * r0;
+    const u64 row = (u64)q * c.nu * sizeof(V);
+    for (u64 o = o0 + threadIdx.x; o < o1; o += U * SP_T) {
+        V v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (o + u * SP_T < o1) v[u] = ld_unit<V>(s + (o + u * SP_T) * sizeof(V));
+        for (u32 r = r0; r < r1; r++) {
+            V* d = reinterpret_cast<V*>(ld_ptr(c.dst, r) + row) + o;
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (o + u * SP_T < o1) d[u * SP_T] = v[u];
+        }
+    }
+}
+
+template <class V>
+static __device__ __noinline__ void copy_tile(const SpreadCall& c, u32 tile) {
+    constexpr int U = 4;
+    const u64 total = (u64)c.ndst * c.nsrc * c.nu;
+    const u64 k1 = min((u64)(tile + 1) * c.per, total);
+    u64 k = (u64)tile * c.per + threadIdx.x;
+    // unit k: row r, block q, unit o of the block; all three advance by SP_T units
+    const u32 nu = (u32)c.nu;
+    const u32 d_o = SP_T % nu, d_q = SP_T / nu % c.nsrc, d_r = SP_T / nu / c.nsrc;
+    const u64 blk = k / nu;
+    u32 o = (u32)(k - blk * nu), r = (u32)(blk / c.nsrc), q = (u32)(blk - (u64)r * c.nsrc);
+    while (k < k1) {
+        V v[U];
+        V* d[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (k < k1) {
+                v[u] = ld_unit<V>(ld_ptr(c.src, q) + c.rs * r + (u64)o * sizeof(V));
+                d[u] = reinterpret_cast<V*>(ld_ptr(c.dst, r)) + ((u64)q * nu + o);
+            } else {
+                d[u] = nullptr;
+            }
+            k += SP_T;
+            o += d_o;
+            q += d_q;
+            r += d_r;
+            if (o >= nu) {
+                o -= nu;
+                q++;
+            }
+            if (q >= c.nsrc) {
+                q -= c.nsrc;
+                r++;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (d[u]) *d[u] = v[u];
+    }
+}
+
+// Loads of a gather tile: the tile's n units of V of every source, one after
+// another in g, SP_T units at a time.
+template <class V>
+static __device__ __forceinline__ void gather_load(const SpreadCall& c, u64 at, u32 n, char* g) {
+    const u32 total = n * c.nsrc;
+    const u32 d_q = SP_T / n, d_i = SP_T % n;
+    u32 q = threadIdx.x / n, i = threadIdx.x % n;
+    const u32 g_s = (u32)__cvta_generic_to_shared(g);
+    for (u32 k = threadIdx.x; k < total; k += SP_T) {
+        const char* p = ld_ptr(c.src, q) + at + (u64)i * sizeof(V);
+        if constexpr (sizeof(V) >= 4) cp_async<sizeof(V)>(g_s + k * (u32)sizeof(V), p);
+        else reinterpret_cast<V*>(g)[k] = ld_unit<V>(p);
+        q += d_q;
+        i += d_i;
+        if (i >= n) {
+            i -= n;
+            q++;
+        }
+    }
+}
+
+// Stores of a gather tile: the n units of V at `res` to every destination.
+template <class V>
+static __device__ __forceinline__ void gather_store(const SpreadCall& c, u64 at, u32 n, const char* res) {
+    const u32 total = n * c.ndst;
+    const u32 d_r = SP_T / n, d_i = SP_T % n;
+    u32 r = threadIdx.x / n, i = threadIdx.x % n;
+    for (u32 k = threadIdx.x; k < total; k += SP_T) {
+        reinterpret_cast<V*>(ld_ptr(c.dst, r) + at)[i] = reinterpret_cast<const V*>(res)[i];
+        r += d_r;
+        i += d_i;
+        if (i >= n) {
+            i -= n;
+            r++;
+        }
+    }
+}
+
+template <class T, class O>
+static __device__ void gather_tile(const SpreadCall& c, u32 tile, char* ring) {
+    const u64 lo = (u64)tile * c.per;
+    const u32 m = (u32)min((u64)c.per, c.nu - lo);
+    const u64 at = c.off + lo * sizeof(T);
+    if (c.ub == 16) gather_load<uint4>(c, at, m * (u32)sizeof(T) / 16, ring);
+    else gather_load<T>(c, at, m, ring);
+    cp_commit();
+    cp_wait<0>();
+    __syncthreads();
+    const T* g = reinterpret_cast<const T*>(ring);
+    // the results replace the first source's elements
+    T* res = reinterpret_cast<T*>(ring);
+    for (u32 i = threadIdx.x; i < m; i += SP_T) {
+        T acc = g[i];
+        u32 q = 1;
+        for (; q + 8 <= c.nsrc; q += 8) {
+            T x[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) x[k] = g[(q + k) * m + i];
+#pragma unroll
+            for (int k = 0; k < 8; k++) acc = O::f(x[k], acc);
+        }
+        for (; q < c.nsrc; q++) acc = O::f(g[q * m + i], acc);
+        res[i] = acc;
+    }
+    __syncthreads();
+    if (c.ub == 16) gather_store<uint4>(c, at, m * (u32)sizeof(T) / 16, ring);
+    else gather_store<T>(c, at, m, ring);
+}
+
+// Every thread copies its own vectors into its own ring slots and reads only
+// those, so the pipeline needs no barrier: cp.async groups complete in order
+// and wait_group tells the thread when its oldest group has arrived.  GL loads
+// make a group; the ring holds SP_RING bytes per block whatever the vector.
+template <class T, class O, class V>
+static __device__ void stream_tile(const SpreadCall& c, u32 tile, char* ring, const char* const* st, char* const* dt) {
+    constexpr int B = sizeof(V);
+    constexpr int GL = 4;
+    constexpr int NG = (int)(SP_RING / (SP_T * B)) / GL;
+    static_assert(NG >= 2, "ring");
+    const u64 nvec = c.nu * sizeof(T) / B;
+    const u64 v0 = (u64)tile * c.per * SP_T + threadIdx.x;
+    const u32 rows = (u32)min((u64)c.per, (nvec - (u64)tile * c.per * SP_T + SP_T - 1) / SP_T);
+    const u32 K = rows * c.nsrc;
+    const u32 ng = (K + GL - 1) / GL;
+    const u32 mine = (u32)__cvta_generic_to_shared(ring) + threadIdx.x * B;
+    const V* slot = reinterpret_cast<const V*>(ring) + threadIdx.x;
+    u64 iv = v0, cv = v0;
+    u32 istep = 0, iq = 0, q = 0, ig = 0, cg = 0;
+    auto issue = [&]() {
+#pragma unroll
+        for (int g = 0; g < GL; g++) {
+            if (istep < K && iv < nvec) cp_async<B>(mine + (ig * GL + g) * (SP_T * B), st[iq] + c.off + iv * B);
+            istep++;
+            if (++iq == c.nsrc) {
+                iq = 0;
+                iv += SP_T;
+            }
+        }
+        cp_commit();
+        if (++ig == NG) ig = 0;
+    };
+#pragma unroll 1
+    for (int g = 0; g < NG - 1; g++) issue();
+    V acc{};
+    for (u32 k = 0; k < ng; k++) {
+        issue();   // into the slots that step k - 1 emptied
+        cp_wait<NG - 1>();
+#pragma unroll
+        for (int g = 0; g < GL; g++) {
+            if (k * GL + g < K) {
+                const V x = slot[(cg * GL + g) * SP_T];
+                if (q == 0) acc = x;
+                else combine<T, O>(acc, x);
+                if (++q == c.nsrc) {
+                    if (cv < nvec)
+                        for (u32 r = 0; r < c.ndst; r++) *reinterpret_cast<V*>(dt[r] + c.off + cv * B) = acc;
+                    q = 0;
+                    cv += SP_T;
+                }
+            }
+        }
+        if (++cg == NG) cg = 0;
+    }
+    cp_wait<0>();
+}
+
+template <class T, class O>
+static __device__ __noinline__ void fold_tile(const SpreadCall& c, u32 tile, char* smem) {
+    if (c.kind == SP_GATHER) {
+        gather_tile<T, O>(c, tile, smem);
+        return;
+    }
+    const char* const* st = c.src;
+    char* const* dt = c.dst;
+    if (c.nsrc <= SP_TAB) {
+        const char** ts = reinterpret_cast<const char**>(smem + SP_RING);
+        char** td = reinterpret_cast<char**>(smem + SP_RING) + SP_TAB;
+        for (u32 q = threadIdx.x; q < c.nsrc; q += SP_T) ts[q] = ld_ptr(c.src, q);
+        for (u32 r = threadIdx.x; r < c.ndst; r += SP_T) td[r] = ld_ptr(c.dst, r);
+        __syncthreads();
+        st = ts;
+        dt = td;
+    }
+    if (c.ub == 16) stream_tile<T, O, uint4>(c, tile, smem, st, dt);
+    else if constexpr (sizeof(T) >= 4) stream_tile<T, O, T>(c, tile, smem, st, dt);
+}
+
+// ---- bulk copies into the ring
+//
+// Every warp has its own part of the ring, cut into stages, and its own
+// barriers: one lane loads a row into a stage by a bulk copy, the warp waits
+// for it, uses it, and loads the stage again.  No block barrier is on the way.
+struct Ring {
+    u64 full[SP_WARPS][SP_MAX_STAGES];
+    u32 failed;     // a wait ran out: the block's later waits return at once
+};
+
+static __device__ __forceinline__ u32 smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
+
+static __device__ __forceinline__ u32 bar_done(u32 bar, u32 parity) {
+    u32 done;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done;
+}
+
+// Wait for the loads of the warp's stage; bit `stage` of phases is the parity
+// to wait for.  After the job's time limit the launch is marked failed.
+static __device__ __forceinline__ void ring_wait(Ring& ring, u32 stage, u32& phases, Job* job) {
+    const u32 bar = smem_addr(&ring.full[threadIdx.x >> 5][stage]);
+    const u32 parity = (phases >> stage) & 1;
+    phases ^= 1u << stage;
+    if (bar_done(bar, parity)) return;
+    const u64 t0 = gtime();
+    while (!bar_done(bar, parity)) {
+        if (*(volatile u32*)&ring.failed) return;
+        if (gtime() - t0 > job->timeout_ns) {
+            job_fail(job, (int)blockIdx.x, GPUMPI_ERR_TIMEOUT, "a bulk load did not complete");
+            *(volatile u32*)&ring.failed = 1;
+        }
+    }
+}
+
+// Load `bytes` (a multiple of 16, may be 0) from src to dst for the warp's stage.
+static __device__ __forceinline__ void ring_load(Ring& ring, u32 stage, char* dst, const char* src, u32 bytes) {
+    const u32 bar = smem_addr(&ring.full[threadIdx.x >> 5][stage]);
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    if (bytes)
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// ---- SP_MOVE
+
+// A row in the ring.
+struct MoveRow {
+    u64 dst;           // address (one destination) or offset in every destination
+    const char* src;   // first byte of the row
+    u32 at, len;       // bytes in shared memory: the first one's place, how many
+    u32 head, tail;    // bytes before and after them that were not loaded (a row at its buffer's start or end)
+    u32 r0, pad;
+};
+static_assert(sizeof(MoveRow) * SP_WARPS * SP_MAX_STAGES <= 2 * SP_TAB * sizeof(char*), "row table");
+
+template <class V>
+static __device__ __forceinline__ void move_units(char* d, const char* s, u32 n, u32 lane) {
+    V* dv = reinterpret_cast<V*>(d);
+    const V* sv = reinterpret_cast<const V*>(s);
+    u32 i = lane;
+    for (; i + 96 < n; i += 128) {
+        const V a = sv[i], b = sv[i + 32], e = sv[i + 64], f = sv[i + 96];
+        dv[i] = a;
+        dv[i + 32] = b;
+        dv[i + 64] = e;
+        dv[i + 96] = f;
+    }
+    for (; i < n; i += 32) dv[i] = sv[i];
+}
+
+// n bytes from shared memory s to d by one warp: the widest unit that both
+// alignments share, bytes up to the first and after the last whole one; with
+// no common alignment of 4, destination words put together from two source words.
+static __device__ __forceinline__ void move_row(char* d, const char* s, u32 n, u32 lane) {
+    const u32 delta = ((u32)(uintptr_t)d - smem_addr(s)) & 15;
+    const u32 unit = delta == 0 ? 16 : delta == 8 ? 8 : 4;
+    u32 h = (0u - (u32)(uintptr_t)d) & (unit - 1);
+    if (h > n) h = n;
+    const u32 nw = (n - h) / unit;
+    if (unit == 16) {
+        move_units<uint4>(d + h, s + h, nw, lane);
+    } else if (unit == 8) {
+        move_units<uint2>(d + h, s + h, nw, lane);
+    } else if ((delta & 3) == 0) {
+        move_units<u32>(d + h, s + h, nw, lane);
+    } else {
+        const u32* w = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(s + h) & ~(uintptr_t)3);
+        const u32 sh = (smem_addr(s + h) & 3) * 8;
+        for (u32 i = lane; i < nw; i += 32) reinterpret_cast<u32*>(d + h)[i] = __funnelshift_r(w[i], w[i + 1], sh);
+    }
+    // at most 15 bytes on either side
+    const u32 done = h + nw * unit;
+    if (lane < h) d[lane] = s[lane];
+    if (done + lane < n) d[done + lane] = s[done + lane];
+}
+
+static __device__ __noinline__ void move_tile(const SpreadCall& c, u32 tile, char* smem, Ring& ring, u32& phases,
+                                              Job* job) {
+    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const u32 pieces = (u32)((c.nu + c.per - 1) / c.per);
+    const u32 all = pieces * c.nsrc * ((c.ndst + c.group - 1) / c.group);
+    const u32 row0 = tile * c.rows, row1 = min(row0 + c.rows, all);
+    const u32 n = row1 - row0 > warp ? (row1 - row0 - warp + SP_WARPS - 1) / SP_WARPS : 0;   // this warp's rows
+    const u32 pitch = c.per + 32;
+    const u64 extent = c.rs ? c.rs * c.ndst : c.nu;   // bytes of a source buffer
+    char* part = smem + warp * SP_PART;
+    MoveRow* info = reinterpret_cast<MoveRow*>(smem + SP_RING) + warp * SP_MAX_STAGES;
+    // lane i of 32 prepares rows i, 32 + i, ... of the warp and loads them when their turn comes
+    MoveRow m;
+    const char* from = nullptr;
+    u32 bytes = 0;
+    auto prepare = [&](u32 i) {
+        if (i >= n) return;
+        const u32 row = row0 + i * SP_WARPS + warp;
+        const u32 piece = row % pieces, rest = row / pieces;
+        const u32 q = rest % c.nsrc, r0 = rest / c.nsrc * c.group;
+        const u64 p0 = (u64)piece * c.per;
+        const u32 len = (u32)min((u64)c.per, c.nu - p0);
+        const u64 off = c.rs * r0 + p0;
+        m.src = ld_ptr(c.src, q) + off;
+        m.dst = (u64)q * c.nu + p0;
+        if (c.group == 1) m.dst += (u64)ld_ptr(c.dst, r0);
+        // the 16-byte units the row touches, but none that leave the buffer
+        const uintptr_t a = (uintptr_t)m.src, e = a + len;
+        const uintptr_t x0 = off >= 16 ? a & ~(uintptr_t)15 : (a + 15) & ~(uintptr_t)15;
+        const uintptr_t x1 = off + len + 16 <= extent ? (e + 15) & ~(uintptr_t)15 : e & ~(uintptr_t)15;
+        from = reinterpret_cast<const char*>(x0);
+        bytes = x1 > x0 ? (u32)(x1 - x0) : 0;
+        m.head = bytes ? (x0 > a ? (u32)(x0 - a) : 0) : len;
+        m.tail = bytes && e > x1 ? (u32)(e - x1) : 0;
+        m.len = len - m.head - m.tail;
+        m.at = x0 < a ? (u32)(a - x0) : 0;
+        m.r0 = r0;
+    };
+    auto issue = [&](u32 i, u32 stage) {
+        if ((i & 31) == 0) prepare(i + lane);
+        if (lane == (i & 31)) {
+            info[stage] = m;
+            ring_load(ring, stage, part + stage * pitch, from, bytes);
+        }
+    };
+    // the ring may hold what other tiles wrote with ordinary stores
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+    for (u32 i = 0; i < c.stages && i < n; i++) issue(i, i);
+    u32 stage = 0;
+    for (u32 i = 0; i < n; i++) {
+        ring_wait(ring, stage, phases, job);
+        const MoveRow w = info[stage];
+        const char* at = part + stage * pitch + w.at;
+        const u32 r1 = min(w.r0 + c.group, c.ndst);
+        for (u32 r = w.r0; r < r1; r++) {
+            char* d = reinterpret_cast<char*>(c.group == 1 ? w.dst : (u64)ld_ptr(c.dst, r) + w.dst);
+            move_row(d + w.head, at, w.len, lane);
+            if (w.head | w.tail) {
+                for (u32 k = lane; k < w.head; k += 32) d[k] = __ldcg(w.src + k);
+                const u32 done = w.head + w.len;
+                for (u32 k = lane; k < w.tail; k += 32) d[done + k] = __ldcg(w.src + done + k);
+            }
+        }
+        __syncwarp();   // the stage has been read
+        if (i + c.stages < n && !*(volatile u32*)&ring.failed) issue(i + c.stages, stage);
+        if (++stage == c.stages) stage = 0;
+    }
+}
+
+template <template <class> class O>
+static __device__ void fold_types(const SpreadCall& c, u32 tile, char* smem) {
+    switch (c.fn >> 2) {
+        case FT_I8: fold_tile<signed char, O<signed char>>(c, tile, smem); break;
+        case FT_I16: fold_tile<short, O<short>>(c, tile, smem); break;
+        case FT_I32: fold_tile<int, O<int>>(c, tile, smem); break;
+        case FT_I64: fold_tile<long long, O<long long>>(c, tile, smem); break;
+        case FT_F32: fold_tile<float, O<float>>(c, tile, smem); break;
+        case FT_F64: fold_tile<double, O<double>>(c, tile, smem); break;
+        default: break;
+    }
+}
+
+template <template <class> class O>
+static __device__ void fold_unsigned(const SpreadCall& c, u32 tile, char* smem) {
+    switch (c.fn >> 2) {
+        case FT_U8: fold_tile<unsigned char, O<unsigned char>>(c, tile, smem); break;
+        case FT_U16: fold_tile<unsigned short, O<unsigned short>>(c, tile, smem); break;
+        case FT_U32: fold_tile<unsigned, O<unsigned>>(c, tile, smem); break;
+        case FT_U64: fold_tile<unsigned long long, O<unsigned long long>>(c, tile, smem); break;
+        default: break;
+    }
+}
+
+static __device__ void run_tile(const SpreadCall& c, u32 tile, char* smem, Ring& ring, u32& phases, Job* job) {
+    if (c.kind == SP_MOVE) {
+        move_tile(c, tile, smem, ring, phases, job);
+    } else if (c.kind == SP_FAN) {
+        switch (c.ub) {
+            case 16: fan_tile<uint4>(c, tile); break;
+            case 8: fan_tile<uint2>(c, tile); break;
+            case 4: fan_tile<u32>(c, tile); break;
+            case 2: fan_tile<unsigned short>(c, tile); break;
+            default: fan_tile<unsigned char>(c, tile); break;
+        }
+    } else if (c.kind == SP_COPY) {
+        switch (c.ub) {
+            case 16: copy_tile<uint4>(c, tile); break;
+            case 8: copy_tile<uint2>(c, tile); break;
+            case 4: copy_tile<u32>(c, tile); break;
+            case 2: copy_tile<unsigned short>(c, tile); break;
+            default: copy_tile<unsigned char>(c, tile); break;
+        }
+    } else {
+        switch (c.fn & 3) {
+            case GPUMPI_OP_MAX:
+                fold_types<OMax>(c, tile, smem);
+                fold_unsigned<OMax>(c, tile, smem);
+                break;
+            case GPUMPI_OP_MIN:
+                fold_types<OMin>(c, tile, smem);
+                fold_unsigned<OMin>(c, tile, smem);
+                break;
+            case GPUMPI_OP_SUM: fold_types<OSum>(c, tile, smem); break;
+            default: fold_types<OProd>(c, tile, smem); break;
+        }
+    }
+}
+
+}  // namespace gm
+
+using namespace gm;
+
+extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
+    gpumpi_spread_kernel(const __grid_constant__ SpreadArgs A) {
+    extern __shared__ __align__(16) char sp_smem[];
+    // the tile's call: in shared memory, so that no thread holds it in registers
+    __shared__ SpreadCall c;
+    __shared__ Ring ring;
+    u32 phases = 0;
+    if (threadIdx.x < SP_WARPS * SP_MAX_STAGES) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&ring.full[0][0] + threadIdx.x)) : "memory");
+        ring.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (u32 t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
+        constexpr u32 W = sizeof(SpreadCall) / 8;
+        if (A.ncalls == 1) {
+            if (threadIdx.x < W)
+                reinterpret_cast<u64*>(&c)[threadIdx.x] = reinterpret_cast<const u64*>(&A.one)[threadIdx.x];
+        } else {
+            // the call whose range holds tile t: exactly one thread finds it
+            __shared__ u32 s_call;
+            for (u32 i = threadIdx.x; i < A.ncalls; i += SP_T) {
+                const u32 f = __ldg(&A.calls[i].first_tile), n = __ldg(&A.calls[i].ntiles);
+                if (t - f < n) s_call = i;
+            }
+            __syncthreads();
+            if (threadIdx.x < W)
+                reinterpret_cast<u64*>(&c)[threadIdx.x] =
+                    __ldg(reinterpret_cast<const u64*>(A.calls + s_call) + threadIdx.x);
+        }
+        __syncthreads();
+        run_tile(c, t - c.first_tile, sp_smem, ring, phases, A.job);
+        __syncthreads();
+    }
+    if (ring.failed) {
+        // loads may still be on their way into this block's shared memory
+        const u64 t0 = gtime();
+        while (gtime() - t0 < 1000000000ull) __nanosleep(1000);
+    }
+}
+
+// ------------------------------------------------------------------ host
+
+namespace gm {
+
+static int fold_type(int dtype) {
+    switch (dtype) {
+        case MPI_SIGNED_CHAR: case MPI_INT8_T: return FT_I8;
+        case MPI_UNSIGNED_CHAR: case MPI_UINT8_T: case MPI_BYTE: return FT_U8;
+        case MPI_SHORT: case MPI_INT16_T: return FT_I16;
+        case MPI_UNSIGNED_SHORT: case MPI_UINT16_T: return FT_U16;
+        case MPI_INT: case MPI_INT32_T: return FT_I32;
+        case MPI_UNSIGNED: case MPI_UINT32_T: return FT_U32;
+        case MPI_LONG: case MPI_LONG_LONG_INT: case MPI_LONG_LONG: case MPI_INT64_T: return FT_I64;
+        case MPI_UNSIGNED_LONG: case MPI_UNSIGNED_LONG_LONG: case MPI_UINT64_T: return FT_U64;
+        case MPI_FLOAT: return FT_F32;
+        case MPI_DOUBLE: return FT_F64;
+        default: return FT_NONE;
+    }
+}
+
+// Alltoall blocks from here on move by bulk copies; shorter ones go one unit
+// per thread (SP_COPY) or one unit per thread and block (SP_FAN).  A row costs
+// its warp some 80 instructions whatever its length, a unit per thread some 15
+// each: with 16-byte units the lines cross near 8 KiB (int32 Alltoall of
+// communicators of 4..256 ranks, 2^17 elements per rank: 251 us with bulk
+// copies from 2 KiB, 218 us from 8 KiB; FP64 at 2^20 3.74 ms without them,
+// 2.9 ms with), with 4- or 8-byte units near 512 bytes (int32, 2^12 per rank:
+// 18.3 us from 256 bytes, 15.0 us from 512; 2^20: 1010 us without, 768 us with).
+constexpr u64 SP_MOVE_ALIGNED = 8192;
+constexpr u64 SP_MOVE_BYTES = 512;
+constexpr u64 SP_PIECE = 1920;       // longest piece: three fit a warp's part of the ring
+
+static bool is_fold(int op) { return op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE; }
+
+bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
+    if (d.algo != 0 || d.sync != 0 || d.op == GPUMPI_COLL_BARRIER || !d.recvbufs || P > SP_MAX_RANKS) return false;
+    if (is_fold(d.op) && fold_type(d.dtype) == FT_NONE) return false;
+    auto usable = [&](const void* p) { return p != nullptr && p != MPI_IN_PLACE && (uintptr_t)p % esize == 0; };
+    for (int r = 0; r < P; r++) {
+        if (d.op != GPUMPI_COLL_BCAST && !usable(d.sendbufs ? d.sendbufs[r] : d.recvbufs[r])) return false;
+        if ((d.op != GPUMPI_COLL_REDUCE || r == d.root) && !usable(d.recvbufs[r])) return false;
+    }
+    return true;
+}
+
+double SpreadBuilder::traffic(const gpumpi_coll_desc& d, int P, int esize) {
+    const double e = (double)d.count * esize;
+    switch (d.op) {
+        case GPUMPI_COLL_BCAST: return e * P;
+        case GPUMPI_COLL_REDUCE: return e * (P + 1);
+        case GPUMPI_COLL_ALLREDUCE: return 2 * e * P;
+        default: return 2 * e * P * P;
+    }
+}
+
+void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double total) {
+    if (d.count == 0) return;
+    // traffic of one tile: a few tiles for each of the blocks that run at once
+    const double target = std::min(1048576.0, std::max(16384.0, total / (152.0 * SP_BLOCKS_PER_SM * 2)));
+    std::vector<void*> src, dst;
+    auto sendbuf = [&](int r) { return d.sendbufs ? d.sendbufs[r] : d.recvbufs[r]; };
+    switch (d.op) {
+        case GPUMPI_COLL_BCAST:
+            src.push_back(d.recvbufs[d.root]);
+            for (int r = 0; r < P; r++)
+                if (r != d.root && d.recvbufs[r] != d.recvbufs[d.root]) dst.push_back(d.recvbufs[r]);
+            break;
+        case GPUMPI_COLL_REDUCE:
+            for (int r = 0; r < P; r++) src.push_back(sendbuf(r));
+            dst.push_back(d.recvbufs[d.root]);
+            break;
+        default:
+            for (int r = 0; r < P; r++) {
+                src.push_back(sendbuf(r));
+                dst.push_back(d.recvbufs[r]);
+            }
+    }
+    if (dst.empty() || (P == 1 && src[0] == dst[0])) return;
+    uintptr_t bits = 0;   // alignment that every address shares
+    for (void* p : src) bits |= (uintptr_t)p;
+    for (void* p : dst) bits |= (uintptr_t)p;
+    SpreadCall c;
+    memset(&c, 0, sizeof(c));
+    c.src = (const char* const*)ptrs.size();
+    ptrs.insert(ptrs.end(), src.begin(), src.end());
+    c.dst = (char* const*)ptrs.size();
+    ptrs.insert(ptrs.end(), dst.begin(), dst.end());
+    c.nsrc = (u32)src.size();
+    c.ndst = (u32)dst.size();
+    const u64 bytes = d.count * (u64)esize;
+    if (is_fold(d.op)) {
+        int ft = fold_type(d.dtype);
+        if (d.redop == GPUMPI_OP_SUM || d.redop == GPUMPI_OP_PROD) {
+            if (ft == FT_U8 || ft == FT_U16 || ft == FT_U32 || ft == FT_U64) ft--;
+        }
+        c.fn = ft * 4 + d.redop;
+        const u64 V = 16 / esize;
+        const bool aligned = bits % 16 == 0;
+        const u64 main = aligned ? d.count / V * V : d.count;   // elements in whole vectors
+        auto rows = [&](u32 ub) { return (double)(c.nsrc + c.ndst) * SP_T * ub; };   // traffic of one row
+        c.ub = 0;
+        if (aligned && rows(16) <= 2 * target) c.ub = 16;
+        else if (esize >= 4 && rows(esize) <= 2 * target) c.ub = esize;
+        const u64 whole = c.ub == 16 ? main : d.count;
+        if (c.ub && whole * esize >= (u64)SP_T * c.ub) {
+            c.kind = SP_STREAM;
+            c.nu = whole;
+            const u64 nrows = (whole * esize / c.ub + SP_T - 1) / SP_T;
+            c.per = (u32)std::max(1.0, std::min((double)nrows, target / rows(c.ub)));
+            c.ntiles = (u32)((nrows + c.per - 1) / c.per);
+            calls.push_back(c);
+            if (whole == d.count) return;
+            c.off = whole * esize;
+        }
+        // the whole vector, or the elements after its last whole 16 bytes
+        c.nu = d.count - c.off / esize;
+        c.kind = SP_GATHER;
+        c.ub = aligned && c.nu % V == 0 ? 16 : esize;
+        u64 m = (u64)(std::min(target / 2, (double)SP_RING) / ((double)P * esize));
+        const u64 step = c.ub == 16 ? V : 1;
+        m = std::max(step, std::min(m, c.nu) / step * step);
+        c.per = (u32)m;
+        c.ntiles = (u32)((c.nu + m - 1) / m);
+        calls.push_back(c);
+        return;
+    }
+    const bool a2a = d.op == GPUMPI_COLL_ALLTOALL;
+    c.rs = a2a ? bytes : 0;
+    if (a2a && bytes >= ((bits | bytes) % 16 == 0 ? SP_MOVE_ALIGNED : SP_MOVE_BYTES)) {
+        c.kind = SP_MOVE;
+        c.nu = bytes;
+        const u64 pieces = (bytes + SP_PIECE - 1) / SP_PIECE;
+        const u64 step = pieces > 1 ? 128 : 16;
+        c.per = (u32)(((bytes + pieces - 1) / pieces + step - 1) / step * step);
+        c.stages = std::min((u32)SP_MAX_STAGES, SP_PART / (c.per + 32));
+        c.group = 1;
+        const u64 rows = (bytes + c.per - 1) / c.per * c.nsrc * c.ndst;
+        c.rows = (u32)std::max(1.0, target / (2.0 * c.per));
+        c.ntiles = (u32)((rows + c.rows - 1) / c.rows);
+        calls.push_back(c);
+        return;
+    }
+    bits |= bytes;
+    c.ub = bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
+    c.nu = bytes / c.ub;
+    if (c.nu >= 2 * SP_T) {
+        c.kind = SP_FAN;
+        // a piece: 8 units per thread, more when the launch is large, fewer when the block is short
+        u64 per = 8 * SP_T;
+        if (a2a) per *= (u64)std::max(1.0, target / (2.0 * per * c.ub));
+        const u64 pieces = (c.nu + per - 1) / per;
+        per = ((c.nu + pieces - 1) / pieces + SP_T - 1) / SP_T * SP_T;
+        c.per = (u32)per;
+        c.group = a2a ? 1 : (u32)std::max(1.0, std::min((double)c.ndst, target / ((double)per * c.ub)));
+        c.ntiles = (u32)((c.nu + per - 1) / per * c.nsrc * ((c.ndst + c.group - 1) / c.group));
+    } else {
+        c.kind = SP_COPY;
+        const u64 units = (u64)c.ndst * c.nsrc * c.nu;
+        u64 per = SP_T * (u64)std::max(1.0, target / (2.0 * SP_T * c.ub));
+        c.per = (u32)per;
+        c.ntiles = (u32)((units + per - 1) / per);
+    }
+    calls.push_back(c);
+}
+
+u32 SpreadBuilder::finish(const char* ptr_base) {
+    u32 n = 0;
+    for (SpreadCall& c : calls) {
+        c.src = (const char* const*)(ptr_base + (size_t)c.src * sizeof(void*));
+        c.dst = (char* const*)(ptr_base + (size_t)c.dst * sizeof(void*));
+        c.first_tile = n;
+        n += c.ntiles;
+    }
+    return n;
+}
+
+}  // namespace gm

@@ -1,0 +1,109 @@
+// Spread form of launch-ordered plans: the work of every call of a launch as
+// one list of independent tiles, one thread block per tile.
+//
+// The rank form (gpumpi_plan_kernel) gives each rank one block, which runs
+// its rank's share of one call after another.  A launch of 8 ranks then uses
+// 8 of 152 SMs, a communicator of 256 ranks finishes long after one of 4, and
+// six one-element calls take six times one call's latency.  In a
+// launch-ordered plan nothing of that is needed: the calls touch disjoint
+// memory and every input was complete when the launch started, so any block
+// may do any piece of any call.  The results are those of the rank form, bit
+// for bit: copies are copies, and a fold takes its inputs in rank order.
+//
+// Measured (rank form -> spread form, one launch): Allreduce of 8 ranks of 16
+// MiB 2515 -> 52 us; the 16-communicator batch of Bcast, Allreduce and Alltoall
+// at 1 element per rank 81 -> 16 us, at 301 326 -> 27 us, at 2^15 477 -> 379
+// us, at 100003 (rank buffers aligned to their elements only) 1909 -> 1202 us,
+// at 2^20 11.55 -> 10.29 ms.
+#pragma once
+
+#include <stdint.h>
+#include <string.h>
+
+#include <vector>
+
+#include "gpumpi.h"
+#include "rt.cuh"
+
+namespace gm {
+
+constexpr int SP_T = 256;               // threads of a block
+constexpr u32 SP_RING = 48 * 1024;      // staging bytes of a block
+constexpr int SP_TAB = 256;             // ranks whose buffer addresses fit in shared memory
+constexpr int SP_MAX_RANKS = SP_RING / 16;   // a gather tile holds 16 bytes of every rank
+constexpr u32 SP_SMEM = SP_RING + 2 * SP_TAB * (u32)sizeof(char*);
+constexpr int SP_WARPS = SP_T / 32;
+constexpr u32 SP_PART = SP_RING / SP_WARPS;   // a warp's part of the ring
+constexpr int SP_MAX_STAGES = 8;
+constexpr int SP_BLOCKS_PER_SM = 4;     // 208 KiB of shared memory, 64 registers a thread
+
+// What the tiles of one SpreadCall do.  Units of a copy are `ub` bytes.
+enum SpreadKind : int {
+    // Blocks of `nu` units: block q of every destination row comes from source
+    // q.  A tile is `per` units of one block for `group` rows: loaded once,
+    // stored to each (Bcast: one source; Allgather; Alltoall with group = 1,
+    // whose source block lies `rs` bytes further for each row).
+    SP_FAN = 0,
+    // The same blocks when they are short: a tile is `per` units of the
+    // sequence of all rows, each loaded and stored by one thread.
+    SP_COPY = 1,
+    // Fold of `nu` elements over all sources in rank order, written to every
+    // destination.  A tile is `per` elements: the block loads them from all
+    // sources into shared memory at once, then thread i folds element i.
+    SP_GATHER = 2,
+    // The same fold for long vectors: a tile is `per` rows of one `ub`-byte
+    // vector per thread, every thread streams its own vectors of one source
+    // after another through its part of a ring in shared memory.
+    SP_STREAM = 3,
+    // Copies of longer blocks of any alignment (Alltoall, Allgather, Bcast): a
+    // row is a piece of `per` bytes of one block for `group` destinations, a
+    // tile is `rows` rows.  Each warp loads its rows by bulk copies of the
+    // 16-byte units they touch, `stages` rows ahead, and stores them from the
+    // ring, shifted to each destination's alignment.  `nu` is in bytes.
+    SP_MOVE = 4,
+};
+
+struct alignas(16) SpreadCall {
+    const char* const* src;     // [nsrc]
+    char* const* dst;           // [ndst]
+    u64 nu;
+    u64 rs;
+    u64 off;                    // folds: bytes added to every address
+    u32 first_tile, ntiles;
+    int kind;
+    int fn;                     // folds: element type and operator
+    u32 nsrc, ndst;
+    u32 per, group;
+    u32 ub;
+    u32 rows, stages;           // SP_MOVE: rows of a tile, stages of a warp's part of the ring
+    u32 pad;
+};
+
+struct SpreadArgs {
+    SpreadCall one;             // the call of a launch with a single SpreadCall
+    Job* job;                   // error words and the limit of every wait
+    const SpreadCall* calls;    // [ncalls]
+    u32 ncalls;
+    u32 ntiles;
+};
+
+// Collects the tiles of descriptors for one launch.  `ptr_base` is the device
+// address that `ptrs` will be copied to.
+struct SpreadBuilder {
+    std::vector<SpreadCall> calls;      // src / dst hold indexes into ptrs until relocate()
+    std::vector<void*> ptrs;
+
+    // True when the spread form covers the call (schedule and flag rounds left
+    // to the runtime, element type with the operator, no NULL buffer).
+    static bool covers(const gpumpi_coll_desc& d, int nranks, int esize);
+    // Bytes the call reads and writes.
+    static double traffic(const gpumpi_coll_desc& d, int nranks, int esize);
+    // Append the call's tiles, sized for a launch of `total` bytes of traffic.
+    void add(const gpumpi_coll_desc& d, int nranks, int esize, double total);
+    // Number the tiles and turn indexes into addresses.  Returns the tiles.
+    u32 finish(const char* ptr_base);
+};
+
+}  // namespace gm
+
+extern "C" __global__ void gpumpi_spread_kernel(const __grid_constant__ gm::SpreadArgs A);

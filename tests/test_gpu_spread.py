@@ -1,0 +1,152 @@
+"""Launch-ordered plans in spread form against the rank form and the host.
+
+A launch-ordered plan whose calls leave the schedule to the runtime runs as
+independent tiles over the whole GPU; with flag rounds (set_sync(1)) the same
+plan runs one block per rank.  Both are exact, so every output byte must be
+equal, and the bytes around each output untouched; Allreduce is also compared
+with a host fold in rank order (acc = x_0; acc = op(x_q, acc)).
+"""
+import ctypes
+import importlib.util
+import os
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# element types of the API: datatype value, NumPy type
+TYPES = {"i1": (6, np.int8), "u1": (29, np.uint8), "i2": (1, np.int16), "u2": (8, np.uint16), "i4": (2, np.int32),
+         "u4": (9, np.uint32), "i8": (20, np.int64), "u8": (11, np.uint64), "f4": (12, np.float32),
+         "f8": (13, np.float64)}
+OPS = {"max": 0, "min": 1, "sum": 2, "prod": 3}
+
+
+@pytest.fixture(scope="module")
+def api(gpu_built):
+    spec = importlib.util.spec_from_file_location("gpumpi_coll", os.path.join(gpu_built.PKG, "gpumpi_coll.py"))
+    mod = importlib.util.module_from_spec(spec)
+    sys.modules[spec.name] = mod
+    spec.loader.exec_module(mod)
+    return mod, mod.bind(gpu_built.load_library())
+
+
+def _values(rng, count, dt):
+    t = TYPES[dt][1]
+    if dt in ("f4", "f8"):
+        return rng.uniform(-1.5, 1.5, count).astype(t)
+    info = np.iinfo(t)
+    return rng.integers(info.min, info.max, count, dtype=t, endpoint=True)
+
+
+def _fold(xs, op):
+    acc = xs[0].copy()
+    with np.errstate(over="ignore", under="ignore"):
+        for x in xs[1:]:
+            acc = {"sum": lambda: x + acc, "prod": lambda: x * acc, "max": lambda: np.where(x > acc, x, acc),
+                   "min": lambda: np.where(x > acc, acc, x)}[op]()
+    return acc
+
+
+class Buffers:
+    """P buffers of `count` elements in one allocation, 64 guard bytes around each, starting `skew` elements
+    (times the rank) past a 16-byte boundary."""
+
+    def __init__(self, torch, p, count, dt, skew, values=None):
+        es = np.dtype(TYPES[dt][1]).itemsize
+        self.stride = (count * es + 15) // 16 * 16 + 160
+        self.host = np.full(p * self.stride, 0xA5, dtype=np.uint8)
+        self.at = [r * self.stride + 64 + (r * skew * es) % 16 for r in range(p)]
+        self.n = count * es
+        if values is not None:
+            for a, v in zip(self.at, values):
+                self.host[a:a + self.n] = v.view(np.uint8)
+        self.dev = torch.from_numpy(self.host.copy()).cuda()
+        self.ptrs = [self.dev.data_ptr() + a for a in self.at]
+
+    def reset(self, torch):
+        self.dev.copy_(torch.from_numpy(self.host))
+
+    def rows(self, dt):
+        """The buffers' contents; everything outside them must be as it was."""
+        now = self.dev.cpu().numpy()
+        inside = np.zeros(len(now), dtype=bool)
+        for a in self.at:
+            inside[a:a + self.n] = True
+        assert np.array_equal(now[~inside], self.host[~inside]), "bytes outside the buffers changed"
+        return [now[a:a + self.n].copy().view(TYPES[dt][1]) for a in self.at]
+
+
+def _run(api, p, n, dt, op, skew, batched):
+    import torch
+
+    coll, lib = api
+    rng = np.random.default_rng(p * 100003 + n * 7 + skew)
+    comm = coll.Comm(lib, p)
+    keep, descs, outs = [], [], []
+
+    def call(kind, count, send, recv, root=0):
+        s = coll.ptr_array(send.ptrs) if send else None
+        r = coll.ptr_array(recv.ptrs)
+        keep.extend([s, r, send, recv])
+        d = coll.Desc(comm.h, kind, TYPES[dt][0], OPS[op], root, count,
+                      ctypes.cast(s, ctypes.POINTER(ctypes.c_void_p)) if send else None,
+                      ctypes.cast(r, ctypes.POINTER(ctypes.c_void_p)), 0, 0)
+        descs.append(d)
+        outs.append(recv)
+
+    xs = [_values(rng, n, dt) for _ in range(p)]
+    call(coll.COLL_ALLREDUCE, n, Buffers(torch, p, n, dt, skew, xs), Buffers(torch, p, n, dt, skew))
+    place = Buffers(torch, p, n, dt, skew, xs)
+    call(coll.COLL_ALLREDUCE, n, place, place)
+    call(coll.COLL_REDUCE, n, Buffers(torch, p, n, dt, skew, xs), Buffers(torch, p, n, dt, 0), p - 1)
+    call(coll.COLL_BCAST, n, None, Buffers(torch, p, n, dt, skew, [_values(rng, n, dt) for _ in range(p)]), p // 2)
+    per = max(1, n // p)
+    call(coll.COLL_ALLTOALL, per, Buffers(torch, p, per * p, dt, skew, [_values(rng, per * p, dt) for _ in range(p)]),
+         Buffers(torch, p, per * p, dt, 3 * skew))
+    call(coll.COLL_ALLGATHER, per, Buffers(torch, p, per, dt, skew, [_values(rng, per, dt) for _ in range(p)]),
+         Buffers(torch, p, per * p, dt, 5 * skew))
+    plan = coll.Plan(lib, descs, threads=64, batched=batched)
+    assert plan.launch_ordered
+    got = []
+    for mode in (0, 1):
+        plan.set_sync(mode)
+        for o in outs:
+            o.reset(torch)
+        torch.cuda.synchronize()
+        plan.launch()
+        torch.cuda.synchronize()
+        assert coll.status(lib) is None
+        got.append([o.rows(dt) for o in outs])
+    plan.close()
+    comm.close()
+    for k, (a, b) in enumerate(zip(*got)):
+        if k == 1:
+            continue   # in place: with flag rounds a rank may fold a buffer that its owner has written already
+        for r in range(p):
+            assert a[r].tobytes() == b[r].tobytes(), "call %d rank %d" % (k, r)
+    want = _fold(xs, op)
+    for r in range(p):
+        assert got[0][0][r].tobytes() == want.tobytes() and got[0][1][r].tobytes() == want.tobytes()
+    assert got[0][2][p - 1].tobytes() == want.tobytes()
+
+
+@pytest.mark.parametrize("dt", sorted(TYPES))
+@pytest.mark.parametrize("op", ["max", "min", "sum", "prod"])
+def test_every_type_and_operator(api, dt, op):
+    _run(api, 5, 1000, dt, op, 0, True)
+    _run(api, 9, 333, dt, op, 1, False)
+
+
+@pytest.mark.parametrize("p,n", [(1, 1), (2, 1), (3, 31), (33, 32), (64, 255), (257, 1), (257, 300)])
+@pytest.mark.parametrize("dt", ["f8", "i4"])
+@pytest.mark.parametrize("skew", [0, 1])
+def test_short_calls(api, p, n, dt, skew):
+    _run(api, p, n, dt, "sum", skew, True)
+
+
+@pytest.mark.parametrize("p,n", [(2, 4096), (3, 50001), (8, 131072), (8, 262149), (48, 65537), (300, 6001)])
+@pytest.mark.parametrize("dt,skew", [("f8", 0), ("f8", 1), ("i4", 0), ("i4", 1), ("u1", 0), ("u1", 1), ("u2", 3)])
+def test_long_calls(api, p, n, dt, skew):
+    _run(api, p, n, dt, "max" if dt in ("u1", "u2") else "sum", skew, True)
