@@ -220,9 +220,10 @@ int api_job() {
     // in shared memory: prefer the largest shared-memory carve-out
     CK(cudaFuncSetAttribute((const void*)gpumpi_plan_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                             (int)cudaSharedmemCarveoutMaxShared));
-    CK(cudaFuncSetAttribute((const void*)gpumpi_spread_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                            (int)cudaSharedmemCarveoutMaxShared));
-    CK(cudaFuncSetAttribute((const void*)gpumpi_spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM));
+    for (const void* k : {(const void*)gpumpi_spread_kernel, (const void*)gpumpi_spread_levels_kernel}) {
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM));
+    }
     Job hj;
     memset(&hj, 0, sizeof(hj));
     char* mem = nullptr;
@@ -264,14 +265,17 @@ void desc_bytes(const gpumpi_coll_desc& d, int P, size_t* in, size_t* out) {
     }
 }
 
-// True when no call of the list writes memory that another call reads or
-// writes (and none is a barrier): the plan kernel may then run every call in
-// its launch-ordered form.  Each call's spans: the bytes each rank reads and
-// writes (Bcast: the root's buffer is read, the others written).  Spans of one
-// call never conflict with each other here (in-place forms are the
-// schedules' concern); spans are sorted by start and compared with the spans
-// still open.
-bool plan_independent(const gpumpi_coll_desc* descs, int ndesc) {
+// Levels of the calls of a list: a call is one level above the highest earlier
+// call that it shares memory with, one of the two writing it, so the calls of
+// one level touch disjoint memory.  Each call's spans: the bytes each rank
+// reads and writes (Bcast: the root's buffer is read, the others written).
+// Spans of one call never conflict with each other here (in-place forms are
+// the schedules' concern); spans are sorted by start and compared with the
+// spans still open.  Returns the number of levels, or 0 when the list holds a
+// barrier or is too long to be levelled.  One level means that the plan kernel
+// may run every call in its launch-ordered form.
+constexpr int MAX_LEVEL_CALLS = 2048;
+int plan_levels(const gpumpi_coll_desc* descs, int ndesc, std::vector<int>& level) {
     struct Span {
         uintptr_t lo, hi;
         int call, w;
@@ -279,7 +283,7 @@ bool plan_independent(const gpumpi_coll_desc* descs, int ndesc) {
     std::vector<Span> v;
     for (int i = 0; i < ndesc; i++) {
         const gpumpi_coll_desc& d = descs[i];
-        if (d.op == GPUMPI_COLL_BARRIER) return false;
+        if (d.op == GPUMPI_COLL_BARRIER) return 0;
         const int P = d.comm->n;
         const size_t e = (size_t)esize_of(d.dtype) * d.count;
         auto add = [&](void* const* tab, int r, size_t bytes, int w) {
@@ -290,7 +294,7 @@ bool plan_independent(const gpumpi_coll_desc* descs, int ndesc) {
             switch (d.op) {
                 case GPUMPI_COLL_BCAST: add(d.recvbufs, r, e, r != d.root); break;
                 case GPUMPI_COLL_REDUCE:
-                    add(d.sendbufs, r, e, 0);
+                    add(d.sendbufs ? d.sendbufs : d.recvbufs, r, e, 0);
                     if (r == d.root) add(d.recvbufs, r, e, 1);
                     break;
                 case GPUMPI_COLL_ALLREDUCE:
@@ -310,20 +314,34 @@ bool plan_independent(const gpumpi_coll_desc* descs, int ndesc) {
         }
     }
     std::sort(v.begin(), v.end(), [](const Span& a, const Span& b) { return a.lo < b.lo; });
+    std::vector<std::vector<char>> after;   // after[i][j], j < i: call i comes after call j
     std::vector<Span> open;
     for (const Span& x : v) {
         size_t k = 0;
         for (size_t j = 0; j < open.size(); j++)
             if (open[j].hi > x.lo) open[k++] = open[j];
         open.resize(k);
-        for (const Span& o : open)
-            if (o.call != x.call && (o.w || x.w)) return false;
+        for (const Span& o : open) {
+            if (o.call == x.call || !(o.w || x.w)) continue;
+            if (ndesc > MAX_LEVEL_CALLS) return 0;
+            if (after.empty()) after.resize(ndesc);
+            const int i = std::max(o.call, x.call), j = std::min(o.call, x.call);
+            if (after[i].empty()) after[i].assign(i, 0);
+            after[i][j] = 1;
+        }
         open.push_back(x);
     }
-    return true;
+    level.assign(ndesc, 0);
+    int n = 1;
+    for (size_t i = 0; i < after.size(); i++) {
+        for (size_t j = 0; j < after[i].size(); j++)
+            if (after[i][j]) level[i] = std::max(level[i], level[j] + 1);
+        n = std::max(n, level[i] + 1);
+    }
+    return n;
 }
 
-int launch(const void* kern, int grid, int threads, size_t smem, PlanArgs* args, cudaStream_t st) {
+int launch(const void* kern, int grid, int threads, size_t smem, void* args, cudaStream_t st) {
     void* params[] = {args};
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -341,8 +359,11 @@ int launch(const void* kern, int grid, int threads, size_t smem, PlanArgs* args,
     return GPUMPI_OK;
 }
 
-// Tiles are independent: any number of blocks, no cooperative launch.
+// Tiles of one level are independent: any number of blocks, no cooperative
+// launch.  Several levels need every block resident.
 int launch_spread(SpreadArgs* args, cudaStream_t st) {
+    if (args->nlevels > 1)
+        return launch((const void*)gpumpi_spread_levels_kernel, (int)args->blocks, SP_T, SP_SMEM, args, st);
     void* params[] = {args};
     const u32 grid = std::max(1u, std::min(args->ntiles, 1u << 30));
     CK(cudaLaunchKernel((const void*)gpumpi_spread_kernel, dim3(grid), dim3(SP_T), params, SP_SMEM, st));
@@ -468,30 +489,37 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     const size_t off_sp = off_pubt + sizeof(Pub) * (ptrs / 2);   // SpreadCalls, then their address tables
     // the spread form: the whole batched launch, or each plain launch it covers
     gpumpi_plan_s* p = new gpumpi_plan_s();
-    p->independent = plan_independent(descs, ndesc) ? 1 : 0;
+    std::vector<int> level;
+    const int nlevels = plan_levels(descs, ndesc, level);
+    p->independent = nlevels == 1;
     std::vector<SpreadBuilder> spread(batched ? 1 : ndesc);
     p->plain_spread.assign(ndesc, 0);
     p->plain_tiles.resize(ndesc);
     auto covers = [&](int i) { return SpreadBuilder::covers(descs[i], descs[i].comm->n, esize_of(descs[i].dtype)); };
     auto traffic = [&](int i) { return SpreadBuilder::traffic(descs[i], descs[i].comm->n, esize_of(descs[i].dtype)); };
     if (batched) {
-        double bytes = 0;
-        p->batch_spread = p->independent != 0;
+        std::vector<double> bytes(nlevels, 0.0);
+        p->batch_spread = nlevels > 0;
         for (int i = 0; i < ndesc && p->batch_spread; i++) {
             p->batch_spread = covers(i);
-            bytes += traffic(i);
+            bytes[level[i]] += traffic(i);
         }
-        for (int i = 0; i < ndesc && p->batch_spread; i++)
-            spread[0].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), bytes);
+        for (int l = 0; l < nlevels && p->batch_spread; l++) {
+            for (int i = 0; i < ndesc; i++)
+                if (level[i] == l) spread[0].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), bytes[l]);
+            spread[0].end_level();
+        }
     } else {
         for (int k = 0; k < ndesc; k++) {
             const int i = order[k];
             p->plain_spread[k] = covers(i);
-            if (p->plain_spread[k]) spread[k].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), traffic(i));
+            if (!p->plain_spread[k]) continue;
+            spread[k].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), traffic(i));
+            spread[k].end_level();
         }
     }
     size_t total = off_sp;
-    for (const SpreadBuilder& b : spread) total += sizeof(SpreadCall) * b.calls.size() + sizeof(void*) * b.ptrs.size() + 64;
+    for (const SpreadBuilder& b : spread) total += b.bytes() + 64;
     CK(cudaMalloc(&p->base, total));
     char* base = p->base;
     std::vector<char> h(total, 0);
@@ -553,21 +581,11 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     }
     size_t at = off_sp;
     for (size_t k = 0; k < spread.size(); k++) {
-        SpreadBuilder& b = spread[k];
+        at = (at + 63) & ~(size_t)63;
         SpreadArgs& a = batched ? p->batch_tiles : p->plain_tiles[k];
-        memset(&a, 0, sizeof(a));
-        const size_t calls_at = (at + 63) & ~(size_t)63;
-        at = calls_at + sizeof(SpreadCall) * b.calls.size();
-        a.ntiles = b.finish(base + at);
-        if (!b.calls.empty()) {
-            memcpy(h.data() + calls_at, b.calls.data(), sizeof(SpreadCall) * b.calls.size());
-            memcpy(h.data() + at, b.ptrs.data(), sizeof(void*) * b.ptrs.size());
-            a.one = b.calls[0];
-        }
-        at += sizeof(void*) * b.ptrs.size();
-        a.calls = (const SpreadCall*)(base + calls_at);
-        a.ncalls = (u32)b.calls.size();
+        spread[k].image(h.data() + at, base + at, &a);
         a.job = g_api.djob;
+        at += spread[k].bytes();
     }
     CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));
     p->ndesc = ndesc;
@@ -606,6 +624,10 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     int per = 0, sms = 0, dev = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (p->batch_spread && nlevels > 1) {
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)gpumpi_spread_levels_kernel, SP_T, SP_SMEM));
+        p->batch_tiles.blocks = std::max(1u, std::min((u32)(per * sms), p->batch_tiles.blocks));
+    }
     p->plain_smem.assign(ndesc, rank_smem_bytes(0));
     for (int k = 0; k <= ndesc; k++) {
         // k < ndesc: each plain launch at its own thread count; k == ndesc: the batched launch
@@ -634,7 +656,7 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
 static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
     const void* k = (const void*)gpumpi_plan_kernel;
     if (p->batched) {
-        if (p->batch_spread && p->batch_args.ordered) return launch_spread(&p->batch_tiles, st);
+        if (p->batch_spread && p->sync_mode == 0) return launch_spread(&p->batch_tiles, st);
         return launch(k, p->total_slots, p->threads, p->smem, &p->batch_args, st);
     }
     for (int i = 0; i < p->ndesc; i++) {

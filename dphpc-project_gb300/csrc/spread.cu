@@ -480,6 +480,88 @@ static __device__ void run_tile(const SpreadCall& c, u32 tile, char* smem, Ring&
     }
 }
 
+// Shared state of a block: its current call and the ring's barriers.
+struct Block {
+    SpreadCall c;   // in shared memory, so that no thread holds it in registers
+    u32 found;
+    Ring ring;
+};
+
+static __device__ __forceinline__ void block_begin(Block& b) {
+    if (threadIdx.x < SP_WARPS * SP_MAX_STAGES) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&b.ring.full[0][0] + threadIdx.x))
+                     : "memory");
+        b.ring.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+}
+
+static __device__ __forceinline__ void block_end(Block& b) {
+    if (b.ring.failed) {
+        // loads may still be on their way into this block's shared memory
+        const u64 t0 = gtime();
+        while (gtime() - t0 < 1000000000ull) __nanosleep(1000);
+    }
+}
+
+// This block's tiles of a level.
+static __device__ __forceinline__ void run_tiles(Block& b, const SpreadCall* one, const SpreadCall* calls, u32 ncalls,
+                                                 u32 ntiles, char* smem, u32& phases, Job* job) {
+    constexpr u32 W = sizeof(SpreadCall) / 8;
+    for (u32 t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        if (one) {
+            if (threadIdx.x < W)
+                reinterpret_cast<u64*>(&b.c)[threadIdx.x] = reinterpret_cast<const u64*>(one)[threadIdx.x];
+        } else {
+            // the call whose range holds tile t: exactly one thread finds it
+            for (u32 i = threadIdx.x; i < ncalls; i += SP_T) {
+                const u32 f = __ldg(&calls[i].first_tile), n = __ldg(&calls[i].ntiles);
+                if (t - f < n) b.found = i;
+            }
+            __syncthreads();
+            if (threadIdx.x < W)
+                reinterpret_cast<u64*>(&b.c)[threadIdx.x] =
+                    __ldg(reinterpret_cast<const u64*>(calls + b.found) + threadIdx.x);
+        }
+        __syncthreads();
+        run_tile(b.c, t - b.c.first_tile, smem, b.ring, phases, job);
+        __syncthreads();
+    }
+}
+
+// Every block of the launch has finished its tiles and sees the results of
+// all.  `arrived` counts blocks over all barriers of all launches of the plan
+// (each block adds `left` once it gives up, so that the count stays a whole
+// number of barriers).  Returns false when the wait ran out.
+static __device__ bool grid_barrier(Block& b, u64* arrived, u32 left, Job* job) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const u64 old = atomicAdd(arrived, 1ull);
+        const u64 target = (old / gridDim.x + 1) * gridDim.x;
+        u32 ok = 1;
+        if (ld_acquire(arrived) < target) {
+            const u64 t0 = gtime();
+            for (u32 i = 1; ld_acquire(arrived) < target; i++) {
+                if ((i & 255) == 0 && gtime() - t0 > job->timeout_ns) {
+                    job_fail(job, (int)blockIdx.x, GPUMPI_ERR_TIMEOUT, "a level of a plan did not complete");
+                    atomicAdd(arrived, (u64)left);
+                    ok = 0;
+                    break;
+                }
+            }
+        }
+        __threadfence();
+        b.found = ok;
+    }
+    __syncthreads();
+    const bool ok = b.found != 0;
+    // the next level's bulk loads read what ordinary stores of this level wrote
+    asm volatile("fence.proxy.async.global;" ::: "memory");
+    __syncthreads();
+    return ok;
+}
+
 }  // namespace gm
 
 using namespace gm;
@@ -487,41 +569,27 @@ using namespace gm;
 extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
     gpumpi_spread_kernel(const __grid_constant__ SpreadArgs A) {
     extern __shared__ __align__(16) char sp_smem[];
-    // the tile's call: in shared memory, so that no thread holds it in registers
-    __shared__ SpreadCall c;
-    __shared__ Ring ring;
+    __shared__ Block b;
     u32 phases = 0;
-    if (threadIdx.x < SP_WARPS * SP_MAX_STAGES) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&ring.full[0][0] + threadIdx.x)) : "memory");
-        ring.failed = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    block_begin(b);
+    run_tiles(b, A.ncalls == 1 ? &A.one : nullptr, A.calls, A.ncalls, A.ntiles, sp_smem, phases, A.job);
+    block_end(b);
+}
+
+// Calls that depend on each other: the levels one after another, a barrier of
+// all blocks (a cooperative launch) between two.
+extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
+    gpumpi_spread_levels_kernel(const __grid_constant__ SpreadArgs A) {
+    extern __shared__ __align__(16) char sp_smem[];
+    __shared__ Block b;
+    u32 phases = 0;
+    block_begin(b);
+    for (u32 l = 0; l < A.nlevels; l++) {
+        const SpreadLevel L = A.levels[l];
+        run_tiles(b, nullptr, A.calls + L.first_call, L.ncalls, L.ntiles, sp_smem, phases, A.job);
+        if (l + 1 < A.nlevels && !grid_barrier(b, A.arrived, A.nlevels - 2 - l, A.job)) break;
     }
-    for (u32 t = blockIdx.x; t < A.ntiles; t += gridDim.x) {
-        constexpr u32 W = sizeof(SpreadCall) / 8;
-        if (A.ncalls == 1) {
-            if (threadIdx.x < W)
-                reinterpret_cast<u64*>(&c)[threadIdx.x] = reinterpret_cast<const u64*>(&A.one)[threadIdx.x];
-        } else {
-            // the call whose range holds tile t: exactly one thread finds it
-            __shared__ u32 s_call;
-            for (u32 i = threadIdx.x; i < A.ncalls; i += SP_T) {
-                const u32 f = __ldg(&A.calls[i].first_tile), n = __ldg(&A.calls[i].ntiles);
-                if (t - f < n) s_call = i;
-            }
-            __syncthreads();
-            if (threadIdx.x < W)
-                reinterpret_cast<u64*>(&c)[threadIdx.x] =
-                    __ldg(reinterpret_cast<const u64*>(A.calls + s_call) + threadIdx.x);
-        }
-        __syncthreads();
-        run_tile(c, t - c.first_tile, sp_smem, ring, phases, A.job);
-        __syncthreads();
-    }
-    if (ring.failed) {
-        // loads may still be on their way into this block's shared memory
-        const u64 t0 = gtime();
-        while (gtime() - t0 < 1000000000ull) __nanosleep(1000);
-    }
+    block_end(b);
 }
 
 // ------------------------------------------------------------------ host
@@ -689,15 +757,46 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double tota
     calls.push_back(c);
 }
 
-u32 SpreadBuilder::finish(const char* ptr_base) {
-    u32 n = 0;
-    for (SpreadCall& c : calls) {
-        c.src = (const char* const*)(ptr_base + (size_t)c.src * sizeof(void*));
-        c.dst = (char* const*)(ptr_base + (size_t)c.dst * sizeof(void*));
-        c.first_tile = n;
-        n += c.ntiles;
+void SpreadBuilder::end_level() {
+    SpreadLevel l = {};
+    l.first_call = levels.empty() ? 0 : levels.back().first_call + levels.back().ncalls;
+    l.ncalls = (u32)calls.size() - l.first_call;
+    for (u32 i = l.first_call; i < (u32)calls.size(); i++) {
+        calls[i].first_tile = l.ntiles;
+        l.ntiles += calls[i].ntiles;
     }
-    return n;
+    levels.push_back(l);
+}
+
+size_t SpreadBuilder::bytes() const {
+    return sizeof(u64) * 2 + sizeof(SpreadCall) * calls.size() + sizeof(SpreadLevel) * levels.size() +
+           sizeof(void*) * ptrs.size();
+}
+
+void SpreadBuilder::image(char* host, char* dev, SpreadArgs* a) {
+    const size_t calls_at = sizeof(u64) * 2, levels_at = calls_at + sizeof(SpreadCall) * calls.size(),
+                 ptrs_at = levels_at + sizeof(SpreadLevel) * levels.size();
+    for (SpreadCall& c : calls) {
+        c.src = (const char* const*)(dev + ptrs_at + (size_t)c.src * sizeof(void*));
+        c.dst = (char* const*)(dev + ptrs_at + (size_t)c.dst * sizeof(void*));
+    }
+    memset(a, 0, sizeof(*a));
+    memset(host, 0, sizeof(u64) * 2);
+    if (!calls.empty()) {
+        a->one = calls[0];
+        memcpy(host + calls_at, calls.data(), sizeof(SpreadCall) * calls.size());
+        memcpy(host + ptrs_at, ptrs.data(), sizeof(void*) * ptrs.size());
+    }
+    memcpy(host + levels_at, levels.data(), sizeof(SpreadLevel) * levels.size());
+    a->arrived = (u64*)dev;
+    a->calls = (const SpreadCall*)(dev + calls_at);
+    a->levels = (const SpreadLevel*)(dev + levels_at);
+    a->nlevels = (u32)levels.size();
+    a->ncalls = (u32)calls.size();
+    for (const SpreadLevel& l : levels) {
+        a->ntiles = l.ntiles;
+        a->blocks = std::max(a->blocks, l.ntiles);
+    }
 }
 
 }  // namespace gm

@@ -79,31 +79,44 @@ struct alignas(16) SpreadCall {
     u32 pad;
 };
 
+// The tiles of a launch, level by level: the calls of a level touch disjoint
+// memory, those of the next may use their results.
+struct SpreadLevel {
+    u32 first_call, ncalls, ntiles, pad;
+};
+
 struct SpreadArgs {
     SpreadCall one;             // the call of a launch with a single SpreadCall
     Job* job;                   // error words and the limit of every wait
-    const SpreadCall* calls;    // [ncalls]
-    u32 ncalls;
+    const SpreadCall* calls;
+    const SpreadLevel* levels;  // [nlevels], for more than one
+    u64* arrived;               // blocks that reached the end of a level, over all launches
+    u32 ncalls;                 // one level: its calls and tiles
     u32 ntiles;
+    u32 nlevels;
+    u32 blocks;                 // more than one level: blocks of the launch
 };
 
-// Collects the tiles of descriptors for one launch.  `ptr_base` is the device
-// address that `ptrs` will be copied to.
+// Collects the tiles of descriptors for one launch.
 struct SpreadBuilder {
-    std::vector<SpreadCall> calls;      // src / dst hold indexes into ptrs until relocate()
+    std::vector<SpreadCall> calls;      // src / dst hold indexes into ptrs until image()
     std::vector<void*> ptrs;
+    std::vector<SpreadLevel> levels;
 
     // True when the spread form covers the call (schedule and flag rounds left
     // to the runtime, element type with the operator, no NULL buffer).
     static bool covers(const gpumpi_coll_desc& d, int nranks, int esize);
     // Bytes the call reads and writes.
     static double traffic(const gpumpi_coll_desc& d, int nranks, int esize);
-    // Append the call's tiles, sized for a launch of `total` bytes of traffic.
+    // Append the call's tiles, sized for a level of `total` bytes of traffic.
     void add(const gpumpi_coll_desc& d, int nranks, int esize, double total);
-    // Number the tiles and turn indexes into addresses.  Returns the tiles.
-    u32 finish(const char* ptr_base);
+    void end_level();
+    // Device image (calls, levels, counter, addresses) of bytes() bytes, and the launch arguments.
+    size_t bytes() const;
+    void image(char* host, char* dev, SpreadArgs* args);
 };
 
 }  // namespace gm
 
 extern "C" __global__ void gpumpi_spread_kernel(const __grid_constant__ gm::SpreadArgs A);
+extern "C" __global__ void gpumpi_spread_levels_kernel(const __grid_constant__ gm::SpreadArgs A);

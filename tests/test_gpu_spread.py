@@ -150,3 +150,55 @@ def test_short_calls(api, p, n, dt, skew):
 @pytest.mark.parametrize("dt,skew", [("f8", 0), ("f8", 1), ("i4", 0), ("i4", 1), ("u1", 0), ("u1", 1), ("u2", 3)])
 def test_long_calls(api, p, n, dt, skew):
     _run(api, p, n, dt, "max" if dt in ("u1", "u2") else "sum", skew, True)
+
+
+@pytest.mark.parametrize("p,n,skew", [(2, 64, 0), (7, 1001, 1), (48, 20000, 0), (257, 999, 1), (64, 65537, 0)])
+def test_dependent_calls_in_levels(api, p, n, skew):
+    """Calls that use each other's results, write buffers that earlier calls
+    read, and one that depends on nothing, in one launch: the same bytes as
+    with flag rounds, launch after launch."""
+    import torch
+
+    coll, lib = api
+    rng = np.random.default_rng(p + n)
+    comm, other = coll.Comm(lib, p), coll.Comm(lib, 3)
+    per = n // p
+    x, w, s = (Buffers(torch, p, n, "f8", skew, [_values(rng, n, "f8") for _ in range(p)]) for _ in range(3))
+    j = Buffers(torch, p, per * p, "f8", skew)
+    y, z = (Buffers(torch, 3, 100, "i4", skew, [_values(rng, 100, "i4") for _ in range(3)]) for _ in range(2))
+    keep = []
+
+    def call(c, kind, dt, count, send, recv, op=2, root=0):
+        return coll.make_desc(c, kind, {"f8": "float64", "i4": "int32"}[dt], count, send.ptrs if send else None,
+                              recv.ptrs, op, root, keep)
+
+    plan = coll.Plan(lib, [
+        call(comm, coll.COLL_ALLREDUCE, "f8", n, x, w),              # w: the sum
+        call(comm, coll.COLL_ALLTOALL, "f8", per, w, s),             # reads w
+        call(other, coll.COLL_ALLREDUCE, "i4", 100, y, z),           # on its own
+        call(comm, coll.COLL_ALLGATHER, "f8", per, s, j),            # reads s
+        call(comm, coll.COLL_REDUCE, "f8", per * p, j, x, 0, p - 1),  # writes what the first call read
+        call(comm, coll.COLL_BCAST, "f8", per * p, None, x, 0, p - 1),
+        call(comm, coll.COLL_ALLREDUCE, "f8", per * p, x, w, 3),     # writes w again
+    ], threads=64, batched=True)
+    assert not plan.launch_ordered
+    outs = [x, w, s, j, y, z]
+    types = ["f8"] * 4 + ["i4"] * 2
+    got = []
+    for mode in (0, 0, 1):
+        plan.set_sync(mode)
+        if len(got) == 1:
+            plan.capture()
+        for o in outs:
+            o.reset(torch)
+        torch.cuda.synchronize()
+        plan.launch()
+        torch.cuda.synchronize()
+        assert coll.status(lib) is None
+        got.append([o.rows(t) for o, t in zip(outs, types)])
+    plan.close()
+    comm.close()
+    other.close()
+    for a, b, c in zip(*got):
+        for u, v, t in zip(a, b, c):
+            assert u.tobytes() == v.tobytes() == t.tobytes()
