@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "redop.cuh"
 #include "spread.cuh"
@@ -24,6 +25,8 @@ template <class V>
 static __device__ __forceinline__ V ld_unit(const char* p) {
     return __ldcg(reinterpret_cast<const V*>(p));
 }
+
+static __device__ __forceinline__ u32 smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 
 // Asynchronous copy of B bytes to shared memory; 16-byte copies bypass L1.
 template <int B>
@@ -145,10 +148,9 @@ static __device__ __forceinline__ void gather_store(const SpreadCall& c, u64 at,
 }
 
 template <class T, class O>
-static __device__ void gather_tile(const SpreadCall& c, u32 tile, char* ring) {
-    const u64 lo = (u64)tile * c.per;
-    const u32 m = (u32)min((u64)c.per, c.nu - lo);
-    const u64 at = c.off + lo * sizeof(T);
+static __device__ __noinline__ void gather_tile(const SpreadCall& c, u32 tile, char* ring) {
+    const u32 m = (u32)min((u64)c.per, c.nu - (u64)tile * c.per);
+    const u64 at = c.off + tile * c.rs;
     if (c.ub == 16) gather_load<uint4>(c, at, m * (u32)sizeof(T) / 16, ring);
     else gather_load<T>(c, at, m, ring);
     cp_commit();
@@ -175,16 +177,34 @@ static __device__ void gather_tile(const SpreadCall& c, u32 tile, char* ring) {
     else gather_store<T>(c, at, m, ring);
 }
 
+// The call's addresses in shared memory, or where the host put them when they
+// are many.  The block synchronises before it uses them.
+static __device__ __forceinline__ void tables(const SpreadCall& c, char* smem, const char* const*& st, char* const*& dt) {
+    st = c.src;
+    dt = c.dst;
+    if (c.nsrc > SP_TAB) return;
+    const char** ts = reinterpret_cast<const char**>(smem + SP_RING);
+    char** td = reinterpret_cast<char**>(smem + SP_RING) + SP_TAB;
+    for (u32 q = threadIdx.x; q < c.nsrc; q += SP_T) ts[q] = ld_ptr(c.src, q);
+    for (u32 r = threadIdx.x; r < c.ndst; r += SP_T) td[r] = ld_ptr(c.dst, r);
+    st = ts;
+    dt = td;
+}
+
 // Every thread copies its own vectors into its own ring slots and reads only
 // those, so the pipeline needs no barrier: cp.async groups complete in order
 // and wait_group tells the thread when its oldest group has arrived.  GL loads
 // make a group; the ring holds SP_RING bytes per block whatever the vector.
 template <class T, class O, class V>
-static __device__ void stream_tile(const SpreadCall& c, u32 tile, char* ring, const char* const* st, char* const* dt) {
+static __device__ __noinline__ void stream_tile(const SpreadCall& c, u32 tile, char* ring) {
     constexpr int B = sizeof(V);
     constexpr int GL = 4;
     constexpr int NG = (int)(SP_RING / (SP_T * B)) / GL;
     static_assert(NG >= 2, "ring");
+    const char* const* st;
+    char* const* dt;
+    tables(c, ring, st, dt);
+    __syncthreads();
     const u64 nvec = c.nu * sizeof(T) / B;
     const u64 v0 = (u64)tile * c.per * SP_T + threadIdx.x;
     const u32 rows = (u32)min((u64)c.per, (nvec - (u64)tile * c.per * SP_T + SP_T - 1) / SP_T);
@@ -232,25 +252,111 @@ static __device__ void stream_tile(const SpreadCall& c, u32 tile, char* ring, co
     cp_wait<0>();
 }
 
+// ---- SP_ROWS
+//
+// A warp folds chunks of `per` elements: it copies the 16-byte units that a
+// chunk touches in `batch` sources at a time into its part of the ring, three
+// such groups deep, and every lane folds every 32nd element from there.  So
+// any element alignment costs the same: loads are 16-byte units, shared memory
+// is read without bank conflicts and stores fill whole lines.  No bulk copies:
+// one SM starts one of those every 44 cycles or so (measured with 144-byte
+// rows), which 512-byte rows only just afford.
+constexpr int SP_GROUPS = 3;
+
 template <class T, class O>
-static __device__ __noinline__ void fold_tile(const SpreadCall& c, u32 tile, char* smem) {
-    if (c.kind == SP_GATHER) {
-        gather_tile<T, O>(c, tile, smem);
-        return;
+static __device__ __noinline__ void rows_tile(const SpreadCall& c, u32 tile, char* smem) {
+    constexpr int K = 16 / sizeof(T);    // elements a lane holds of a chunk of 512 bytes
+    const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const char* const* st;
+    char* const* dt;
+    tables(c, smem, st, dt);
+    const u32 all = (u32)((c.nu + c.per - 1) / c.per);
+    const u32 w0 = tile * c.rows + warp, w1 = min(tile * c.rows + c.rows, all);
+    const u32 chunks = w1 > w0 ? (w1 - w0 + SP_WARPS - 1) / SP_WARPS : 0;   // this warp's
+    const u32 groups = (c.nsrc + c.batch - 1) / c.batch;
+    const u32 steps = chunks * groups;
+    const u32 pitch = c.ub, units = pitch / 16, group_bytes = c.batch * pitch;
+    char* part = smem + warp * SP_PART;
+    const u32 part_s = smem_addr(part);
+    // unit `lane` of a group, and how units 32 further on lie
+    const u32 j0 = lane / units, u0 = lane - j0 * units;
+    const u32 d_j = 32 / units, d_u = 32 - d_j * units;
+    u32 iw = w0, iq = 0, ig = 0, left = steps;
+    auto issue = [&]() {
+        if (left) {
+            left--;
+            const u64 e0 = (u64)iw * c.per;
+            const u32 mb = (u32)min((u64)c.per, c.nu - e0) * (u32)sizeof(T);
+            const u32 n = min(c.batch, c.nsrc - iq);
+            const u64 at = c.off + e0 * sizeof(T);
+            const u32 base = part_s + ig * group_bytes;
+            u32 j = j0, u = u0;
+            for (u32 k = lane; j < n; k += 32) {
+                const uintptr_t a = (uintptr_t)st[iq + j] + at;
+                if (u * 16 < ((u32)a & 15) + mb) cp_async<16>(base + k * 16, reinterpret_cast<const char*>((a & ~(uintptr_t)15) + u * 16));
+                j += d_j;
+                u += d_u;
+                if (u >= units) {
+                    u -= units;
+                    j++;
+                }
+            }
+            iq += c.batch;
+            if (iq >= c.nsrc) {
+                iq = 0;
+                iw += SP_WARPS;
+            }
+        }
+        cp_commit();
+        if (++ig == SP_GROUPS) ig = 0;
+    };
+    __syncthreads();   // the tables
+    for (int g = 0; g < SP_GROUPS - 1; g++) issue();
+    u32 cg = 0;
+    for (u32 w = w0; w < w1; w += SP_WARPS) {
+        const u64 e0 = (u64)w * c.per;
+        const u32 m = (u32)min((u64)c.per, c.nu - e0);
+        const u64 at = c.off + e0 * sizeof(T);
+        T acc[K];
+        for (u32 q0 = 0; q0 < c.nsrc; q0 += c.batch) {
+            __syncwarp();   // the group before has been read
+            issue();
+            cp_wait<SP_GROUPS - 1>();
+            __syncwarp();   // every lane's part of this group is there
+            const u32 n = min(c.batch, c.nsrc - q0);
+            const char* row = part + cg * group_bytes + lane * (u32)sizeof(T);
+            auto fold = [&](u32 j, bool first) {
+                const T* r = reinterpret_cast<const T*>(row + j * pitch + (((u32)(uintptr_t)st[q0 + j] + (u32)at) & 15));
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (k * 32 < m) {   // the lanes past the chunk's end fold what is there, and store nothing
+                        const T x = r[k * 32];
+                        acc[k] = first ? x : O::f(x, acc[k]);
+                    }
+                }
+            };
+            u32 j = 0;
+            if (q0 == 0) fold(j++, true);
+#pragma unroll 4
+            for (; j < n; j++) fold(j, false);
+            if (++cg == SP_GROUPS) cg = 0;
+        }
+#pragma unroll 4
+        for (u32 r = 0; r < c.ndst; r++) {
+            T* d = reinterpret_cast<T*>(dt[r] + at) + lane;
+#pragma unroll
+            for (int k = 0; k < K; k++)
+                if (k * 32 + lane < m) d[k * 32] = acc[k];
+        }
     }
-    const char* const* st = c.src;
-    char* const* dt = c.dst;
-    if (c.nsrc <= SP_TAB) {
-        const char** ts = reinterpret_cast<const char**>(smem + SP_RING);
-        char** td = reinterpret_cast<char**>(smem + SP_RING) + SP_TAB;
-        for (u32 q = threadIdx.x; q < c.nsrc; q += SP_T) ts[q] = ld_ptr(c.src, q);
-        for (u32 r = threadIdx.x; r < c.ndst; r += SP_T) td[r] = ld_ptr(c.dst, r);
-        __syncthreads();
-        st = ts;
-        dt = td;
-    }
-    if (c.ub == 16) stream_tile<T, O, uint4>(c, tile, smem, st, dt);
-    else if constexpr (sizeof(T) >= 4) stream_tile<T, O, T>(c, tile, smem, st, dt);
+    cp_wait<0>();
+}
+
+template <class T, class O>
+static __device__ __forceinline__ void fold_tile(const SpreadCall& c, u32 tile, char* smem) {
+    if (c.kind == SP_GATHER) gather_tile<T, O>(c, tile, smem);
+    else if (c.kind == SP_STREAM) stream_tile<T, O, uint4>(c, tile, smem);
+    else rows_tile<T, O>(c, tile, smem);
 }
 
 // ---- bulk copies into the ring
@@ -262,8 +368,6 @@ struct Ring {
     u64 full[SP_WARPS][SP_MAX_STAGES];
     u32 failed;     // a wait ran out: the block's later waits return at once
 };
-
-static __device__ __forceinline__ u32 smem_addr(const void* p) { return (u32)__cvta_generic_to_shared(p); }
 
 static __device__ __forceinline__ u32 bar_done(u32 bar, u32 parity) {
     u32 done;
@@ -624,6 +728,21 @@ constexpr u64 SP_MOVE_ALIGNED = 8192;
 constexpr u64 SP_MOVE_BYTES = 512;
 constexpr u64 SP_PIECE = 1920;       // longest piece: three fit a warp's part of the ring
 
+// Bytes of a rank's vector from which a fold goes by rows instead of gather
+// tiles.  A gather tile's loads are all under way at once, which the fewer
+// warps of a small launch need; rows keep loads under way while they fold,
+// take any alignment in 16-byte units and fill every lane, which counts in
+// large launches and for FP64 (2 additions a clock and SM).  Measured (gather
+// -> rows, us): FP64 Reduce of 64 x 50000 22 -> 16; Allreduce of 48 ranks, 20001
+// FP64 15.1 -> 18.4 and 100001 int32 22.5 -> 18.5; of the 16 communicators of
+// 4..256 ranks, 50001 int32 140 -> 93, 2^14 FP64 86 -> 100, 2^15 FP64 145 -> 121,
+// 2^15 int32 65 -> 70.
+static u64 rows_min(bool aligned, int esize, double total) {
+    const bool large = total >= 268435456.0;
+    if (!aligned) return large ? 131072 : 262144;
+    return large || esize == 8 ? 262144 : 524288;
+}
+
 static bool is_fold(int op) { return op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE; }
 
 bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
@@ -688,34 +807,56 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double tota
             if (ft == FT_U8 || ft == FT_U16 || ft == FT_U32 || ft == FT_U64) ft--;
         }
         c.fn = ft * 4 + d.redop;
-        const u64 V = 16 / esize;
+        const u64 V = 16 / esize, n = d.count;
         const bool aligned = bits % 16 == 0;
-        const u64 main = aligned ? d.count / V * V : d.count;   // elements in whole vectors
-        auto rows = [&](u32 ub) { return (double)(c.nsrc + c.ndst) * SP_T * ub; };   // traffic of one row
-        c.ub = 0;
-        if (aligned && rows(16) <= 2 * target) c.ub = 16;
-        else if (esize >= 4 && rows(esize) <= 2 * target) c.ub = esize;
-        const u64 whole = c.ub == 16 ? main : d.count;
-        if (c.ub && whole * esize >= (u64)SP_T * c.ub) {
+        const double row = (double)(c.nsrc + c.ndst);   // traffic per byte of a row
+        auto gather = [&](u64 first, u64 count, u64 per, u64 distance) {
+            SpreadCall g = c;
+            g.kind = SP_GATHER;
+            g.off = first * esize;
+            g.nu = count;
+            g.per = (u32)per;
+            g.rs = distance * esize;
+            g.ub = aligned && count % V == 0 && per % V == 0 && distance % V == 0 ? 16 : esize;
+            g.ntiles = (u32)((count + per - 1) / per);
+            g.tile_bytes = (u32)(row * per * esize);
+            calls.push_back(g);
+        };
+        // whole vectors, or what lies 16 bytes and more from both ends of the buffers
+        const u64 lo = aligned ? 0 : V, hi = aligned ? n / V * V : n > 2 * V ? n - V : 0;
+        if (aligned && row * SP_T * 16 <= 2 * target && hi >= SP_T * V) {
             c.kind = SP_STREAM;
-            c.nu = whole;
-            const u64 nrows = (whole * esize / c.ub + SP_T - 1) / SP_T;
-            c.per = (u32)std::max(1.0, std::min((double)nrows, target / rows(c.ub)));
+            c.nu = hi;
+            const u64 nrows = (hi / V + SP_T - 1) / SP_T;
+            c.per = (u32)std::max(1.0, std::min((double)nrows, target / (row * SP_T * 16)));
             c.ntiles = (u32)((nrows + c.per - 1) / c.per);
+            c.tile_bytes = (u32)(row * SP_T * 16 * c.per);
             calls.push_back(c);
-            if (whole == d.count) return;
-            c.off = whole * esize;
+            if (hi < n) gather(hi, n - hi, n - hi, n - hi);
+            return;
         }
-        // the whole vector, or the elements after its last whole 16 bytes
-        c.nu = d.count - c.off / esize;
-        c.kind = SP_GATHER;
-        c.ub = aligned && c.nu % V == 0 ? 16 : esize;
+        if (hi > lo && (hi - lo) * esize >= rows_min(aligned, esize, total)) {
+            c.kind = SP_ROWS;
+            c.off = lo * esize;
+            c.nu = hi - lo;
+            u32 chunk = 512;
+            while (chunk > 32 * (u32)esize && row * chunk * SP_WARPS > 4 * target) chunk /= 2;
+            c.per = chunk / esize;
+            c.ub = chunk + (aligned ? 0 : 16);
+            c.batch = std::min(c.nsrc, SP_PART / (SP_GROUPS * c.ub));
+            const u64 chunks = (c.nu + c.per - 1) / c.per;
+            c.rows = (u32)std::min((double)chunks, SP_WARPS * std::max(1.0, target / (row * chunk * SP_WARPS)));
+            c.ntiles = (u32)((chunks + c.rows - 1) / c.rows);
+            c.tile_bytes = (u32)(row * chunk * c.rows);
+            calls.push_back(c);
+            if (lo) gather(0, 2 * lo, lo, n - lo);
+            else if (hi < n) gather(hi, n - hi, n - hi, n - hi);
+            return;
+        }
         u64 m = (u64)(std::min(target / 2, (double)SP_RING) / ((double)P * esize));
-        const u64 step = c.ub == 16 ? V : 1;
-        m = std::max(step, std::min(m, c.nu) / step * step);
-        c.per = (u32)m;
-        c.ntiles = (u32)((c.nu + m - 1) / m);
-        calls.push_back(c);
+        const u64 step = aligned && n % V == 0 ? V : 1;
+        m = std::max(step, std::min(m, n) / step * step);
+        gather(0, n, m, m);
         return;
     }
     const bool a2a = d.op == GPUMPI_COLL_ALLTOALL;
@@ -757,10 +898,24 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double tota
     calls.push_back(c);
 }
 
+// Bytes that a tile moves, for a fold weighted by the length of its chain.
+static double tile_cost(const SpreadCall& c) {
+    switch (c.kind) {
+        case SP_FAN: return (double)c.per * c.ub * (1 + c.group);
+        case SP_COPY: return 2.0 * c.per * c.ub;
+        case SP_MOVE: return 2.0 * c.rows * c.per;
+        default: return (double)c.tile_bytes;
+    }
+}
+
 void SpreadBuilder::end_level() {
     SpreadLevel l = {};
     l.first_call = levels.empty() ? 0 : levels.back().first_call + levels.back().ncalls;
     l.ncalls = (u32)calls.size() - l.first_call;
+    // the longest tiles first: one that starts last would run alone
+    std::stable_sort(calls.begin() + l.first_call, calls.end(), [](const SpreadCall& a, const SpreadCall& b) {
+        return tile_cost(a) > tile_cost(b);
+    });
     for (u32 i = l.first_call; i < (u32)calls.size(); i++) {
         calls[i].first_tile = l.ntiles;
         l.ntiles += calls[i].ntiles;

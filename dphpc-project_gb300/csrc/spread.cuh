@@ -28,9 +28,9 @@
 namespace gm {
 
 constexpr int SP_T = 256;               // threads of a block
-constexpr u32 SP_RING = 48 * 1024;      // staging bytes of a block
+constexpr u32 SP_RING = 50 * 1024;      // staging bytes of a block
 constexpr int SP_TAB = 256;             // ranks whose buffer addresses fit in shared memory
-constexpr int SP_MAX_RANKS = SP_RING / 16;   // a gather tile holds 16 bytes of every rank
+constexpr int SP_MAX_RANKS = 3072;   // a gather tile holds 16 bytes of every rank
 constexpr u32 SP_SMEM = SP_RING + 2 * SP_TAB * (u32)sizeof(char*);
 constexpr int SP_WARPS = SP_T / 32;
 constexpr u32 SP_PART = SP_RING / SP_WARPS;   // a warp's part of the ring
@@ -61,13 +61,17 @@ enum SpreadKind : int {
     // 16-byte units they touch, `stages` rows ahead, and stores them from the
     // ring, shifted to each destination's alignment.  `nu` is in bytes.
     SP_MOVE = 4,
+    // The fold again, of buffers aligned to their elements only or in finer
+    // pieces.  Each warp folds chunks of `per` elements, a tile is `rows`
+    // chunks; `batch` sources are loaded at a time, `ub` bytes apart.
+    SP_ROWS = 5,
 };
 
 struct alignas(16) SpreadCall {
     const char* const* src;     // [nsrc]
     char* const* dst;           // [ndst]
     u64 nu;
-    u64 rs;
+    u64 rs;                     // SP_GATHER: bytes between the starts of two tiles
     u64 off;                    // folds: bytes added to every address
     u32 first_tile, ntiles;
     int kind;
@@ -75,8 +79,10 @@ struct alignas(16) SpreadCall {
     u32 nsrc, ndst;
     u32 per, group;
     u32 ub;
-    u32 rows, stages;           // SP_MOVE: rows of a tile, stages of a warp's part of the ring
-    u32 pad;
+    u32 rows;                   // SP_MOVE: rows of a tile; SP_ROWS: chunks
+    u32 stages;                 // SP_MOVE: stages of a warp's part of the ring
+    u32 batch;                  // SP_ROWS: sources of a group
+    u32 tile_bytes;             // folds: traffic of a tile
 };
 
 // The tiles of a launch, level by level: the calls of a level touch disjoint
