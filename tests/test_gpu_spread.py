@@ -202,3 +202,69 @@ def test_dependent_calls_in_levels(api, p, n, skew):
     for a, b, c in zip(*got):
         for u, v, t in zip(a, b, c):
             assert u.tobytes() == v.tobytes() == t.tobytes()
+
+
+@pytest.mark.parametrize("batched", [True, False])
+def test_launches_of_a_stream_keep_their_order(api, batched):
+    """Launches overlap the end of the one before, but read nothing it writes
+    too early: long and short plans, copies and kernels of one stream in turn,
+    directly and recorded into a graph, each using the one before."""
+    import torch
+
+    coll, lib = api
+    p, n = 6, 100000
+    g = torch.Generator().manual_seed(3)
+    x = torch.randint(-1000, 1000, (p, n), dtype=torch.int32, generator=g).cuda()
+    a, b, c = (torch.zeros(p, n, dtype=torch.int32, device="cuda") for _ in range(3))
+    comm = coll.Comm(lib, p)
+    keep = []
+    rows = lambda t, k=p: [t.data_ptr() + r * n * 4 for r in range(k)]  # noqa: E731
+    add = coll.Plan(lib, [coll.make_desc(comm, coll.COLL_ALLREDUCE, "int32", n, rows(a), rows(b), 2, 0, keep)],
+                    threads=64, batched=batched)
+    spread = coll.Plan(lib, [coll.make_desc(comm, coll.COLL_BCAST, "int32", 5, None, rows(b), 0, 1, keep)],
+                       threads=64, batched=batched)
+    empty = coll.Plan(lib, [coll.make_desc(comm, coll.COLL_ALLREDUCE, "int32", 0, rows(a), rows(b), 2, 0, keep)],
+                      threads=64, batched=batched)
+    turn = coll.Plan(lib, [coll.make_desc(comm, coll.COLL_ALLTOALL, "int32", n // p, rows(b), rows(c), 0, 0, keep)],
+                     threads=64, batched=batched)
+
+    def steps(stream):
+        a.copy_(x)                            # a copy, then plans, then kernels, over and over
+        for k in range(4):
+            add.launch(stream)                # b = sum of a
+            spread.launch(stream)             # a short one that writes b
+            empty.launch(stream)
+            turn.launch(stream)               # c from b
+            torch.add(c, k, out=a)            # a from c
+            c.zero_()
+
+    want = x.cpu().numpy()
+    per = n // p
+    with np.errstate(over="ignore"):
+        for k in range(4):
+            s = np.tile(want.sum(0, dtype=np.int32), (p, 1))
+            out = np.zeros_like(s)
+            for r in range(p):
+                for q in range(p):
+                    out[r, q * per:(q + 1) * per] = s[q, r * per:(r + 1) * per]
+            want = out + np.int32(k)
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(st):
+        steps(st.cuda_stream)
+    torch.cuda.synchronize()
+    assert np.array_equal(a.cpu().numpy(), want)
+    steps(0)
+    torch.cuda.synchronize()
+    assert np.array_equal(a.cpu().numpy(), want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        steps(st.cuda_stream)
+    for _ in range(3):
+        a.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(a.cpu().numpy(), want)
+    for plan in (add, spread, empty, turn):
+        plan.close()
+    comm.close()
