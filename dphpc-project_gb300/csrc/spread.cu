@@ -15,10 +15,11 @@ enum FoldType : int { FT_I8, FT_U8, FT_I16, FT_U16, FT_I32, FT_U32, FT_I64, FT_U
 
 // ------------------------------------------------------------------ device
 
-// Entry i of a table of addresses (constant while a launch runs).
+// Entry i of a table of addresses (constant while a launch runs), in global
+// memory or among the kernel's parameters.
 template <class P>
 static __device__ __forceinline__ P ld_ptr(P const* t, u32 i) {
-    return reinterpret_cast<P>(__ldg(reinterpret_cast<const u64*>(t) + i));
+    return t[i];
 }
 
 template <class V>
@@ -618,7 +619,8 @@ static __device__ __forceinline__ void block_end(Block& b) {
 
 // This block's tiles of a level.
 static __device__ __forceinline__ void run_tiles(Block& b, const SpreadCall* one, const SpreadCall* calls, u32 ncalls,
-                                                 u32 ntiles, char* smem, u32& phases, Job* job) {
+                                                 u32 ntiles, char* smem, u32& phases, Job* job,
+                                                 void* const* ptrs = nullptr) {
     constexpr u32 W = sizeof(SpreadCall) / 8;
     for (u32 t = blockIdx.x; t < ntiles; t += gridDim.x) {
         if (one) {
@@ -627,16 +629,23 @@ static __device__ __forceinline__ void run_tiles(Block& b, const SpreadCall* one
         } else {
             // the call whose range holds tile t: exactly one thread finds it
             for (u32 i = threadIdx.x; i < ncalls; i += SP_T) {
-                const u32 f = __ldg(&calls[i].first_tile), n = __ldg(&calls[i].ntiles);
+                const u32 f = calls[i].first_tile, n = calls[i].ntiles;
                 if (t - f < n) b.found = i;
             }
             __syncthreads();
             if (threadIdx.x < W)
-                reinterpret_cast<u64*>(&b.c)[threadIdx.x] =
-                    __ldg(reinterpret_cast<const u64*>(calls + b.found) + threadIdx.x);
+                reinterpret_cast<u64*>(&b.c)[threadIdx.x] = reinterpret_cast<const u64*>(calls + b.found)[threadIdx.x];
         }
         if (t == blockIdx.x) grid_wait();   // the tables above are the plan's own, the buffers are not
         __syncthreads();
+        if (ptrs) {
+            // src and dst are indexes into ptrs
+            if (threadIdx.x == 0) {
+                b.c.src = reinterpret_cast<const char* const*>(ptrs + reinterpret_cast<size_t>(b.c.src));
+                b.c.dst = reinterpret_cast<char* const*>(ptrs + reinterpret_cast<size_t>(b.c.dst));
+            }
+            __syncthreads();
+        }
         run_tile(b.c, t - b.c.first_tile, smem, b.ring, phases, job);
         __syncthreads();
     }
@@ -688,6 +697,20 @@ extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
     block_begin(b);
     if (blockIdx.x >= A.ntiles) grid_wait();   // no launch ends before the ones it follows
     run_tiles(b, A.ncalls == 1 ? &A.one : nullptr, A.calls, A.ncalls, A.ntiles, sp_smem, phases, A.job);
+    block_end(b);
+}
+
+// One call whose descriptors and addresses come with the launch, for callers
+// without device memory for them.
+extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
+    gpumpi_spread_params_kernel(const __grid_constant__ SpreadParams A) {
+    extern __shared__ __align__(16) char sp_smem[];
+    __shared__ Block b;
+    u32 phases = 0;
+    grid_trigger();
+    block_begin(b);
+    if (blockIdx.x >= A.ntiles) grid_wait();
+    run_tiles(b, nullptr, A.calls, A.ncalls, A.ntiles, sp_smem, phases, nullptr, A.ptrs);
     block_end(b);
 }
 
@@ -932,6 +955,15 @@ void SpreadBuilder::end_level() {
         l.ntiles += calls[i].ntiles;
     }
     levels.push_back(l);
+}
+
+bool SpreadBuilder::params(SpreadParams* p) const {
+    if (calls.size() > SP_PARAM_CALLS || ptrs.size() > 2 * SP_PARAM_RANKS || levels.size() != 1) return false;
+    std::copy(calls.begin(), calls.end(), p->calls);
+    std::copy(ptrs.begin(), ptrs.end(), p->ptrs);
+    p->ncalls = (u32)calls.size();
+    p->ntiles = levels[0].ntiles;
+    return true;
 }
 
 size_t SpreadBuilder::bytes() const {

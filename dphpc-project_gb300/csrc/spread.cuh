@@ -103,6 +103,16 @@ struct SpreadArgs {
     u32 blocks;                 // more than one level: blocks of the launch
 };
 
+// A launch whose calls and addresses are parameters of the kernel (4.5 KiB).
+constexpr int SP_PARAM_RANKS = 256;
+constexpr int SP_PARAM_CALLS = 3;   // a fold's whole vectors and its edges
+struct SpreadParams {
+    SpreadCall calls[SP_PARAM_CALLS];         // src / dst: indexes into ptrs
+    void* ptrs[2 * SP_PARAM_RANKS];
+    u32 ncalls;
+    u32 ntiles;
+};
+
 // Collects the tiles of descriptors for one launch.
 struct SpreadBuilder {
     std::vector<SpreadCall> calls;      // src / dst hold indexes into ptrs until image()
@@ -120,9 +130,12 @@ struct SpreadBuilder {
     // Device image (calls, levels, counter, addresses) of bytes() bytes, and the launch arguments.
     size_t bytes() const;
     void image(char* host, char* dev, SpreadArgs* args);
+    // The same as kernel parameters; false when they hold too few ranks.
+    bool params(SpreadParams* p) const;
 };
 
 }  // namespace gm
 
 extern "C" __global__ void gpumpi_spread_kernel(const __grid_constant__ gm::SpreadArgs A);
+extern "C" __global__ void gpumpi_spread_params_kernel(const __grid_constant__ gm::SpreadParams A);
 extern "C" __global__ void gpumpi_spread_levels_kernel(const __grid_constant__ gm::SpreadArgs A);

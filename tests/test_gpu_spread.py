@@ -268,3 +268,24 @@ def test_launches_of_a_stream_keep_their_order(api, batched):
     for plan in (add, spread, empty, turn):
         plan.close()
     comm.close()
+
+
+@pytest.mark.parametrize("p,n", [(1, 1), (2, 5), (31, 4097), (256, 1), (256, 40001)])
+@pytest.mark.parametrize("dt,skew", [("f8", 0), ("f8", 1), ("i4", 1), ("u2", 1)])
+def test_noalloc_allreduce_matches_the_host(api, p, n, dt, skew):
+    import torch
+
+    coll, lib = api
+    lib.gpumpi_allreduce_noalloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(ctypes.c_void_p),
+                                             ctypes.c_int, ctypes.c_uint64, ctypes.c_int, ctypes.c_int, ctypes.c_int,
+                                             ctypes.c_void_p]
+    rng = np.random.default_rng(p * 17 + n)
+    xs = [_values(rng, n, dt) for _ in range(p)]
+    send, recv = Buffers(torch, p, n, dt, skew, xs), Buffers(torch, p, n, dt, 3 * skew)
+    for _ in range(2):
+        recv.reset(torch)
+        rc = lib.gpumpi_allreduce_noalloc(coll.ptr_array(send.ptrs), coll.ptr_array(recv.ptrs), p, n, TYPES[dt][0],
+                                          OPS["sum"], 128, None)
+        assert rc == 0, lib.gpumpi_last_error().decode()
+        want = _fold(xs, "sum")
+        assert all(row.tobytes() == want.tobytes() for row in recv.rows(dt))
