@@ -415,40 +415,70 @@ struct MoveRow {
 };
 static_assert(sizeof(MoveRow) * SP_WARPS * SP_MAX_STAGES <= 2 * SP_TAB * sizeof(char*), "row table");
 
-template <class V>
-static __device__ __forceinline__ void move_units(char* d, const char* s, u32 n, u32 lane) {
+// L2 policies of a copy's stores: FAN copies store far more than they read, and
+// storing with evict_first leaves L2 to the few lines they read again (Bcast of
+// the 16 communicators at 2^20 FP64 per rank 1329 -> 1250 us, at 2^15 56 -> 48 us;
+// neither Alltoall nor Allreduce gain from it).  Launches that fit L2 keep their
+// results there.
+static __device__ __forceinline__ u64 l2_policy(bool cold) {
+    u64 first, normal;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
+    asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(normal));
+    return cold ? first : normal;
+}
+
+// *p = v; FAN: under an L2 policy.
+template <bool FAN, class V>
+static __device__ __forceinline__ void st_move(V* p, const V& v, u64 policy) {
+    if constexpr (!FAN) {
+        *p = v;
+    } else if constexpr (sizeof(V) == 16) {
+        asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z),
+                     "r"(v.w), "l"(policy) : "memory");
+    } else if constexpr (sizeof(V) == 8) {
+        asm volatile("st.global.L2::cache_hint.v2.b32 [%0], {%1, %2}, %3;" ::"l"(p), "r"(v.x), "r"(v.y), "l"(policy)
+                     : "memory");
+    } else {
+        asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(p), "r"(v), "l"(policy) : "memory");
+    }
+}
+
+template <bool FAN, class V>
+static __device__ __forceinline__ void move_units(char* d, const char* s, u32 n, u32 lane, u64 policy) {
     V* dv = reinterpret_cast<V*>(d);
     const V* sv = reinterpret_cast<const V*>(s);
     u32 i = lane;
     for (; i + 96 < n; i += 128) {
         const V a = sv[i], b = sv[i + 32], e = sv[i + 64], f = sv[i + 96];
-        dv[i] = a;
-        dv[i + 32] = b;
-        dv[i + 64] = e;
-        dv[i + 96] = f;
+        st_move<FAN>(dv + i, a, policy);
+        st_move<FAN>(dv + i + 32, b, policy);
+        st_move<FAN>(dv + i + 64, e, policy);
+        st_move<FAN>(dv + i + 96, f, policy);
     }
-    for (; i < n; i += 32) dv[i] = sv[i];
+    for (; i < n; i += 32) st_move<FAN>(dv + i, sv[i], policy);
 }
 
 // n bytes from shared memory s to d by one warp: the widest unit that both
 // alignments share, bytes up to the first and after the last whole one; with
 // no common alignment of 4, destination words put together from two source words.
-static __device__ __forceinline__ void move_row(char* d, const char* s, u32 n, u32 lane) {
+template <bool FAN>
+static __device__ __forceinline__ void move_row(char* d, const char* s, u32 n, u32 lane, u64 policy) {
     const u32 delta = ((u32)(uintptr_t)d - smem_addr(s)) & 15;
     const u32 unit = delta == 0 ? 16 : delta == 8 ? 8 : 4;
     u32 h = (0u - (u32)(uintptr_t)d) & (unit - 1);
     if (h > n) h = n;
     const u32 nw = (n - h) / unit;
     if (unit == 16) {
-        move_units<uint4>(d + h, s + h, nw, lane);
+        move_units<FAN, uint4>(d + h, s + h, nw, lane, policy);
     } else if (unit == 8) {
-        move_units<uint2>(d + h, s + h, nw, lane);
+        move_units<FAN, uint2>(d + h, s + h, nw, lane, policy);
     } else if ((delta & 3) == 0) {
-        move_units<u32>(d + h, s + h, nw, lane);
+        move_units<FAN, u32>(d + h, s + h, nw, lane, policy);
     } else {
         const u32* w = reinterpret_cast<const u32*>(reinterpret_cast<uintptr_t>(s + h) & ~(uintptr_t)3);
         const u32 sh = (smem_addr(s + h) & 3) * 8;
-        for (u32 i = lane; i < nw; i += 32) reinterpret_cast<u32*>(d + h)[i] = __funnelshift_r(w[i], w[i + 1], sh);
+        for (u32 i = lane; i < nw; i += 32)
+            st_move<FAN>(reinterpret_cast<u32*>(d + h) + i, __funnelshift_r(w[i], w[i + 1], sh), policy);
     }
     // at most 15 bytes on either side
     const u32 done = h + nw * unit;
@@ -456,11 +486,14 @@ static __device__ __forceinline__ void move_row(char* d, const char* s, u32 n, u
     if (done + lane < n) d[done + lane] = s[done + lane];
 }
 
+template <bool FAN>
 static __device__ __noinline__ void move_tile(const SpreadCall& c, u32 tile, char* smem, Ring& ring, u32& phases,
                                               Job* job) {
+    const u64 policy = FAN ? l2_policy(c.cold) : 0;
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const u32 pieces = (u32)((c.nu + c.per - 1) / c.per);
-    const u32 all = pieces * c.nsrc * ((c.ndst + c.group - 1) / c.group);
+    const u32 sets = (c.ndst + c.group - 1) / c.group;   // of destinations
+    const u32 all = pieces * c.nsrc * sets;
     const u32 row0 = tile * c.rows, row1 = min(row0 + c.rows, all);
     const u32 n = row1 - row0 > warp ? (row1 - row0 - warp + SP_WARPS - 1) / SP_WARPS : 0;   // this warp's rows
     const u32 pitch = c.per + 32;
@@ -474,14 +507,24 @@ static __device__ __noinline__ void move_tile(const SpreadCall& c, u32 tile, cha
     auto prepare = [&](u32 i) {
         if (i >= n) return;
         const u32 row = row0 + i * SP_WARPS + warp;
-        const u32 piece = row % pieces, rest = row / pieces;
-        const u32 q = rest % c.nsrc, r0 = rest / c.nsrc * c.group;
+        // Alltoall: a destination's rows follow each other; else a piece's rows do,
+        // which all read it while it is in L2
+        u32 piece, q, r0;
+        if (!FAN) {
+            piece = row % pieces;
+            q = row / pieces % c.nsrc;
+            r0 = row / pieces / c.nsrc;
+        } else {
+            r0 = row % sets * c.group;
+            piece = row / sets % pieces;
+            q = row / sets / pieces;
+        }
         const u64 p0 = (u64)piece * c.per;
         const u32 len = (u32)min((u64)c.per, c.nu - p0);
         const u64 off = c.rs * r0 + p0;
         m.src = ld_ptr(c.src, q) + off;
         m.dst = (u64)q * c.nu + p0;
-        if (c.group == 1) m.dst += (u64)ld_ptr(c.dst, r0);
+        if (!FAN) m.dst += (u64)ld_ptr(c.dst, r0);
         // the 16-byte units the row touches, but none that leave the buffer
         const uintptr_t a = (uintptr_t)m.src, e = a + len;
         const uintptr_t x0 = off >= 16 ? a & ~(uintptr_t)15 : (a + 15) & ~(uintptr_t)15;
@@ -510,20 +553,42 @@ static __device__ __noinline__ void move_tile(const SpreadCall& c, u32 tile, cha
         ring_wait(ring, stage, phases, job);
         const MoveRow w = info[stage];
         const char* at = part + stage * pitch + w.at;
-        const u32 r1 = min(w.r0 + c.group, c.ndst);
-        for (u32 r = w.r0; r < r1; r++) {
-            char* d = reinterpret_cast<char*>(c.group == 1 ? w.dst : (u64)ld_ptr(c.dst, r) + w.dst);
-            move_row(d + w.head, at, w.len, lane);
-            if (w.head | w.tail) {
-                for (u32 k = lane; k < w.head; k += 32) d[k] = __ldcg(w.src + k);
-                const u32 done = w.head + w.len;
-                for (u32 k = lane; k < w.tail; k += 32) d[done + k] = __ldcg(w.src + done + k);
+        const u32 r1 = FAN ? min(w.r0 + c.group, c.ndst) : w.r0 + 1;
+        // rows whose 16-byte units are also their destinations' leave by bulk
+        // copies, a lane for each destination; the rest go through registers
+        const bool whole = ((w.at | w.len | w.head | w.tail) & 15) == 0 && w.head + w.tail == 0;
+        for (u32 rb = w.r0; rb < r1; rb += 32) {
+            const u32 r = rb + lane;
+            const u64 d = r < r1 ? (FAN ? (u64)ld_ptr(c.dst, r) + w.dst : w.dst) : 0;
+            const bool bulk = whole && (d & 15) == 0;
+            if (FAN && bulk && r < r1)
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;"
+                             ::"l"(d), "r"(smem_addr(at)), "r"(w.len), "l"(policy) : "memory");
+            else if (bulk && r < r1)
+                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
+                             ::"l"(d), "r"(smem_addr(at)), "r"(w.len) : "memory");
+            u32 rest = __ballot_sync(~0u, r < r1 && !bulk);
+            while (rest) {
+                const u32 k = __ffs(rest) - 1;
+                rest &= rest - 1;
+                char* to = reinterpret_cast<char*>(__shfl_sync(~0u, d, k));
+                move_row<FAN>(to + w.head, at, w.len, lane, policy);
+                if (w.head | w.tail) {
+                    for (u32 x = lane; x < w.head; x += 32) to[x] = __ldcg(w.src + x);
+                    const u32 done = w.head + w.len;
+                    for (u32 x = lane; x < w.tail; x += 32) to[done + x] = __ldcg(w.src + done + x);
+                }
             }
         }
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         __syncwarp();   // the stage has been read
         if (i + c.stages < n && !*(volatile u32*)&ring.failed) issue(i + c.stages, stage);
         if (++stage == c.stages) stage = 0;
     }
+    // the results are in global memory before a level ends
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async.global;" ::: "memory");
 }
 
 template <template <class> class O>
@@ -552,7 +617,8 @@ static __device__ void fold_unsigned(const SpreadCall& c, u32 tile, char* smem) 
 
 static __device__ void run_tile(const SpreadCall& c, u32 tile, char* smem, Ring& ring, u32& phases, Job* job) {
     if (c.kind == SP_MOVE) {
-        move_tile(c, tile, smem, ring, phases, job);
+        if (c.rs) move_tile<false>(c, tile, smem, ring, phases, job);
+        else move_tile<true>(c, tile, smem, ring, phases, job);
     } else if (c.kind == SP_FAN) {
         switch (c.ub) {
             case 16: fan_tile<uint4>(c, tile); break;
@@ -777,6 +843,24 @@ static u64 rows_min(bool aligned, int esize, double total) {
     return large || esize == 8 ? 262144 : 524288;
 }
 
+// Bcast and Allgather by bulk copies: one load of a piece, a store to each of a
+// group of destinations.  With 16-byte alignment the stores are bulk copies, one
+// lane each, and the larger the group the better (2^20 FP64 per rank, group 8
+// 1461 us, 32 1413 us, all 1336 us; pieces of 6272 bytes 1325 us); otherwise the
+// warp writes one destination after another and 8 keep enough warps busy (100003
+// int32: 8 74 us, 16 79 us, 32 103 us).  It takes a large launch to keep the
+// pipelines full; before that, through registers (SP_FAN): Bcast of FP64 to 200
+// ranks, 105 MB 21.4 us against 21.9, 210 MB 46.3 against 39.6; to 48 ranks, 50 MB
+// 18.6 against 19.1, 400 MB 83 against 70; odd buffers, 210 MB 21.5 against 36.7
+// and 420 MB 87.5 against 76.5; the 16-communicator batch at 500001 per rank 5364
+// against 5104, at 50001 561 against 565.
+constexpr u64 SP_FAN_PIECE = 6272;
+constexpr double SP_FAN_ALIGNED = 1024, SP_FAN_ODD = 8;
+static u64 fan_min(bool units16, double total) {
+    if (units16) return total >= 2e8 ? 8192 : ~0ull;
+    return total >= 1e9 ? 524288 : ~0ull;
+}
+
 static bool is_fold(int op) { return op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE; }
 
 bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
@@ -895,16 +979,21 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double tota
     }
     const bool a2a = d.op == GPUMPI_COLL_ALLTOALL;
     c.rs = a2a ? bytes : 0;
-    if (a2a && bytes >= ((bits | bytes) % 16 == 0 ? SP_MOVE_ALIGNED : SP_MOVE_BYTES)) {
+    const bool units16 = (bits | bytes) % 16 == 0;
+    if (bytes >= (a2a ? units16 ? SP_MOVE_ALIGNED : SP_MOVE_BYTES : fan_min(units16, total))) {
+        const u64 longest = a2a ? SP_PIECE : SP_FAN_PIECE;
         c.kind = SP_MOVE;
+        c.cold = total >= 1e8;
         c.nu = bytes;
-        const u64 pieces = (bytes + SP_PIECE - 1) / SP_PIECE;
+        const u64 pieces = (bytes + longest - 1) / longest;
         const u64 step = pieces > 1 ? 128 : 16;
         c.per = (u32)(((bytes + pieces - 1) / pieces + step - 1) / step * step);
         c.stages = std::min((u32)SP_MAX_STAGES, SP_PART / (c.per + 32));
-        c.group = 1;
-        const u64 rows = (bytes + c.per - 1) / c.per * c.nsrc * c.ndst;
-        c.rows = (u32)std::max(1.0, target / (2.0 * c.per));
+        const double sets = units16 ? SP_FAN_ALIGNED : SP_FAN_ODD;
+        c.group = a2a ? 1 : (u32)std::min((double)c.ndst, std::max(1.0, std::min(sets, target / c.per)));
+        const u64 rows = (bytes + c.per - 1) / c.per * c.nsrc * ((c.ndst + c.group - 1) / c.group);
+        // at least a row for each warp (8 ranks of 2^17 FP64 11.8 -> 7.4 us)
+        c.rows = (u32)std::max(a2a ? (double)SP_WARPS : 1.0, target / ((1.0 + c.group) * c.per));
         c.ntiles = (u32)((rows + c.rows - 1) / c.rows);
         calls.push_back(c);
         return;
@@ -937,7 +1026,7 @@ static double tile_cost(const SpreadCall& c) {
     switch (c.kind) {
         case SP_FAN: return (double)c.per * c.ub * (1 + c.group);
         case SP_COPY: return 2.0 * c.per * c.ub;
-        case SP_MOVE: return 2.0 * c.rows * c.per;
+        case SP_MOVE: return (1.0 + c.group) * c.rows * c.per;
         default: return (double)c.tile_bytes;
     }
 }

@@ -83,6 +83,7 @@ struct alignas(16) SpreadCall {
     u32 stages;                 // SP_MOVE: stages of a warp's part of the ring
     u32 batch;                  // SP_ROWS: sources of a group
     u32 tile_bytes;             // folds: traffic of a tile
+    u32 cold;                   // SP_MOVE to several destinations: the results do not fit L2
 };
 
 // The tiles of a launch, level by level: the calls of a level touch disjoint
