@@ -519,17 +519,16 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     p->plain_spread.assign(ndesc, 0);
     p->plain_tiles.resize(ndesc);
     auto covers = [&](int i) { return SpreadBuilder::covers(descs[i], descs[i].comm->n, esize_of(descs[i].dtype)); };
-    auto traffic = [&](int i) { return SpreadBuilder::traffic(descs[i], descs[i].comm->n, esize_of(descs[i].dtype)); };
     if (batched) {
-        std::vector<double> bytes(nlevels, 0.0);
+        std::vector<SpreadLoad> load(nlevels);
         p->batch_spread = nlevels > 0;
         for (int i = 0; i < ndesc && p->batch_spread; i++) {
             p->batch_spread = covers(i);
-            bytes[level[i]] += traffic(i);
+            load[level[i]].count(descs[i], descs[i].comm->n, esize_of(descs[i].dtype));
         }
         for (int l = 0; l < nlevels && p->batch_spread; l++) {
             for (int i = 0; i < ndesc; i++)
-                if (level[i] == l) spread[0].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), bytes[l]);
+                if (level[i] == l) spread[0].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), load[l]);
             spread[0].end_level();
         }
     } else {
@@ -537,7 +536,9 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
             const int i = order[k];
             p->plain_spread[k] = covers(i);
             if (!p->plain_spread[k]) continue;
-            spread[k].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), traffic(i));
+            SpreadLoad load;
+            load.count(descs[i], descs[i].comm->n, esize_of(descs[i].dtype));
+            spread[k].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), load);
             spread[k].end_level();
         }
     }
@@ -1053,7 +1054,9 @@ extern "C" int gpumpi_allreduce_noalloc(void* const* sendbufs, void* const* recv
         // form below with its image copied in and its status out, 17 us so).
         SpreadBuilder tiles;
         SpreadParams params;
-        tiles.add(call, nranks, es, SpreadBuilder::traffic(call, nranks, es));
+        SpreadLoad load;
+        load.count(call, nranks, es);
+        tiles.add(call, nranks, es, load);
         tiles.end_level();
         if (tiles.params(&params)) {
             lock.unlock();

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <type_traits>
 
 #include "redop.cuh"
@@ -69,44 +70,88 @@ static __device__ __noinline__ void fan_tile(const SpreadCall& c, u32 tile) {
     }
 }
 
-template <class V>
-static __device__ __noinline__ void copy_tile(const SpreadCall& c, u32 tile) {
-    constexpr int U = 4;
-    const u64 total = (u64)c.ndst * c.nsrc * c.nu;
-    const u64 k1 = min((u64)(tile + 1) * c.per, total);
-    u64 k = (u64)tile * c.per + threadIdx.x;
-    // unit k: row r, block q, unit o of the block; all three advance by SP_T units
-    const u32 nu = (u32)c.nu;
-    const u32 d_o = SP_T % nu, d_q = SP_T / nu % c.nsrc, d_r = SP_T / nu / c.nsrc;
-    const u64 blk = k / nu;
-    u32 o = (u32)(k - blk * nu), r = (u32)(blk / c.nsrc), q = (u32)(blk - (u64)r * c.nsrc);
-    while (k < k1) {
-        V v[U];
-        V* d[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            if (k < k1) {
-                v[u] = ld_unit<V>(ld_ptr(c.src, q) + c.rs * r + (u64)o * sizeof(V));
-                d[u] = reinterpret_cast<V*>(ld_ptr(c.dst, r)) + ((u64)q * nu + o);
-            } else {
-                d[u] = nullptr;
-            }
-            k += SP_T;
-            o += d_o;
-            q += d_q;
-            r += d_r;
-            if (o >= nu) {
-                o -= nu;
-                q++;
-            }
-            if (q >= c.nsrc) {
-                q -= c.nsrc;
-                r++;
-            }
+// Where a thread of a copy tile stands in the sequence of all rows: unit o of
+// block q of row r; next() is SP_T units further.
+struct CopyPos {
+    u32 o, q, r;
+    u32 d_o, d_q, d_r;
+    __device__ __forceinline__ CopyPos(const SpreadCall& c, u64 k) {
+        const u32 nu = (u32)c.nu;
+        const u64 blk = k / nu;
+        o = (u32)(k - blk * nu);
+        r = (u32)(blk / c.nsrc);
+        q = (u32)(blk - (u64)r * c.nsrc);
+        d_o = SP_T % nu;
+        d_q = SP_T / nu % c.nsrc;
+        d_r = SP_T / nu / c.nsrc;
+    }
+    __device__ __forceinline__ void next(u32 nu, u32 nsrc) {
+        o += d_o;
+        q += d_q;
+        r += d_r;
+        if (o >= nu) {
+            o -= nu;
+            q++;
         }
+        if (q >= nsrc) {
+            q -= nsrc;
+            r++;
+        }
+    }
+};
+
+template <class V>
+static __device__ __noinline__ void copy_tile(const SpreadCall& c, u32 tile, char* ring) {
+    const u64 total = (u64)c.ndst * c.nsrc * c.nu;
+    const u64 k0 = (u64)tile * c.per + threadIdx.x;
+    const u64 k1 = min((u64)tile * c.per + c.per, total);
+    const u32 n = k0 < k1 ? (u32)((k1 - k0 + SP_T - 1) / SP_T) : 0;   // this thread's units
+    const u32 nu = (u32)c.nu, nsrc = c.nsrc;
+    const u64 rs = c.rs;
+    const char* const* src = c.src;
+    char* const* dst = c.dst;
+    CopyPos to(c, k0);
+    if constexpr (sizeof(V) >= 4) {
+        // through the thread's own part of the ring, as stream_tile does
+        constexpr u32 GL = 4, NG = SP_RING / (SP_T * sizeof(V)) / GL;
+        const u32 mine = smem_addr(ring) + threadIdx.x * (u32)sizeof(V);
+        const V* slot = reinterpret_cast<const V*>(ring) + threadIdx.x;
+        CopyPos from = to;
+        u32 issued = 0, ig = 0, cg = 0;
+        auto issue = [&]() {
 #pragma unroll
-        for (int u = 0; u < U; u++)
-            if (d[u]) *d[u] = v[u];
+            for (u32 g = 0; g < GL; g++) {
+                if (issued < n) {
+                    cp_async<sizeof(V)>(mine + (ig * GL + g) * (u32)(SP_T * sizeof(V)),
+                                        ld_ptr(src, from.q) + rs * from.r + (u64)from.o * sizeof(V));
+                    issued++;
+                    from.next(nu, nsrc);
+                }
+            }
+            cp_commit();
+            if (++ig == NG) ig = 0;
+        };
+#pragma unroll 1
+        for (u32 g = 0; g < NG - 1; g++) issue();
+        for (u32 k = 0; k < n; k += GL) {
+            issue();
+            cp_wait<NG - 1>();
+#pragma unroll
+            for (u32 g = 0; g < GL; g++) {
+                if (k + g < n) {
+                    reinterpret_cast<V*>(ld_ptr(dst, to.r))[(u64)to.q * nu + to.o] = slot[(cg * GL + g) * SP_T];
+                    to.next(nu, nsrc);
+                }
+            }
+            if (++cg == NG) cg = 0;
+        }
+        cp_wait<0>();
+    } else {
+        for (u32 k = 0; k < n; k++) {
+            reinterpret_cast<V*>(ld_ptr(dst, to.r))[(u64)to.q * nu + to.o] =
+                ld_unit<V>(ld_ptr(src, to.q) + rs * to.r + (u64)to.o * sizeof(V));
+            to.next(nu, nsrc);
+        }
     }
 }
 
@@ -629,11 +674,11 @@ static __device__ void run_tile(const SpreadCall& c, u32 tile, char* smem, Ring&
         }
     } else if (c.kind == SP_COPY) {
         switch (c.ub) {
-            case 16: copy_tile<uint4>(c, tile); break;
-            case 8: copy_tile<uint2>(c, tile); break;
-            case 4: copy_tile<u32>(c, tile); break;
-            case 2: copy_tile<unsigned short>(c, tile); break;
-            default: copy_tile<unsigned char>(c, tile); break;
+            case 16: copy_tile<uint4>(c, tile, smem); break;
+            case 8: copy_tile<uint2>(c, tile, smem); break;
+            case 4: copy_tile<u32>(c, tile, smem); break;
+            case 2: copy_tile<unsigned short>(c, tile, smem); break;
+            default: copy_tile<unsigned char>(c, tile, smem); break;
         }
     } else {
         switch (c.fn & 3) {
@@ -658,11 +703,14 @@ struct Block {
     Ring ring;
 };
 
-// Launches of one stream overlap: the next one may start its blocks as soon as
-// every block of this one runs, and reads its plan's tables meanwhile.  It
-// touches no buffer before grid_wait(): everything the stream ran before it is
-// then complete and visible.  Back to back, an Allreduce of one FP64 value over
-// 16 ranks takes 2.6 us instead of 5.1, ten calls of 64 ranks 147 instead of 161.
+// Launches of one stream overlap: the next one starts its blocks and reads its
+// plan's tables while this one runs, and touches no buffer before grid_wait():
+// everything the stream ran before it is then complete and visible.  A launch
+// lets the next one start once it may run itself, so that no third launch waits
+// in the SMs: with three, blocks went wherever one had just ended, several to
+// one SM (Allreduce of 200 ranks of 50000 FP64 134 us, two launches 78 us).
+// Back to back, an Allreduce of one FP64 value over 16 ranks takes 2.6 us instead
+// of 5.1, ten calls of 64 ranks 135 instead of 153.
 static __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 static __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -702,7 +750,10 @@ static __device__ __forceinline__ void run_tiles(Block& b, const SpreadCall* one
             if (threadIdx.x < W)
                 reinterpret_cast<u64*>(&b.c)[threadIdx.x] = reinterpret_cast<const u64*>(calls + b.found)[threadIdx.x];
         }
-        if (t == blockIdx.x) grid_wait();   // the tables above are the plan's own, the buffers are not
+        if (t == blockIdx.x) {
+            grid_wait();   // the tables above are the plan's own, the buffers are not
+            grid_trigger();
+        }
         __syncthreads();
         if (ptrs) {
             // src and dst are indexes into ptrs
@@ -759,7 +810,6 @@ extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
     extern __shared__ __align__(16) char sp_smem[];
     __shared__ Block b;
     u32 phases = 0;
-    grid_trigger();
     block_begin(b);
     if (blockIdx.x >= A.ntiles) grid_wait();   // no launch ends before the ones it follows
     run_tiles(b, A.ncalls == 1 ? &A.one : nullptr, A.calls, A.ncalls, A.ntiles, sp_smem, phases, A.job);
@@ -773,7 +823,6 @@ extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
     extern __shared__ __align__(16) char sp_smem[];
     __shared__ Block b;
     u32 phases = 0;
-    grid_trigger();
     block_begin(b);
     if (blockIdx.x >= A.ntiles) grid_wait();
     run_tiles(b, nullptr, A.calls, A.ncalls, A.ntiles, sp_smem, phases, nullptr, A.ptrs);
@@ -830,17 +879,17 @@ constexpr u64 SP_PIECE = 1920;       // longest piece: three fit a warp's part o
 
 // Bytes of a rank's vector from which a fold goes by rows instead of gather
 // tiles.  A gather tile's loads are all under way at once, which the fewer
-// warps of a small launch need; rows keep loads under way while they fold,
-// take any alignment in 16-byte units and fill every lane, which counts in
-// large launches and for FP64 (2 additions a clock and SM).  Measured (gather
-// -> rows, us): FP64 Reduce of 64 x 50000 22 -> 16; Allreduce of 48 ranks, 20001
-// FP64 15.1 -> 18.4 and 100001 int32 22.5 -> 18.5; of the 16 communicators of
-// 4..256 ranks, 50001 int32 140 -> 93, 2^14 FP64 86 -> 100, 2^15 FP64 145 -> 121,
-// 2^15 int32 65 -> 70.
-static u64 rows_min(bool aligned, int esize, double total) {
+// warps of a small launch need; rows keep loads under way while they fold and
+// take any alignment in 16-byte units, which counts in large launches.
+// Measured, gather -> rows, us: Allreduce FP64 of 64 ranks, 50000 19.5 -> 27.7,
+// 131072 57.9 -> 50.0, 400000 136 -> 98; 50001 23.0 -> 28.2, 131073 68 -> 50; of
+// 200 ranks, 50000 62 -> 78, 131072 144 -> 140; int32 of 64 ranks, 50001 16.7 ->
+// 15.3, 131073 33 -> 26; of the 16 communicators of 4..256 ranks, 2^15 FP64 151 ->
+// 161, 2^16 234 -> 199, 2^16 int32 113 -> 115, 32769 int32 97 -> 89.
+static u64 rows_min(bool aligned, double total) {
     const bool large = total >= 268435456.0;
-    if (!aligned) return large ? 131072 : 262144;
-    return large || esize == 8 ? 262144 : 524288;
+    if (!aligned) return large ? 131072 : 524288;
+    return large ? 524288 : 1048576;
 }
 
 // Bcast and Allgather by bulk copies: one load of a piece, a store to each of a
@@ -874,20 +923,26 @@ bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
     return true;
 }
 
-double SpreadBuilder::traffic(const gpumpi_coll_desc& d, int P, int esize) {
+void SpreadLoad::count(const gpumpi_coll_desc& d, int P, int esize) {
     const double e = (double)d.count * esize;
     switch (d.op) {
-        case GPUMPI_COLL_BCAST: return e * P;
-        case GPUMPI_COLL_REDUCE: return e * (P + 1);
-        case GPUMPI_COLL_ALLREDUCE: return 2 * e * P;
-        default: return 2 * e * P * P;
+        case GPUMPI_COLL_BCAST: bytes += e * P; break;
+        case GPUMPI_COLL_REDUCE: bytes += e * (P + 1); break;
+        case GPUMPI_COLL_ALLREDUCE: bytes += 2 * e * P; break;
+        default: bytes += 2 * e * P * P;
     }
+    if (is_fold(d.op)) folded += (double)d.count;
 }
 
-void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double total) {
+void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const SpreadLoad& level) {
     if (d.count == 0) return;
-    // traffic of one tile: a few tiles for each of the blocks that run at once
-    const double target = std::min(1048576.0, std::max(16384.0, total / (152.0 * SP_BLOCKS_PER_SM * 2)));
+    // Traffic of one tile: three tiles for each of the blocks that run at once.
+    // Fewer leave blocks idle at the end (2^14 per rank: two 222 us, three 194 us,
+    // four 207 us, six 221 us); a tile starts and ends with its pipeline empty, so
+    // large ones are better (2^20: at most 0.5 MiB 10.18 ms, 1 MiB 9.90, 2 MB 9.79,
+    // 8 MB 9.92).
+    const double total = level.bytes;
+    const double target = std::min(2e6, std::max(16384.0, total / (152.0 * SP_BLOCKS_PER_SM * 3)));
     std::vector<void*> src, dst;
     auto sendbuf = [&](int r) { return d.sendbufs ? d.sendbufs[r] : d.recvbufs[r]; };
     switch (d.op) {
@@ -953,7 +1008,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double tota
             if (hi < n) gather(hi, n - hi, n - hi, n - hi);
             return;
         }
-        if (hi > lo && (hi - lo) * esize >= rows_min(aligned, esize, total)) {
+        if (hi > lo && (hi - lo) * esize >= rows_min(aligned, total)) {
             c.kind = SP_ROWS;
             c.off = lo * esize;
             c.nu = hi - lo;
@@ -971,9 +1026,14 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double tota
             else if (hi < n) gather(hi, n - hi, n - hi, n - hi);
             return;
         }
-        u64 m = (u64)(std::min(target / 2, (double)SP_RING) / ((double)P * esize));
         const u64 step = aligned && n % V == 0 ? V : 1;
-        m = std::max(step, std::min(m, n) / step * step);
+        // A warp's addition takes the same time however many lanes add: fill it as
+        // far as that leaves two tiles for each block (the 16-communicator batch at
+        // 301 per rank 20.7 -> 18.2 us, at 1024 28.7 -> 23.4 us)
+        const double fill = std::min(32.0, std::ceil(level.folded / (152 * SP_BLOCKS_PER_SM * 2)));
+        const double fits = (double)SP_RING / ((double)P * esize);
+        const double per = std::min(fits, std::max(target / 2 / ((double)P * esize), fill));
+        const u64 m = std::max(step, (u64)std::min(per, (double)n) / step * step);
         gather(0, n, m, m);
         return;
     }
@@ -1001,15 +1061,18 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, double tota
     bits |= bytes;
     c.ub = bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
     c.nu = bytes / c.ub;
-    if (c.nu >= 2 * SP_T) {
+    if (!a2a && c.nu >= 2 * SP_T) {
         c.kind = SP_FAN;
-        // a piece: 8 units per thread, more when the launch is large, fewer when the block is short
-        u64 per = 8 * SP_T;
-        if (a2a) per *= (u64)std::max(1.0, target / (2.0 * per * c.ub));
+        // a tile stores 64 KiB and more (256 KiB when the launch is large) to 4 to 8
+        // destinations, less only to give every SM a tile
+        const double stored = std::min(262144.0, std::max(65536.0, target));
+        u64 per = c.ub == 16 && target < 262144.0 ? 4 * SP_T : 8 * SP_T;
+        const double sets = std::min(8.0, std::max(4.0, stored / ((double)per * c.ub)));
+        c.group = (u32)std::min((double)c.ndst, sets);
+        while (per > 2 * SP_T && (double)c.nu * c.nsrc * c.ndst < 152.0 * per * c.group) per /= 2;
         const u64 pieces = (c.nu + per - 1) / per;
         per = ((c.nu + pieces - 1) / pieces + SP_T - 1) / SP_T * SP_T;
         c.per = (u32)per;
-        c.group = a2a ? 1 : (u32)std::max(1.0, std::min((double)c.ndst, target / ((double)per * c.ub)));
         c.ntiles = (u32)((c.nu + per - 1) / per * c.nsrc * ((c.ndst + c.group - 1) / c.group));
     } else {
         c.kind = SP_COPY;

@@ -114,6 +114,13 @@ struct SpreadParams {
     u32 ntiles;
 };
 
+// What the calls of a level amount to.
+struct SpreadLoad {
+    double bytes = 0;     // read and written
+    double folded = 0;    // elements of their folds' results
+    void count(const gpumpi_coll_desc& d, int nranks, int esize);
+};
+
 // Collects the tiles of descriptors for one launch.
 struct SpreadBuilder {
     std::vector<SpreadCall> calls;      // src / dst hold indexes into ptrs until image()
@@ -123,10 +130,8 @@ struct SpreadBuilder {
     // True when the spread form covers the call (schedule and flag rounds left
     // to the runtime, element type with the operator, no NULL buffer).
     static bool covers(const gpumpi_coll_desc& d, int nranks, int esize);
-    // Bytes the call reads and writes.
-    static double traffic(const gpumpi_coll_desc& d, int nranks, int esize);
-    // Append the call's tiles, sized for a level of `total` bytes of traffic.
-    void add(const gpumpi_coll_desc& d, int nranks, int esize, double total);
+    // Append the call's tiles, sized for the level it is part of.
+    void add(const gpumpi_coll_desc& d, int nranks, int esize, const SpreadLoad& level);
     void end_level();
     // Device image (calls, levels, counter, addresses) of bytes() bytes, and the launch arguments.
     size_t bytes() const;
