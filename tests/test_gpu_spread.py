@@ -289,3 +289,77 @@ def test_noalloc_allreduce_matches_the_host(api, p, n, dt, skew):
         assert rc == 0, lib.gpumpi_last_error().decode()
         want = _fold(xs, "sum")
         assert all(row.tobytes() == want.tobytes() for row in recv.rows(dt))
+
+
+@pytest.mark.parametrize("how", ["pinned", "in place", "shared input", "pageable", "captured"])
+def test_host_buffer_calls_in_groups(api, how):
+    """A host-buffer call large enough to copy in, run and copy out in groups
+    gives the bytes that the one-after-another form (flag rounds) gives, call
+    after call with new inputs; also where the groups do not apply: results over
+    the inputs in host memory, two calls filling one device buffer, pageable
+    memory, a stream under capture."""
+    import torch
+
+    coll, lib = api
+    rng = np.random.default_rng(17)
+    shapes = [("allreduce", 16, 20000), ("alltoall", 16, 1300), ("bcast", 16, 20001), ("reduce", 5, 40000),
+              ("allgather", 5, 7001), ("allreduce", 5, 30001)]
+    comms = {p: coll.Comm(lib, p) for p in (16, 5)}
+    kinds = {"allreduce": coll.COLL_ALLREDUCE, "alltoall": coll.COLL_ALLTOALL, "bcast": coll.COLL_BCAST,
+             "reduce": coll.COLL_REDUCE, "allgather": coll.COLL_ALLGATHER}
+    keep, descs, hs, hr, ins, outs = [], [], [], [], [], []
+    first = None
+    for kind, p, n in shapes:
+        ns = n * p if kind == "alltoall" else n
+        nr = n * p if kind in ("alltoall", "allgather") else n
+        dev_in = torch.zeros(p, ns, dtype=torch.float64, device="cuda")
+        if how == "shared input" and kind == "allreduce" and p == 5:
+            dev_in = first            # the Reduce's input, filled twice by one call
+        elif kind == "reduce":
+            first = dev_in
+        dev_out = torch.zeros(p, nr, dtype=torch.float64, device="cuda")
+        host_in = torch.from_numpy(rng.uniform(-1, 1, (p, dev_in.shape[1])))
+        host_out = torch.zeros(p, nr, dtype=torch.float64)
+        if how != "pageable":
+            host_in, host_out = host_in.pin_memory(), host_out.pin_memory()
+        if how == "in place" and ns == nr and kind != "bcast":
+            host_out = host_in
+        keep += [dev_in, dev_out]
+        rows = lambda t, k=p: [t.data_ptr() + r * t.shape[1] * 8 for r in range(k)]  # noqa: E731
+        descs.append(coll.make_desc(comms[p], kinds[kind], "float64", n, None if kind == "bcast" else rows(dev_in),
+                                    rows(dev_out), coll.OP_SUM, p - 1 if kind in ("reduce", "bcast") else 0, keep))
+        hs += rows(host_in)
+        hr += rows(host_out)
+        ins.append(host_in)
+        outs.append(host_out)
+    plan = coll.Plan(lib, descs, threads=64, batched=True)
+    st = torch.cuda.Stream()
+    got = []
+    for mode in (0, 1):
+        plan.set_sync(mode)
+        rng = np.random.default_rng(23)
+        res = []
+        for _ in range(3):
+            for t in ins:
+                t.copy_(torch.from_numpy(rng.uniform(-1, 1, tuple(t.shape))))
+            for t, i in zip(outs, ins):
+                if t is not i:
+                    t.fill_(-3.0)
+            if how == "captured" and mode == 0:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=st):
+                    plan.run_host(hs, hr, st.cuda_stream)
+                graph.replay()
+            else:
+                bi, bo = plan.run_host(hs, hr, st.cuda_stream)
+                assert bi + bo > 4 << 20
+            torch.cuda.synchronize()
+            assert coll.status(lib) is None
+            res.append([t.numpy().copy() for t in outs])
+        got.append(res)
+    plan.close()
+    for c in comms.values():
+        c.close()
+    for a, b in zip(*got):
+        for x, y in zip(a, b):
+            assert x.tobytes() == y.tobytes()
