@@ -568,6 +568,55 @@ __device__ int tiny_stream(int rank, int size) {
     return ok;
 }
 
+// Blocking messages around each size at which the transfer changes (inline
+// words, one batch of vectors, the bulk engine, one stage of it, the eager
+// size), from and into buffers at 16-, 8- and 4-byte offsets, whole and into a
+// longer receive; the bytes around the received ones stay untouched.
+__device__ unsigned char size_byte(int n, int i, int s) { return (unsigned char)(n * 5 + i * 3 + (i >> 8) + s); }
+
+__device__ int sizes(int rank, int size) {
+    const int at[] = {0, 16, 32, 112, 128, 144, 256, 496, 512, 1024, 4080, 4096, 4112, 8192, 16384};
+    const int off[] = {0, 8, 4};
+    const int cap = 16384 + 64;
+    unsigned char* sb = (unsigned char*)malloc(cap);
+    unsigned char* rb = (unsigned char*)malloc(cap);
+    int ok = sb && rb && size >= 2;
+    for (int a = 0; ok && a < (int)(sizeof(at) / sizeof(at[0])); a++)
+        for (int d = -1; d <= 1; d++)
+            for (int o = 0; o < 3; o++) {
+                const int n = at[a] + d;
+                if (n < 0) continue;
+                const int so = off[o], ro = off[(o + (d != 0 ? 1 : 0)) % 3] + 16;
+                if (rank == 0) {
+                    for (int i = 0; i < n; i++) sb[so + i] = size_byte(n, i, 0);
+                    if (MPI_Send(sb + so, n, MPI_BYTE, 1, a, MPI_COMM_WORLD) != MPI_SUCCESS) ok = 0;
+                }
+                if (rank < 2) {
+                    for (int i = 0; i < n + 48; i++) rb[i] = 0xEE;
+                    MPI_Status st;
+                    const int room = n + (o == 2 ? 8 : 0);   // 8 unused bytes behind the message
+                    if (MPI_Recv(rb + ro, room, MPI_BYTE, 1 - rank, a, MPI_COMM_WORLD, &st) != MPI_SUCCESS) ok = 0;
+                    int cnt = -1;
+                    MPI_Get_count(&st, MPI_BYTE, &cnt);
+                    if (cnt != n || st.MPI_SOURCE != 1 - rank || st.MPI_TAG != a) ok = 0;
+                    for (int i = 0; i < n; i++)
+                        if (rb[ro + i] != size_byte(n, i, rank == 0 ? 1 : 0)) ok = 0;
+                    for (int i = 0; i < ro; i++)
+                        if (rb[i] != 0xEE) ok = 0;
+                    for (int i = ro + n; i < n + 48; i++)
+                        if (rb[i] != 0xEE) ok = 0;
+                }
+                if (rank == 1) {
+                    for (int i = 0; i < n; i++) sb[so + i] = size_byte(n, i, 1);
+                    if (MPI_Send(sb + so, n, MPI_BYTE, 0, a, MPI_COMM_WORLD) != MPI_SUCCESS) ok = 0;
+                }
+            }
+    free(sb);
+    free(rb);
+    MPI_Barrier(MPI_COMM_WORLD);
+    return ok;
+}
+
 __device__ int __gpu_main(int argc, char** argv) {
     int rank, size, ok = 0;
     MPI_Init(&argc, &argv);
@@ -590,6 +639,7 @@ __device__ int __gpu_main(int argc, char** argv) {
     else if (!strcmp(s, "split_p2p")) ok = split_p2p(rank, size);
     else if (!strcmp(s, "posted_order")) ok = posted_order(rank, size);
     else if (!strcmp(s, "tiny_stream")) ok = tiny_stream(rank, size);
+    else if (!strcmp(s, "sizes")) ok = sizes(rank, size);
     printf("%s rank %d ok %d\n", s, rank, ok);
     MPI_Finalize();
     return 0;
