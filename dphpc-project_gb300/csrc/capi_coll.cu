@@ -540,6 +540,7 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     const int nlevels = plan_levels(descs, ndesc, level);
     p->independent = nlevels == 1;
     std::vector<SpreadBuilder> spread(batched ? 1 : ndesc);
+    std::vector<char> overlap(ndesc, 0);
     p->plain_spread.assign(ndesc, 0);
     p->plain_tiles.resize(ndesc);
     auto covers = [&](int i) { return SpreadBuilder::covers(descs[i], descs[i].comm->n, esize_of(descs[i].dtype)); };
@@ -564,6 +565,14 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
             load.count(descs[i], descs[i].comm->n, esize_of(descs[i].dtype));
             spread[k].add(descs[i], descs[i].comm->n, esize_of(descs[i].dtype), load);
             spread[k].end_level();
+        }
+        // launch k need not wait for those from k0, the last that does, to k - 1
+        // when they are of one level: calls of a level touch disjoint memory
+        int k0 = 0;
+        for (int k = 0; k < ndesc; k++) {
+            overlap[k] = k > k0 && nlevels > 0 && p->plain_spread[k] && p->plain_spread[k - 1] &&
+                         level[order[k]] == level[order[k0]];
+            if (!overlap[k]) k0 = k;
         }
     }
     size_t total = off_sp;
@@ -633,6 +642,7 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
         SpreadArgs& a = batched ? p->batch_tiles : p->plain_tiles[k];
         spread[k].image(h.data() + at, base + at, &a);
         a.job = g_api.djob;
+        a.overlap = !batched && overlap[k];
         at += spread[k].bytes();
     }
     CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));

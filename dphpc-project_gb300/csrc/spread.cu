@@ -862,9 +862,14 @@ extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
     block_begin(b);
     const SpreadCall* one = A.ncalls == 1 ? &A.one : nullptr;
     first_call(b, one, A.calls, A.ncalls, A.ntiles, sp_smem);
-    grid_wait();   // blocks without a tile too: no launch ends before the ones it follows
+    if (A.overlap) {
+        if (threadIdx.x == 0) __threadfence();   // no line that L1 kept from before the first of them
+    } else {
+        grid_wait();   // blocks without a tile too: no launch ends before the ones it follows
+    }
     grid_trigger();
     run_tiles(b, one, A.calls, A.ncalls, A.ntiles, sp_smem, phases, A.job);
+    if (A.overlap && blockIdx.x == 0) grid_wait();   // no launch ends before the ones it follows
     block_end(b);
 }
 

@@ -102,6 +102,7 @@ struct SpreadArgs {
     u32 ntiles;
     u32 nlevels;
     u32 blocks;                 // more than one level: blocks of the launch
+    u32 overlap;                // touches nothing that the launches since the last one without this mark touch
 };
 
 // A launch whose calls and addresses are parameters of the kernel (4.5 KiB).

@@ -363,3 +363,93 @@ def test_host_buffer_calls_in_groups(api, how):
     for a, b in zip(*got):
         for x, y in zip(a, b):
             assert x.tobytes() == y.tobytes()
+
+
+@pytest.mark.parametrize("n", [17, 60001, 262144])
+def test_plain_launches_without_a_common_buffer_overlap(api, n):
+    """A plain plan's launches wait for one another only where they share
+    memory; they still see what the stream ran before the plan, and what follows
+    the plan sees all of them.  Inputs change and outputs are cleared between
+    the launches, directly and recorded into a graph."""
+    import torch
+
+    coll, lib = api
+    p, q, m, rounds = 6, 3, 500, 6
+    g = torch.Generator().manual_seed(n)
+    n = n // p * p
+    a0 = torch.randint(-1000, 1000, (p, n), dtype=torch.int32, generator=g)
+    d0 = torch.randint(-1000, 1000, (q, m), dtype=torch.int32, generator=g)
+    a, d = torch.zeros_like(a0, device="cuda"), torch.zeros_like(d0, device="cuda")
+    b, c, h = (torch.zeros(p, n, dtype=torch.int32, device="cuda") for _ in range(3))
+    e = torch.zeros(q, m, dtype=torch.int32, device="cuda")
+    f = torch.zeros(q, q * m, dtype=torch.int32, device="cuda")
+    w = torch.zeros(p, n, dtype=torch.int32, device="cuda")
+    big, small = coll.Comm(lib, p), coll.Comm(lib, q)
+    keep = []
+    rows = lambda t: [t.data_ptr() + r * t.shape[1] * 4 for r in range(t.shape[0])]  # noqa: E731
+    plan = coll.Plan(lib, [
+        coll.make_desc(big, coll.COLL_ALLREDUCE, "int32", n, rows(a), rows(b), 2, 0, keep),
+        coll.make_desc(big, coll.COLL_ALLTOALL, "int32", n // p, rows(a), rows(c), 0, 0, keep),
+        coll.make_desc(big, coll.COLL_REDUCE, "int32", n, rows(a), rows(h), 0, 2, keep),
+        coll.make_desc(big, coll.COLL_BCAST, "int32", n, None, rows(w), 0, 1, keep),
+        coll.make_desc(small, coll.COLL_ALLREDUCE, "int32", m, rows(d), rows(e), 2, 0, keep),
+        coll.make_desc(small, coll.COLL_ALLGATHER, "int32", m, rows(e), rows(f), 0, 0, keep),   # uses the one before
+        coll.make_desc(big, coll.COLL_ALLREDUCE, "int32", n, rows(w), rows(c), 2, 0, keep),     # and these two
+        coll.make_desc(big, coll.COLL_ALLREDUCE, "int32", n, rows(h), rows(w), 1, 0, keep),
+    ], threads=64, batched=False)
+    outs = [b, c, h, w, e, f]
+    sums = [torch.zeros_like(t) for t in outs]
+
+    def steps(stream):
+        a.copy_(a0_dev)
+        d.copy_(d0_dev)
+        for s in sums:
+            s.zero_()
+        for k in range(rounds):
+            a.add_(k)
+            d.add_(k)
+            w.copy_(a)
+            plan.launch(stream)
+            for s, t in zip(sums, outs):
+                s.add_(t)
+                t.zero_()
+
+    a0_dev, d0_dev = a0.cuda(), d0.cuda()
+    want = [np.zeros(t.shape, dtype=np.int32) for t in outs]
+    x, y = a0.numpy().copy(), d0.numpy().copy()
+    for k in range(rounds):
+        x, y = x + np.int32(k), y + np.int32(k)
+        hh = np.zeros((p, n), dtype=np.int32)
+        hh[2] = x.max(0)
+        ee = np.tile(y.sum(0, dtype=np.int32), (q, 1))
+        got = [np.tile(x.sum(0, dtype=np.int32), (p, 1)), np.tile(x[1] * np.int32(p), (p, 1)), hh,
+               np.tile(hh.min(0), (p, 1)), ee, np.tile(ee.reshape(-1), (q, 1))]
+        for u, v in zip(want, got):
+            u += v
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def check():
+        torch.cuda.synchronize()
+        assert coll.status(lib) is None
+        for s, u in zip(sums, want):
+            assert np.array_equal(s.cpu().numpy(), u)
+
+    for _ in range(3):
+        with torch.cuda.stream(st):
+            steps(st.cuda_stream)
+        check()
+    plan.capture()
+    with torch.cuda.stream(st):
+        steps(st.cuda_stream)
+    check()
+    plan.set_sync(0)   # drops the plan's own graph
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=st):
+        steps(st.cuda_stream)
+    for _ in range(3):
+        graph.replay()
+        check()
+    plan.close()
+    big.close()
+    small.close()
