@@ -234,7 +234,8 @@ static __device__ __forceinline__ char** dst_table(char* smem) {
 // The call's addresses in shared memory (there already for a block's first
 // tile), or where the host put them when they are many.  The block
 // synchronises before it uses them.
-static __device__ __forceinline__ void tables(const SpreadCall& c, char* smem, const char* const*& st, char* const*& dt) {
+static __device__ __forceinline__ void tables(const SpreadCall& c, char* smem, const char* const*& st,
+                                              char* const*& dt) {
     st = c.src;
     dt = c.dst;
     const char** ts = src_table(smem);
@@ -977,6 +978,36 @@ static u64 fan_min(bool units16, double total) {
     return total >= 1e9 ? 524288 : ~0ull;
 }
 
+// A call that has a level to itself and moves up to this much is cut into one,
+// two or four equal tiles for each SM, which all run at once: no tail, and no
+// more of the 1 to 2 us with which a tile starts (its call, its addresses, the
+// first loads) than it takes to keep loads under way.  Three tiles for each
+// block that fits, as in a level of many calls, leave a tail and are short.
+// Measured with 152, 304, 608 and 1216 tiles for each kind, 4..200 ranks, 0.1 to
+// 200 MB, three tiles -> here, us: Allreduce of 64 ranks of 15616 FP64 10.4 -> 6.4,
+// of 124992 float32 16.6 -> 12.4; of 200 of 4992 FP64 32 -> 12.5; Reduce of 16 of
+// 124992 float32 6.3 -> 3.6; Alltoall of 4 of 1 MB blocks 24.3 -> 8.6, of 64 of
+// 7.8 KB 14.2 -> 8.6; Bcast of 32 MB to 64 ranks 10.5 -> 7.1.  The same for 200 MB
+// (Alltoall 50 -> 36) but not much beyond: large calls want tiles of 2 MB.
+constexpr double SP_LONE_BYTES = 2.5e8;
+constexpr u32 SP_SMS = 152;
+
+static u64 split(u64 units, u64 tiles) { return (units + tiles - 1) / tiles; }
+static u64 round_up(u64 v, u64 step) { return (v + step - 1) / step * step; }
+
+// Elements of a lone fold's gather tile, or 0 when the ring is too small for
+// four tiles for each SM or a thread would fold more than two elements.  One
+// tile for each SM is enough while a thread folds one (64 ranks of 3904 FP64: one
+// 5.1, two 5.2, four 5.4 us; 4 of 62496: 3.3, 3.0, 3.1; 4 of 500000 float32, four
+// tiles 5.3, SP_STREAM 4.6).
+static u64 lone_gather(u64 n, u64 step, u64 fits) {
+    for (u64 k = 1; k <= 4; k *= 2) {
+        const u64 m = round_up(split(n, SP_SMS * k), step);
+        if (m <= fits && m <= (k > 1 ? 2 : 1) * SP_T) return m;
+    }
+    return 0;
+}
+
 static bool is_fold(int op) { return op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE; }
 
 bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
@@ -992,6 +1023,7 @@ bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
 
 void SpreadLoad::count(const gpumpi_coll_desc& d, int P, int esize) {
     const double e = (double)d.count * esize;
+    calls++;
     switch (d.op) {
         case GPUMPI_COLL_BCAST: bytes += e * P; break;
         case GPUMPI_COLL_REDUCE: bytes += e * (P + 1); break;
@@ -1009,7 +1041,9 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     // large ones are better (2^20: at most 0.5 MiB 10.18 ms, 1 MiB 9.90, 2 MB 9.79,
     // 8 MB 9.92).
     const double total = level.bytes;
-    const double target = std::min(2e6, std::max(16384.0, total / (152.0 * SP_BLOCKS_PER_SM * 3)));
+    const bool lone = level.calls == 1 && total <= SP_LONE_BYTES;
+    const double target = lone ? total / (SP_SMS * 2)
+                               : std::min(2e6, std::max(16384.0, total / (SP_SMS * SP_BLOCKS_PER_SM * 3.0)));
     std::vector<void*> src, dst;
     auto sendbuf = [&](int r) { return d.sendbufs ? d.sendbufs[r] : d.recvbufs[r]; };
     switch (d.op) {
@@ -1064,18 +1098,35 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         };
         // whole vectors, or what lies 16 bytes and more from both ends of the buffers
         const u64 lo = aligned ? 0 : V, hi = aligned ? n / V * V : n > 2 * V ? n - V : 0;
-        if (aligned && row * SP_T * 16 <= 2 * target && hi >= SP_T * V) {
+        const u64 step = aligned && n % V == 0 ? V : 1;
+        const double fits = (double)SP_RING / ((double)P * esize);
+        const u64 most = (u64)fits / step * step;   // elements of the largest gather tile
+        const u64 nrows = split(hi / V, SP_T);
+        if (lone) {
+            const u64 m = lone_gather(n, step, most);
+            if (m) {
+                gather(0, n, m, m);
+                return;
+            }
+        }
+        // A lone fold that does not fit streams when that gives two tiles for each
+        // SM (4 ranks of 10^6 FP64: rows 13.7, stream 12.3, gather 14.6 us; 64 of
+        // 62496, 122 rows: 23.0, 19.3, 18.7; 200 of 20000, 39 rows: 52, 52, 26)
+        if (aligned && (lone ? nrows >= 2 * SP_SMS : row * SP_T * 16 <= 2 * target) && hi >= SP_T * V) {
             c.kind = SP_STREAM;
             c.nu = hi;
-            const u64 nrows = (hi / V + SP_T - 1) / SP_T;
             c.per = (u32)std::max(1.0, std::min((double)nrows, target / (row * SP_T * 16)));
+            if (lone) c.per = (u32)split(nrows, 2 * SP_SMS);
             c.ntiles = (u32)((nrows + c.per - 1) / c.per);
             c.tile_bytes = (u32)(row * SP_T * 16 * c.per);
             calls.push_back(c);
             if (hi < n) gather(hi, n - hi, n - hi, n - hi);
             return;
         }
-        if (hi > lo && (hi - lo) * esize >= rows_min(aligned, total)) {
+        // a lone fold of buffers aligned to their elements (4 ranks of 2 * 10^6 int32:
+        // gather 19.4, rows 13.7 us; 64 of 62497 FP64, 500 KB each: 20.0, 24.6 us)
+        if (hi > lo && (lone ? !aligned && (hi - lo) * esize >= 524288
+                             : (hi - lo) * esize >= rows_min(aligned, total))) {
             c.kind = SP_ROWS;
             c.off = lo * esize;
             c.nu = hi - lo;
@@ -1086,6 +1137,13 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
             c.batch = std::min(c.nsrc, SP_PART / (SP_GROUPS * c.ub));
             const u64 chunks = (c.nu + c.per - 1) / c.per;
             c.rows = (u32)std::min((double)chunks, SP_WARPS * std::max(1.0, target / (row * chunk * SP_WARPS)));
+            if (lone) {
+                // two tiles for each SM, or four where each folds many sources in a short
+                // call (two / four: 16 ranks of 500001 int32 16.0 / 14.0 us, of 1562497
+                // 38.5 / 43.5; Reduce of 64 of 390625 33.5 / 30.1)
+                const u32 k = c.nsrc < 16 || (c.nsrc < 32 && total >= 1e8) ? 2 : 4;
+                c.rows = (u32)round_up(split(chunks, k * SP_SMS), SP_WARPS);
+            }
             c.ntiles = (u32)((chunks + c.rows - 1) / c.rows);
             c.tile_bytes = (u32)(row * chunk * c.rows);
             calls.push_back(c);
@@ -1093,12 +1151,19 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
             else if (hi < n) gather(hi, n - hi, n - hi, n - hi);
             return;
         }
-        const u64 step = aligned && n % V == 0 ? V : 1;
+        if (lone) {
+            // two whole waves rather than one and a bit, unless that halves the warps'
+            // additions too (64 ranks of 62496 FP64, 100 elements 21.4, 52 18.7 us; 200
+            // of 124992 float32, 64 elements 40.4, 52 44.5 us)
+            const u64 m = round_up(split(n, 8 * SP_SMS), step);
+            const u64 per = m >= 48 && m <= most ? m : most;
+            gather(0, n, per, per);
+            return;
+        }
         // A warp's addition takes the same time however many lanes add: fill it as
         // far as that leaves two tiles for each block (the 16-communicator batch at
         // 301 per rank 20.7 -> 18.2 us, at 1024 28.7 -> 23.4 us)
         const double fill = std::min(32.0, std::ceil(level.folded / (152 * SP_BLOCKS_PER_SM * 2)));
-        const double fits = (double)SP_RING / ((double)P * esize);
         const double per = std::min(fits, std::max(target / 2 / ((double)P * esize), fill));
         const u64 m = std::max(step, (u64)std::min(per, (double)n) / step * step);
         gather(0, n, m, m);
@@ -1106,8 +1171,32 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     }
     const bool a2a = d.op == GPUMPI_COLL_ALLTOALL;
     c.rs = a2a ? bytes : 0;
-    const bool units16 = (bits | bytes) % 16 == 0;
-    if (bytes >= (a2a ? units16 ? SP_MOVE_ALIGNED : SP_MOVE_BYTES : fan_min(units16, total))) {
+    bits |= bytes;
+    const bool units16 = bits % 16 == 0;
+    c.ub = units16 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
+    bool move = bytes >= (a2a ? units16 ? SP_MOVE_ALIGNED : SP_MOVE_BYTES : fan_min(units16, total));
+    bool fan = !a2a && bytes / c.ub >= 2 * SP_T;
+    u32 even = 2 * SP_SMS;   // tiles of a lone call
+    if (lone && a2a) {
+        // A unit per thread through the deep ring of a few long SP_COPY tiles beats
+        // bulk copies for 8- and 16-byte units at every size, and for 4-byte units
+        // while the call is short (64 ranks, SP_COPY / SP_MOVE: 64 MB 8.6 / 14.3 us,
+        // 16 MB 4.1 / 8.1; 8-byte units 200 MB 42 / 45; 4-byte units of 16 ranks 4 MB
+        // 4.5 / 5.2, of 64 ranks 64 MB 23.8 / 17.1, 200 MB 68 / 45)
+        move = bytes >= SP_MOVE_BYTES && (c.ub < 4 || (c.ub == 4 && total >= 8e6));
+        if (move) even = total < 4e6 ? SP_SMS : total < 3e7 ? 2 * SP_SMS : 4 * SP_SMS;
+    } else if (lone) {
+        // Bulk copies need the call to be large and a few hundred pieces (Allgather of
+        // 64 ranks, 100 MB: SP_MOVE 18.1, SP_FAN 26, SP_COPY 23.5 us; 32 MB 8.7, 9.0, 8.6;
+        // Bcast of 500 KB to 200 ranks, 80 pieces: 26, 20.8, 23).  SP_FAN reads a unit
+        // once for several destinations, which pays once the stores no longer fit the
+        // same few tiles (Bcast of 16-byte units to 16 ranks, SP_FAN / SP_COPY: 8 MB 6.1 /
+        // 4.0 us, 32 MB 7.6 / 8.3; of 8-byte units 8 MB 3.6 / 5.2, 32 MB 7.0 / 12.6).
+        move = total >= 8e7 && bytes >= 2048 && split(bytes, SP_FAN_PIECE) * c.nsrc >= 200;
+        fan = fan && (!units16 || total >= 1.6e7);
+        if (move && units16) even = SP_SMS;
+    }
+    if (move) {
         const u64 longest = a2a ? SP_PIECE : SP_FAN_PIECE;
         c.kind = SP_MOVE;
         c.cold = total >= 1e8;
@@ -1117,19 +1206,41 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         c.per = (u32)(((bytes + pieces - 1) / pieces + step - 1) / step * step);
         c.stages = std::min((u32)SP_MAX_STAGES, SP_PART / (c.per + 32));
         const double sets = units16 ? SP_FAN_ALIGNED : SP_FAN_ODD;
-        c.group = a2a ? 1 : (u32)std::min((double)c.ndst, std::max(1.0, std::min(sets, target / c.per)));
+        const double stored = lone ? total / even : target;
+        c.group = a2a ? 1 : (u32)std::min((double)c.ndst, std::max(1.0, std::min(sets, stored / c.per)));
         const u64 rows = (bytes + c.per - 1) / c.per * c.nsrc * ((c.ndst + c.group - 1) / c.group);
         // at least a row for each warp (8 ranks of 2^17 FP64 11.8 -> 7.4 us)
         c.rows = (u32)std::max(a2a ? (double)SP_WARPS : 1.0, target / ((1.0 + c.group) * c.per));
+        if (lone) c.rows = (u32)split(rows, even);
         c.ntiles = (u32)((rows + c.rows - 1) / c.rows);
         calls.push_back(c);
         return;
     }
-    bits |= bytes;
-    c.ub = bits % 16 == 0 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
     c.nu = bytes / c.ub;
-    if (!a2a && c.nu >= 2 * SP_T) {
+    if (fan) {
         c.kind = SP_FAN;
+        // (shorter calls and larger ones of small units are better off with the sizes
+        // below: Bcast of 8-byte units, 2 MB 2.9 against 3.2 us; of 4-byte units to 200
+        // ranks, 100 MB 23.7 against 27.6)
+        if (lone && total >= 4e6 && (units16 || total < 8e7)) {
+            // The least that the SM with most tiles moves, a tile's start counting as
+            // 20000 bytes (Bcast of 32 MB to 64 ranks, 275 tiles 7.2, 325 tiles 11.3 us)
+            double best = 1e30;
+            for (u32 g = 1; g <= std::min(c.ndst, 16u); g++)
+                for (u64 k = 1; k <= 16; k++) {
+                    const u64 per = std::min(k * SP_T, round_up(c.nu, SP_T));
+                    const u64 tiles = split(c.nu, per) * c.nsrc * split(c.ndst, g);
+                    const double tile = 20000.0 + (double)std::min(per, c.nu) * c.ub * (g + 1);
+                    const double cost = (double)split(tiles, SP_SMS) * tile;
+                    if (cost >= best) continue;
+                    best = cost;
+                    c.group = g;
+                    c.per = (u32)per;
+                    c.ntiles = (u32)tiles;
+                }
+            calls.push_back(c);
+            return;
+        }
         // a tile stores 64 KiB and more (256 KiB when the launch is large) to 4 to 8
         // destinations, less only to give every SM a tile
         const double stored = std::min(262144.0, std::max(65536.0, target));
@@ -1145,6 +1256,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         c.kind = SP_COPY;
         const u64 units = (u64)c.ndst * c.nsrc * c.nu;
         u64 per = SP_T * (u64)std::max(1.0, target / (2.0 * SP_T * c.ub));
+        if (lone) per = round_up(split(units, even), SP_T);
         c.per = (u32)per;
         c.ntiles = (u32)((units + per - 1) / per);
     }

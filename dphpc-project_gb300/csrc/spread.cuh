@@ -117,6 +117,7 @@ struct SpreadParams {
 
 // What the calls of a level amount to.
 struct SpreadLoad {
+    int calls = 0;
     double bytes = 0;     // read and written
     double folded = 0;    // elements of their folds' results
     void count(const gpumpi_coll_desc& d, int nranks, int esize);

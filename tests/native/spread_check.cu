@@ -36,7 +36,8 @@ int main(int argc, char** argv) {
         d.sendbufs = op == 1 ? nullptr : s.data(); d.recvbufs = r.data();
         if (!SpreadBuilder::covers(d, P, es)) continue;
         SpreadLoad lv; lv.count(d, P, es);
-        if (it % 3 == 0) { lv.bytes *= R(1, 200); lv.folded *= R(1, 200); }
+        if (it % 3 == 0) { lv.calls = 2; lv.bytes *= R(1, 200); lv.folded *= R(1, 200); }   // one of several calls of its level
+        if (it % 3 == 1) lv.bytes *= R(1, 30);   // the choices of larger calls
         SpreadBuilder b; b.add(d, P, es, lv); b.end_level();
         if (b.levels[0].ntiles > 3000) continue;
         std::vector<Buf> src, dst;
