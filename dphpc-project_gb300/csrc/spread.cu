@@ -933,15 +933,16 @@ static int fold_type(int dtype) {
     }
 }
 
-// Alltoall blocks from here on move by bulk copies; shorter ones go one unit
-// per thread (SP_COPY) or one unit per thread and block (SP_FAN).  A row costs
-// its warp some 80 instructions whatever its length, a unit per thread some 15
-// each: with 16-byte units the lines cross near 8 KiB (int32 Alltoall of
-// communicators of 4..256 ranks, 2^17 elements per rank: 251 us with bulk
-// copies from 2 KiB, 218 us from 8 KiB; FP64 at 2^20 3.74 ms without them,
-// 2.9 ms with), with 4- or 8-byte units near 512 bytes (int32, 2^12 per rank:
-// 18.3 us from 256 bytes, 15.0 us from 512; 2^20: 1010 us without, 768 us with).
-constexpr u64 SP_MOVE_ALIGNED = 8192;
+// Alltoall blocks from here on move by bulk copies; shorter ones go one unit per
+// thread (SP_COPY).  A row costs its warp some 80 instructions whatever its
+// length, a unit per thread some 15 each, so with units of 4 bytes and more the
+// lines cross near 8 KiB (16-byte units, int32 Alltoall of communicators of 4..256
+// ranks, 2^17 elements per rank: 251 us with bulk copies from 2 KiB, 218 us from 8
+// KiB; FP64 at 2^20 3.74 ms without them, 2.9 ms with.  4- and 8-byte units, the
+// 16-communicator batch, from 512 bytes / 8 KiB: 2^14 per rank 195 / 180 us, 2^15
+// 330 / 318, 30001 370 / 362; no difference to 16 and 32 KiB).  Units of 1 and 2
+// bytes cannot take the ring and do so from 512 bytes.
+constexpr u64 SP_MOVE_UNITS = 8192;
 constexpr u64 SP_MOVE_BYTES = 512;
 constexpr u64 SP_PIECE = 1920;       // longest piece: three fit a warp's part of the ring
 
@@ -1174,7 +1175,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     bits |= bytes;
     const bool units16 = bits % 16 == 0;
     c.ub = units16 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
-    bool move = bytes >= (a2a ? units16 ? SP_MOVE_ALIGNED : SP_MOVE_BYTES : fan_min(units16, total));
+    bool move = bytes >= (a2a ? c.ub >= 4 ? SP_MOVE_UNITS : SP_MOVE_BYTES : fan_min(units16, total));
     bool fan = !a2a && bytes / c.ub >= 2 * SP_T;
     u32 even = 2 * SP_SMS;   // tiles of a lone call
     if (lone && a2a) {
