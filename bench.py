@@ -796,7 +796,7 @@ def main():
                        "diagnostic subset of the batched collectives: " + "+".join(kinds),
                        "elements_per_rank": n, "comm_sizes": COMM_SIZES,
                        "threads_per_rank": threads,
-                       "form": "batched, CUDA graph replay, " + ("launch-ordered (independent calls, no flag rounds)"
+                       "form": "batched, one launch, " + ("launch-ordered (independent calls, no flag rounds)"
                                                                   if ordered else "flag rounds"),
                        "tuning": tuning,
                        "l2": "inputs larger than L2 (each step touches ~%.0f GB)" % (nbytes / 1e9),

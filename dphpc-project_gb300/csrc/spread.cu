@@ -1012,7 +1012,8 @@ static u64 lone_gather(u64 n, u64 step, u64 fits) {
 static bool is_fold(int op) { return op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE; }
 
 bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
-    if (d.algo != 0 || d.sync != 0 || d.op == GPUMPI_COLL_BARRIER || !d.recvbufs || P > SP_MAX_RANKS) return false;
+    if (d.op == GPUMPI_COLL_BARRIER || !d.recvbufs || P > SP_MAX_RANKS) return false;
+    if ((d.algo != 0 && d.algo != tiles_schedule(d.op)) || d.sync != 0) return false;
     if (is_fold(d.op) && fold_type(d.dtype) == FT_NONE) return false;
     auto usable = [&](const void* p) { return p != nullptr && p != MPI_IN_PLACE && (uintptr_t)p % esize == 0; };
     for (int r = 0; r < P; r++) {

@@ -8,8 +8,9 @@
 // to fifteen other communicators, so the batched choice is measured in the
 // batched launch itself: for each co-resident thread count, every descriptor
 // takes its best schedule at that count, the whole list is timed, and at the
-// winning count each (collective, type) group tries every schedule in turn,
-// then flag rounds for its calls (`sync`) in a launch-ordered plan.
+// winning count the list as tiles (spread.cuh), then each (collective, type)
+// group tries every schedule in turn, then flag rounds for its calls (`sync`)
+// in a launch-ordered plan.
 // Timing: two untimed launches, then `reps` launches between CUDA events on
 // a stream of its own.  Plain results are cached, one line per shape, thread
 // count and GPU:
@@ -28,6 +29,7 @@
 
 #include "gpumpi.h"
 #include "hostjob.h"
+#include "spread.cuh"
 
 using namespace gm;
 
@@ -228,6 +230,18 @@ extern "C" int gpumpi_autotune(gpumpi_coll_desc* descs, int ndesc, const gpumpi_
             *out = cand < inc * (1.0 - ADOPT_MARGIN);
             return 0;
         };
+        // every call as tiles: one call with another schedule keeps the whole launch
+        // in rank blocks, so moving one group at a time would not get there
+        if (!rc) {
+            std::vector<int> algo(ndesc), sync(ndesc, 0);
+            for (int i = 0; i < ndesc; i++) algo[i] = tiles_schedule(descs[i].op);
+            double us = 0.0;
+            int adopt = 0;
+            rc = better(algo, sync, &us, &adopt);
+            if (!rc && verbose)
+                fprintf(stderr, "GPUMPI tune: batched as tiles: %.2f us%s\n", us, adopt ? " (adopted)" : "");
+            if (!rc && adopt) best_algo = algo;
+        }
         std::vector<std::pair<int, int>> groups;
         for (int i = 0; i < ndesc && !rc; i++) {
             const std::pair<int, int> g(descs[i].op, descs[i].dtype);

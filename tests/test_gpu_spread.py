@@ -78,7 +78,7 @@ class Buffers:
         return [now[a:a + self.n].copy().view(TYPES[dt][1]) for a in self.at]
 
 
-def _run(api, p, n, dt, op, skew, batched):
+def _run(api, p, n, dt, op, skew, batched, named=False):
     import torch
 
     coll, lib = api
@@ -107,6 +107,8 @@ def _run(api, p, n, dt, op, skew, batched):
          Buffers(torch, p, per * p, dt, 3 * skew))
     call(coll.COLL_ALLGATHER, per, Buffers(torch, p, per, dt, skew, [_values(rng, per, dt) for _ in range(p)]),
          Buffers(torch, p, per * p, dt, 5 * skew))
+    for d in descs if named else []:
+        d.algo = {coll.COLL_BCAST: 1, coll.COLL_REDUCE: 2, coll.COLL_ALLREDUCE: 3}.get(d.op, 4)
     plan = coll.Plan(lib, descs, threads=64, batched=batched)
     assert plan.launch_ordered
     got = []
@@ -150,6 +152,13 @@ def test_short_calls(api, p, n, dt, skew):
 @pytest.mark.parametrize("dt,skew", [("f8", 0), ("f8", 1), ("i4", 0), ("i4", 1), ("u1", 0), ("u1", 1), ("u2", 3)])
 def test_long_calls(api, p, n, dt, skew):
     _run(api, p, n, dt, "max" if dt in ("u1", "u2") else "sum", skew, True)
+
+
+@pytest.mark.parametrize("batched", [True, False])
+@pytest.mark.parametrize("p,n,skew", [(3, 31, 1), (16, 20000, 0), (8, 262149, 1)])
+def test_calls_that_name_the_schedule_of_the_tiles(api, p, n, skew, batched):
+    _run(api, p, n, "f8", "sum", skew, batched, named=True)
+    _run(api, p, n, "u2", "max", skew, batched, named=True)
 
 
 @pytest.mark.parametrize("p,n,skew", [(2, 64, 0), (7, 1001, 1), (48, 20000, 0), (257, 999, 1), (64, 65537, 0)])
