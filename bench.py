@@ -8,8 +8,7 @@ data uniform in [-2^20, 2^20) and FP64 data uniform in [-1, 1), 2^20
 elements per rank (Alltoall: 2^20 / P elements to each peer).
 
 One step = all 96 collective calls.  `value` is algorithmic GB/s of the
-batched form (one persistent cooperative launch, replayed as a CUDA graph),
-with the inputs resident in HBM; algorithmic bytes per call: Bcast P*b,
+batched form (one launch), with the inputs resident in HBM; algorithmic bytes per call: Bcast P*b,
 Allreduce 2*P*n*s, Alltoall 2*P^2*m.  The plain form (one launch per call and
 communicator) runs the same schedules on the same buffers for comparison.
 `e2e` times the host-buffer entry point (host->device copies of every send
@@ -114,9 +113,9 @@ class ClockSampler:
 
 # DRAM bytes (read + write) of one batched launch at 2^16 elements per rank,
 # from a one-pass ncu capture of dram__bytes_read.sum + dram__bytes_write.sum
-# (profiles/gpumpi_plan_kernel_batched_collectives.md); other per-rank counts
+# (profiles/gpumpi_spread_kernel_batched_collectives.md); other per-rank counts
 # scale it by their elements per rank.
-NCU_TRAFFIC_BYTES_2_16 = 1834974208 + 2673922048
+NCU_TRAFFIC_BYTES_2_16 = 1673782528 + 2393776384
 
 
 ALL_KINDS = ("bcast", "allreduce", "alltoall")
@@ -571,7 +570,7 @@ def main():
     stream = torch.cuda.Stream()
     peak, peak_kind = load_peaks()
 
-    # batched form, graph-captured; schedules and thread counts from the autotuner
+    # batched form; schedules and thread counts from the autotuner
     # (it times candidates on these buffers before the timed region)
     kinds = tuple(k for k in ALL_KINDS if k in args.kinds.split(","))
     plan, comms, keep, items, descs = build_plan(coll, lib, torch, COMM_SIZES, n, True, args.threads, kinds=kinds)
@@ -810,7 +809,7 @@ def main():
                          "frac": round(kernel_gbs / peak, 4), "peak_kind": peak_kind,
                          "traffic": int(NCU_TRAFFIC_BYTES_2_16 * n / (1 << 16)) if kinds == ALL_KINDS else None,
                          "traffic_note": ("bytes per launch: ncu DRAM read+write of the same launch at 2^16 "
-                                          "elements per rank (4.51 GB, 1.12x its algorithmic bytes), scaled by "
+                                          "elements per rank (4.07 GB, 1.01x its algorithmic bytes), scaled by "
                                           "elements per rank"),
                          "algorithmic_bytes": int(nbytes)},
             "e2e": {"value": round(e2e_gbs, 3), "unit": "GB/s", "h2d_bytes_per_step": int(h2d),

@@ -1026,7 +1026,8 @@ extern "C" int gpumpi_plan_run_host(gpumpi_plan_t p, void* const* host_send, voi
     if (d2h_bytes) *d2h_bytes = bo;
     // Copies in, launches and copies out of groups of calls on three streams: the
     // link carries both directions at once (three communicators of 128, 88 and 40
-    // ranks, 2^14 elements per rank: 1438 us one after another, 1010 us so; alone, with a wait, 1.80 and 1.31 ms).
+    // ranks, 2^14 elements per rank: 1438 us one after another, 1010 us so; alone,
+    // with a wait, 1.80 and 1.31 ms).
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &capturing));
     if (bi + bo >= PIPE_MIN_BYTES && p->sync_mode == 0 && capturing == cudaStreamCaptureStatusNone) {

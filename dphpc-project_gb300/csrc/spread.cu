@@ -950,8 +950,10 @@ constexpr u64 SP_PIECE = 1920;       // longest piece: three fit a warp's part o
 // tiles.  A gather tile's loads are all under way at once, which the fewer
 // warps of a small launch need; rows keep loads under way while they fold and
 // take any alignment in 16-byte units, which counts in large launches.
-// Measured, gather -> rows, us: Allreduce FP64 of 64 ranks, 50000 19.5 -> 27.7,
-// 131072 57.9 -> 50.0, 400000 136 -> 98; 50001 23.0 -> 28.2, 131073 68 -> 50; of
+// For calls among others, and lone ones above SP_LONE_BYTES.  Measured one call at
+// a time with the tiles of such a level, gather -> rows, us: Allreduce FP64 of 64
+// ranks, 50000 19.5 -> 27.7, 131072 57.9 -> 50.0, 400000 136 -> 98; 50001 23.0 ->
+// 28.2, 131073 68 -> 50; of
 // 200 ranks, 50000 62 -> 78, 131072 144 -> 140; int32 of 64 ranks, 50001 16.7 ->
 // 15.3, 131073 33 -> 26; of the 16 communicators of 4..256 ranks, 2^15 FP64 151 ->
 // 161, 2^16 234 -> 199, 2^16 int32 113 -> 115, 32769 int32 97 -> 89.
@@ -971,7 +973,8 @@ static u64 rows_min(bool aligned, double total) {
 // ranks, 105 MB 21.4 us against 21.9, 210 MB 46.3 against 39.6; to 48 ranks, 50 MB
 // 18.6 against 19.1, 400 MB 83 against 70; odd buffers, 210 MB 21.5 against 36.7
 // and 420 MB 87.5 against 76.5; the 16-communicator batch at 500001 per rank 5364
-// against 5104, at 50001 561 against 565.
+// against 5104, at 50001 561 against 565.  (Lone calls up to SP_LONE_BYTES have
+// their own rule in add().)
 constexpr u64 SP_FAN_PIECE = 6272;
 constexpr double SP_FAN_ALIGNED = 1024, SP_FAN_ODD = 8;
 static u64 fan_min(bool units16, double total) {

@@ -191,6 +191,11 @@ typedef struct gpumpi_comm_s* gpumpi_comm_t;
  *              one bulk asynchronous copy pipeline (cp.async.bulk), 4 the
  *              16-byte vectors of all peer blocks spread over every thread
  *              (launch-ordered plans; elsewhere as 0)
+ * 0, and the schedule that tiles carry out (BCAST 1, REDUCE 2, ALLREDUCE 3,
+ * ALLTOALL and ALLGATHER 4), run as tiles over the whole GPU where the call is
+ * covered: sync 0, at most 3072 ranks, buffers aligned to their elements, and
+ * for the folds an integer, float or double type.  One call of a batched plan
+ * that is not covered keeps the whole launch in rank blocks.
  * gpumpi_autotune fills it in, and `sync` in the batched form. */
 typedef struct gpumpi_coll_desc {
     gpumpi_comm_t comm;
@@ -211,18 +216,23 @@ int gpumpi_comm_create(int nranks, gpumpi_comm_t* comm);
 int gpumpi_comm_destroy(gpumpi_comm_t comm);
 int gpumpi_comm_size(gpumpi_comm_t comm, int* nranks);
 
-/* Plain form: one cooperative kernel launch of comm-size blocks per
- * descriptor; synchronises the stream and reports device errors. */
+/* Plain form: one kernel launch per descriptor (tiles over the whole GPU, or
+ * a cooperative launch of comm-size blocks); synchronises the stream and
+ * reports device errors. */
 int gpumpi_coll_plain(const gpumpi_coll_desc* descs, int ndesc, int threads_per_rank, void* stream);
 
-/* Batched form: every descriptor in one persistent cooperative launch; the
- * blocks of each communicator run that communicator's calls in order.
- * Synchronises the stream and reports device errors. */
+/* Batched form: every descriptor in one launch.  As tiles, calls that use one
+ * another's results run level by level; as rank blocks, the blocks of each
+ * communicator run that communicator's calls in order.  Synchronises the
+ * stream and reports device errors. */
 int gpumpi_coll_batched(const gpumpi_coll_desc* descs, int ndesc, int threads_per_rank, void* stream);
 
 /* Reusable plan of collective calls (descriptors are copied to the device
  * once).  batched = 0: one launch per descriptor; 1: one launch in total.
- * threads_per_rank 0 = 128. */
+ * threads_per_rank 0 = 128 (rank blocks; tiles have their own).  A launch of
+ * tiles may start while the one before it on the stream ends, and plain
+ * launches of calls without a common buffer may run together; none reads or
+ * writes a buffer before what the stream ran ahead of it is complete. */
 typedef struct gpumpi_plan_s* gpumpi_plan_t;
 int gpumpi_plan_create(const gpumpi_coll_desc* descs, int ndesc, int threads_per_rank, int batched,
                        gpumpi_plan_t* plan);
@@ -238,7 +248,9 @@ int gpumpi_plan_launch(gpumpi_plan_t plan, void* stream);
  * launch-ordered form, which needs no flag round between the ranks: the
  * inputs were complete when the launch started and the end of the launch
  * orders the results.  A plain launch holds one call and is always
- * launch-ordered in mode 0.  mode 1: every call synchronises its ranks with
+ * launch-ordered in mode 0.  A batched plan whose calls depend on each other
+ * runs as levels of independent tiles with a barrier of the launch between
+ * two, or, where a call is not covered by tiles, with flag rounds.  mode 1: every call synchronises its ranks with
  * arrive/depart flags, as the device MPI_* calls do.  Drops a captured graph
  * (capture again to replay).  No counterpart in the reference. */
 int gpumpi_plan_set_sync(gpumpi_plan_t plan, int mode);
@@ -246,10 +258,16 @@ int gpumpi_plan_set_sync(gpumpi_plan_t plan, int mode);
 int gpumpi_plan_launch_ordered(gpumpi_plan_t plan);
 /* Capture the plan's launches once as a CUDA graph; later launches replay it
  * on the stream given to gpumpi_plan_launch.  `stream` is not used (the
- * capture runs on a private stream). */
+ * capture runs on a private stream).  A batched plan that is one launch of
+ * independent tiles is left as it is: launched directly it can overlap its
+ * neighbours, which a graph cannot. */
 int gpumpi_plan_capture(gpumpi_plan_t plan, void* stream);
 /* Host-buffer form: per-rank host->device copies of the send data, the plan,
- * device->host copies of the results, all enqueued on one stream.  host_send
+ * device->host copies of the results, ordered on `stream`.  A batched plan of
+ * independent tiles with 4 MiB and more in pinned host memory goes in up to
+ * eight groups of calls on two further streams, joined to `stream` at both
+ * ends, so that one group's results leave while the next one's inputs arrive;
+ * calls on one plan from several threads take turns.  host_send
  * and host_recv list, descriptor by descriptor (creation order), one host
  * pointer per rank; nullptr entries are skipped.  Reports the bytes copied. */
 int gpumpi_plan_run_host(gpumpi_plan_t plan, void* const* host_send, void* const* host_recv,
@@ -283,13 +301,15 @@ int gpumpi_api_status(char* msg, int len);
  * For callers that may not allocate on their call path -- a server that
  * reserved all of HBM at start-up, code under a fixed pooled-allocator
  * budget, or a thread that must not let cudaMalloc/cudaFree synchronise the
- * device.  The runtime's synchronisation state lives in a fixed 64 KiB array
- * in device memory, so nranks is limited to 256 (larger requests fail with
- * GPUMPI_EINVAL).  sendbufs/recvbufs are host arrays of nranks device
+ * device.  Where the call is covered by tiles (see algo) its addresses travel
+ * with the launch; otherwise the runtime's synchronisation state lives in a
+ * fixed 64 KiB array in device memory.  Either way nranks is limited to 256
+ * (larger requests fail with GPUMPI_EINVAL).  sendbufs/recvbufs are host arrays of nranks device
  * pointers; count elements of dtype are reduced with redop in rank order.
  * The first call on a device looks up the array's address (with that device
- * current) and should therefore come before any stream capture.  All calls
- * share the array: calls whose kernels overlap on the GPU race.  The call
+ * current) and should therefore come before any stream capture.  Calls that
+ * are not covered by tiles share the array: if their kernels overlap on the
+ * GPU they race.  The call
  * synchronises `stream` and returns 0 or an error code. */
 int gpumpi_allreduce_noalloc(void* const* sendbufs, void* const* recvbufs, int nranks,
                              uint64_t count, int dtype, int redop, int threads_per_rank,
