@@ -1040,15 +1040,19 @@ void SpreadLoad::count(const gpumpi_coll_desc& d, int P, int esize) {
 
 void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const SpreadLoad& level) {
     if (d.count == 0) return;
-    // Traffic of one tile: three tiles for each of the blocks that run at once.
-    // Fewer leave blocks idle at the end (2^14 per rank: two 222 us, three 194 us,
-    // four 207 us, six 221 us); a tile starts and ends with its pipeline empty, so
-    // large ones are better (2^20: at most 0.5 MiB 10.18 ms, 1 MiB 9.90, 2 MB 9.79,
-    // 8 MB 9.92).
+    // Traffic of one tile in a level of several calls: 1.75 tiles for each of the
+    // blocks that run at once in a short launch, three in a long one.  More of them
+    // even out the end, fewer start less often, each with its pipeline empty (the
+    // 16-communicator batch with 1.25 / 1.75 / 2 / 3 of them, us: 700 per rank 17.4,
+    // 17.5, 20.0, 20.9; 1500 30.1, 28.7, 29.7, 32.3; 4096 60.4, 57.7, 58.0, 62.2; 8192
+    // 117, 103.5, 97.4, 102.0; 16384 218, 178.5, 178.4, 181.4; 24000 367, 297, 272, 261;
+    // 32768 with 2 / 3 / 4 362, 319, 345).  At most 2 MB: 2^20 with 0.5 MiB 10.18 ms, 1
+    // MiB 9.90, 2 MB 9.79, 8 MB 9.92.
     const double total = level.bytes;
     const bool lone = level.calls == 1 && total <= SP_LONE_BYTES;
+    const double waves = total < 3.2e8 ? 1.75 : total < 1.1e9 ? 2 : 3;
     const double target = lone ? total / (SP_SMS * 2)
-                               : std::min(2e6, std::max(16384.0, total / (SP_SMS * SP_BLOCKS_PER_SM * 3.0)));
+                               : std::min(2e6, std::max(16384.0, total / (SP_SMS * SP_BLOCKS_PER_SM * waves)));
     std::vector<void*> src, dst;
     auto sendbuf = [&](int r) { return d.sendbufs ? d.sendbufs[r] : d.recvbufs[r]; };
     switch (d.op) {
