@@ -70,20 +70,19 @@ static __device__ __noinline__ void fan_tile(const SpreadCall& c, u32 tile) {
     }
 }
 
-// Where a thread of a copy tile stands in the sequence of all rows: unit o of
-// block q of row r; next() is SP_T units further.
+// Where a thread of a copy tile stands in the sequence of all rows: item o of
+// block q of row r, each block of nu items; next() is `step` items further.
 struct CopyPos {
     u32 o, q, r;
     u32 d_o, d_q, d_r;
-    __device__ __forceinline__ CopyPos(const SpreadCall& c, u64 k) {
-        const u32 nu = (u32)c.nu;
+    __device__ __forceinline__ CopyPos(u32 nu, u32 nsrc, u64 k, u32 step) {
         const u64 blk = k / nu;
         o = (u32)(k - blk * nu);
-        r = (u32)(blk / c.nsrc);
-        q = (u32)(blk - (u64)r * c.nsrc);
-        d_o = SP_T % nu;
-        d_q = SP_T / nu % c.nsrc;
-        d_r = SP_T / nu / c.nsrc;
+        r = (u32)(blk / nsrc);
+        q = (u32)(blk - (u64)r * nsrc);
+        d_o = step % nu;
+        d_q = step / nu % nsrc;
+        d_r = step / nu / nsrc;
     }
     __device__ __forceinline__ void next(u32 nu, u32 nsrc) {
         o += d_o;
@@ -110,7 +109,7 @@ static __device__ __noinline__ void copy_tile(const SpreadCall& c, u32 tile, cha
     const u64 rs = c.rs;
     const char* const* src = c.src;
     char* const* dst = c.dst;
-    CopyPos to(c, k0);
+    CopyPos to(nu, nsrc, k0, SP_T);
     if constexpr (sizeof(V) >= 4) {
         // through the thread's own part of the ring, as stream_tile does
         constexpr u32 GL = 4, NG = SP_RING / (SP_T * sizeof(V)) / GL;
@@ -153,6 +152,57 @@ static __device__ __noinline__ void copy_tile(const SpreadCall& c, u32 tile, cha
             to.next(nu, nsrc);
         }
     }
+}
+
+// The same for blocks of a few hundred units and more: a warp takes SP_CHUNK units
+// of a block at a time, four of a lane, which share the walk and the addresses.
+// With a unit at a time those were most of the instructions: int32 Alltoall of the
+// 16 communicators at 100003 per rank issued 0.63 instructions a clock and
+// scheduler and reached 55 % of the DRAM rate; alone it takes 160 us so, 182 before.
+template <class V>
+static __device__ __noinline__ void chunk_tile(const SpreadCall& c, u32 tile, char* ring) {
+    constexpr u32 GL = SP_CHUNK / 32, NG = SP_RING / (SP_T * sizeof(V)) / GL;
+    const u32 nu = (u32)c.nu, nsrc = c.nsrc, lane = threadIdx.x & 31;
+    const u32 len = (nu + SP_CHUNK - 1) / SP_CHUNK;   // chunks of a block
+    const u64 total = (u64)c.ndst * nsrc * len;
+    const u64 k0 = (u64)tile * c.per + (threadIdx.x >> 5);
+    const u64 k1 = min((u64)tile * c.per + c.per, total);
+    const u32 n = k0 < k1 ? (u32)((k1 - k0 + SP_WARPS - 1) / SP_WARPS) : 0;   // this warp's
+    const u64 rs = c.rs;
+    const char* const* src = c.src;
+    char* const* dst = c.dst;
+    const u32 mine = smem_addr(ring) + threadIdx.x * (u32)sizeof(V);
+    const V* slot = reinterpret_cast<const V*>(ring) + threadIdx.x;
+    CopyPos to(len, nsrc, k0, SP_WARPS), from = to;
+    u32 issued = 0, ig = 0, cg = 0;
+    auto issue = [&]() {
+        if (issued < n) {
+            const u32 at = from.o * SP_CHUNK + lane;
+            const char* s = ld_ptr(src, from.q) + rs * from.r + (u64)at * sizeof(V);
+#pragma unroll
+            for (u32 g = 0; g < GL; g++)
+                if (at + 32 * g < nu)
+                    cp_async<sizeof(V)>(mine + (ig * GL + g) * (u32)(SP_T * sizeof(V)), s + 32 * g * sizeof(V));
+            issued++;
+            from.next(len, nsrc);
+        }
+        cp_commit();
+        if (++ig == NG) ig = 0;
+    };
+#pragma unroll 1
+    for (u32 g = 0; g < NG - 1; g++) issue();
+    for (u32 k = 0; k < n; k++) {
+        issue();
+        cp_wait<NG - 1>();
+        const u32 at = to.o * SP_CHUNK + lane;
+        V* d = reinterpret_cast<V*>(ld_ptr(dst, to.r)) + (u64)to.q * nu + at;
+#pragma unroll
+        for (u32 g = 0; g < GL; g++)
+            if (at + 32 * g < nu) d[32 * g] = slot[(cg * GL + g) * SP_T];
+        to.next(len, nsrc);
+        if (++cg == NG) cg = 0;
+    }
+    cp_wait<0>();
 }
 
 // Loads of a gather tile: the tile's n units of V of every source, one after
@@ -683,7 +733,9 @@ static __device__ void run_tile(const SpreadCall& c, u32 tile, char* smem, Ring&
             default: fan_tile<unsigned char>(c, tile); break;
         }
     } else if (c.kind == SP_COPY) {
-        switch (c.ub) {
+        switch (c.group ? c.ub + 1 : c.ub) {
+            case 9: chunk_tile<uint2>(c, tile, smem); break;
+            case 5: chunk_tile<u32>(c, tile, smem); break;
             case 16: copy_tile<uint4>(c, tile, smem); break;
             case 8: copy_tile<uint2>(c, tile, smem); break;
             case 4: copy_tile<u32>(c, tile, smem); break;
@@ -1041,7 +1093,8 @@ void SpreadLoad::count(const gpumpi_coll_desc& d, int P, int esize) {
 void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const SpreadLoad& level) {
     if (d.count == 0) return;
     // Traffic of one tile in a level of several calls: 1.75 tiles for each of the
-    // blocks that run at once in a short launch, three in a long one.  More of them
+    // blocks that run at once in a short launch, three in a long one and for a
+    // single large call (Allreduce of 8 ranks, 268 MB: 1.75 48.0, three 46.0 us).  More of them
     // even out the end, fewer start less often, each with its pipeline empty (the
     // 16-communicator batch with 1.25 / 1.75 / 2 / 3 of them, us: 700 per rank 17.4,
     // 17.5, 20.0, 20.9; 1500 30.1, 28.7, 29.7, 32.3; 4096 60.4, 57.7, 58.0, 62.2; 8192
@@ -1050,7 +1103,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     // MiB 9.90, 2 MB 9.79, 8 MB 9.92.
     const double total = level.bytes;
     const bool lone = level.calls == 1 && total <= SP_LONE_BYTES;
-    const double waves = total < 3.2e8 ? 1.75 : total < 1.1e9 ? 2 : 3;
+    const double waves = level.calls == 1 || total >= 1.1e9 ? 3 : total < 3.2e8 ? 1.75 : 2;
     const double target = lone ? total / (SP_SMS * 2)
                                : std::min(2e6, std::max(16384.0, total / (SP_SMS * SP_BLOCKS_PER_SM * waves)));
     std::vector<void*> src, dst;
@@ -1185,14 +1238,22 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     c.ub = units16 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
     bool move = bytes >= (a2a ? c.ub >= 4 ? SP_MOVE_UNITS : SP_MOVE_BYTES : fan_min(units16, total));
     bool fan = !a2a && bytes / c.ub >= 2 * SP_T;
+    // SP_COPY by chunks, where at most a quarter of the lanes' turns is empty: for
+    // 4-byte units (int32 Alltoall of the 16 communicators, 30001 per rank 73.9 ->
+    // 53.4 us, 100003 182 -> 160; the whole batch at 50000 511 -> 505) and lone calls
+    // of 8-byte units (16 ranks, 64 MB 13.2 -> 8.7 us, but FP64 Alltoall of all 16
+    // communicators at 100003 284 -> 296).  16-byte units gain nothing (64 MB 9.4,
+    // 10.1), nor do shorter blocks among other calls (the batch at 301 17.3, 17.6 us).
+    const u64 units = bytes / c.ub;
+    const bool chunks = units >= (lone ? 1 : 4 * SP_CHUNK) && (c.ub == 4 || (lone && c.ub == 8)) &&
+                        round_up(units, SP_CHUNK) * 3 <= units * 4;
     u32 even = 2 * SP_SMS;   // tiles of a lone call
     if (lone && a2a) {
-        // A unit per thread through the deep ring of a few long SP_COPY tiles beats
-        // bulk copies for 8- and 16-byte units at every size, and for 4-byte units
-        // while the call is short (64 ranks, SP_COPY / SP_MOVE: 64 MB 8.6 / 14.3 us,
-        // 16 MB 4.1 / 8.1; 8-byte units 200 MB 42 / 45; 4-byte units of 16 ranks 4 MB
-        // 4.5 / 5.2, of 64 ranks 64 MB 23.8 / 17.1, 200 MB 68 / 45)
-        move = bytes >= SP_MOVE_BYTES && (c.ub < 4 || (c.ub == 4 && total >= 8e6));
+        // The deep ring of a few long SP_COPY tiles beats bulk copies for units of 4
+        // bytes and more (64 ranks, SP_COPY / SP_MOVE: 16-byte units, 16 MB 4.1 / 8.1 us,
+        // 64 MB 8.6 / 14.3; 8-byte units 200 MB 40 / 45; 4-byte units 64 MB 11.1 / 17.1, 200
+        // MB 41 / 45), unless 4-byte units have to go one at a time (64 MB 23.8 / 17.1)
+        move = bytes >= SP_MOVE_BYTES && (c.ub < 4 || (c.ub == 4 && !chunks && total >= 8e6));
         if (move) even = total < 4e6 ? SP_SMS : total < 3e7 ? 2 * SP_SMS : 4 * SP_SMS;
     } else if (lone) {
         // Bulk copies need the call to be large and a few hundred pieces (Allgather of
@@ -1263,11 +1324,13 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         c.ntiles = (u32)((c.nu + per - 1) / per * c.nsrc * ((c.ndst + c.group - 1) / c.group));
     } else {
         c.kind = SP_COPY;
-        const u64 units = (u64)c.ndst * c.nsrc * c.nu;
-        u64 per = SP_T * (u64)std::max(1.0, target / (2.0 * SP_T * c.ub));
-        if (lone) per = round_up(split(units, even), SP_T);
+        c.group = chunks;
+        const u64 item = c.group ? SP_CHUNK : 1, step = SP_T / 32 * (c.group ? 1 : 32);
+        const u64 items = (u64)c.ndst * c.nsrc * split(units, item);
+        u64 per = step * (u64)std::max(1.0, target / (2.0 * step * item * c.ub));
+        if (lone) per = round_up(split(items, even), step);
         c.per = (u32)per;
-        c.ntiles = (u32)((units + per - 1) / per);
+        c.ntiles = (u32)split(items, per);
     }
     calls.push_back(c);
 }
@@ -1276,7 +1339,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
 static double tile_cost(const SpreadCall& c) {
     switch (c.kind) {
         case SP_FAN: return (double)c.per * c.ub * (1 + c.group);
-        case SP_COPY: return 2.0 * c.per * c.ub;
+        case SP_COPY: return 2.0 * c.per * c.ub * (c.group ? SP_CHUNK : 1);
         case SP_MOVE: return (1.0 + c.group) * c.rows * c.per;
         default: return (double)c.tile_bytes;
     }

@@ -34,6 +34,7 @@ constexpr int SP_MAX_RANKS = 3072;   // a gather tile holds 16 bytes of every ra
 constexpr u32 SP_SMEM = SP_RING + 2 * SP_TAB * (u32)sizeof(char*);
 constexpr int SP_WARPS = SP_T / 32;
 constexpr u32 SP_PART = SP_RING / SP_WARPS;   // a warp's part of the ring
+constexpr u32 SP_CHUNK = 128;
 constexpr int SP_MAX_STAGES = 8;
 constexpr int SP_BLOCKS_PER_SM = 4;     // 208 KiB of shared memory, 64 registers a thread
 
@@ -45,7 +46,8 @@ enum SpreadKind : int {
     // whose source block lies `rs` bytes further for each row).
     SP_FAN = 0,
     // The same blocks when they are short: a tile is `per` units of the
-    // sequence of all rows, each loaded and stored by one thread.
+    // sequence of all rows, each loaded and stored by one thread; with `group` 1,
+    // `per` chunks of SP_CHUNK units, each of one block and moved by one warp.
     SP_COPY = 1,
     // Fold of `nu` elements over all sources in rank order, written to every
     // destination.  A tile is `per` elements: the block loads them from all

@@ -52,9 +52,16 @@ int main(int argc, char** argv) {
             CHK(c.first_tile + c.ntiles <= b.levels[0].ntiles, "tiles");
             for (u32 t = 0; t < c.ntiles; t++) {
                 if (c.kind == SP_COPY) {
-                    u64 total = (u64)c.ndst * c.nsrc * c.nu, k1 = std::min<u64>((u64)(t + 1) * c.per, total);
-                    CHK(c.nu < (1ull << 32), "nu");
-                    for (u64 k = (u64)t * c.per; k < k1; k++) { u64 blk = k / c.nu, o = k % c.nu, rr = blk / c.nsrc, q = blk % c.nsrc; rd(q, ps(q) + c.rs * rr + o * c.ub, c.ub); CHK((ps(q) + c.rs * rr + o * c.ub) % c.ub == 0 && (pd(rr) + (q * c.nu + o) * c.ub) % c.ub == 0, "align"); wr(pd(rr), pd(rr) + (q * c.nu + o) * c.ub, c.ub); }
+                    // items: units, or chunks of SP_CHUNK units of one block
+                    CHK(c.nu < (1ull << 32) && (!c.group || c.ub >= 4), "nu");
+                    u64 item = c.group ? SP_CHUNK : 1, len = (c.nu + item - 1) / item;
+                    u64 total = (u64)c.ndst * c.nsrc * len, k1 = std::min<u64>((u64)(t + 1) * c.per, total);
+                    CHK((u64)t * c.per < total, "empty tile");
+                    for (u64 k = (u64)t * c.per; k < k1; k++) {
+                        u64 blk = k / len, o = k % len * item, m = std::min(item, c.nu - o), rr = blk / c.nsrc, q = blk % c.nsrc;
+                        u64 from = ps(q) + c.rs * rr + o * c.ub, to = pd(rr) + (q * c.nu + o) * c.ub;
+                        rd(q, from, m * c.ub); CHK(from % c.ub == 0 && to % c.ub == 0, "align"); wr(pd(rr), to, m * c.ub);
+                    }
                 } else if (c.kind == SP_FAN) {
                     u32 pieces = (u32)((c.nu + c.per - 1) / c.per), piece = t % pieces, rest = t / pieces; u64 q = rest % c.nsrc, r0 = (u64)rest / c.nsrc * c.group, r1 = std::min<u64>(r0 + c.group, c.ndst), o0 = (u64)piece * c.per, o1 = std::min<u64>(o0 + c.per, c.nu);
                     CHK(r0 < c.ndst, "r0"); rd(q, ps(q) + c.rs * r0 + o0 * c.ub, (o1 - o0) * c.ub);

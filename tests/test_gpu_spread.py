@@ -155,6 +155,15 @@ def test_long_calls(api, p, n, dt, skew):
 
 
 @pytest.mark.parametrize("batched", [True, False])
+@pytest.mark.parametrize("per", [95, 96, 128, 129, 171, 512, 513, 2047, 2500])
+@pytest.mark.parametrize("dt", ["i4", "f8"])
+def test_blocks_around_whole_chunks(api, per, dt, batched):
+    """Alltoall and Allgather blocks of 4- and 8-byte units that fill a warp's
+    chunks exactly, just miss them, or are too ragged for them."""
+    _run(api, 5, 5 * per, dt, "sum", 1, batched)
+
+
+@pytest.mark.parametrize("batched", [True, False])
 @pytest.mark.parametrize("p,n,skew", [(3, 31, 1), (16, 20000, 0), (8, 262149, 1)])
 def test_calls_that_name_the_schedule_of_the_tiles(api, p, n, skew, batched):
     _run(api, p, n, "f8", "sum", skew, batched, named=True)
