@@ -646,6 +646,9 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
         at += spread[k].bytes();
     }
     CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));
+    // a copy from pageable memory may return before it has arrived, and launches on
+    // any stream read the tables before they wait for anything
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
     p->ndesc = ndesc;
     p->ncomm = ncomm;
     p->batched = batched;
