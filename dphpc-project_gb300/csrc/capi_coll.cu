@@ -412,6 +412,15 @@ int launch_tiles(const void* kern, void* args, u32 ntiles, cudaStream_t st, bool
     return GPUMPI_OK;
 }
 
+// Held while a plan's launches go to a stream: a plain launch that does not wait
+// for those before it must follow its own plan's, not one that another thread
+// put on the stream between two of them.  Streams share locks by their handles.
+std::mutex& stream_lock(cudaStream_t st) {
+    static std::mutex mu[64];
+    const uintptr_t h = st == cudaStreamLegacy ? 0 : (uintptr_t)st;
+    return mu[(h >> 4 ^ h >> 10) % 64];
+}
+
 int launch_spread(SpreadArgs* args, cudaStream_t st) {
     if (args->nlevels > 1)   // a barrier between levels: every block resident
         return launch((const void*)gpumpi_spread_levels_kernel, (int)args->blocks, SP_T, SP_SMEM, args, st);
@@ -716,6 +725,7 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
 
 static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
     const void* k = (const void*)gpumpi_plan_kernel;
+    std::lock_guard<std::mutex> lock(stream_lock(st));
     if (p->batched) {
         if (p->batch_spread && p->sync_mode == 0) return launch_spread(&p->batch_tiles, st);
         return launch(k, p->total_slots, p->threads, p->smem, &p->batch_args, st);
@@ -987,7 +997,10 @@ int run_pipe(gpumpi_plan_t p, HostPipe& pipe, const std::vector<CopyRun>& in, co
         if (rc) break;
         CK(cudaEventRecord(pipe.arrived[g], pipe.in));
         CK(cudaStreamWaitEvent(st, pipe.arrived[g], 0));
-        rc = launch_tiles((const void*)gpumpi_spread_kernel, &pipe.tiles[g], pipe.tiles[g].ntiles, st, false);
+        {
+            std::lock_guard<std::mutex> turn(stream_lock(st));
+            rc = launch_tiles((const void*)gpumpi_spread_kernel, &pipe.tiles[g], pipe.tiles[g].ntiles, st, false);
+        }
         if (rc) break;
         CK(cudaEventRecord(pipe.ran[g], st));
         CK(cudaStreamWaitEvent(pipe.out, pipe.ran[g], 0));
@@ -1240,7 +1253,11 @@ extern "C" int gpumpi_allreduce_noalloc(void* const* sendbufs, void* const* recv
         tiles.end_level();
         if (tiles.params(&params)) {
             lock.unlock();
-            int rc = launch_tiles((const void*)gpumpi_spread_params_kernel, &params, params.ntiles, st);
+            int rc;
+            {
+                std::lock_guard<std::mutex> turn(stream_lock(st));
+                rc = launch_tiles((const void*)gpumpi_spread_params_kernel, &params, params.ntiles, st);
+            }
             if (rc) return rc;
             CK(cudaStreamSynchronize(st));
             return GPUMPI_OK;

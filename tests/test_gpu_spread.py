@@ -471,3 +471,55 @@ def test_plain_launches_without_a_common_buffer_overlap(api, n):
     plan.close()
     big.close()
     small.close()
+
+
+def test_two_threads_on_one_stream_take_turns(api):
+    """Plain plans of two threads on one stream: each plan's launches stay
+    together, so a launch that does not wait for its own plan's earlier ones
+    still waits for the other thread's.  Each plan writes the buffer that the
+    other one's later launches read; every result must be one plan's or the
+    other's, whole."""
+    import threading
+
+    import torch
+
+    coll, lib = api
+    p, n, rounds = 4, 200000, 150
+    comm = coll.Comm(lib, p)
+    keep = []
+    rows = lambda t: [t.data_ptr() + r * n * 4 for r in range(p)]  # noqa: E731
+    shared = torch.full((p, n), 3, dtype=torch.int32, device="cuda")
+    ins = [torch.full((p, n), v, dtype=torch.int32, device="cuda") for v in (1, 2)]
+    outs = [[torch.zeros(p, n, dtype=torch.int32, device="cuda") for _ in range(2)] for _ in range(2)]
+    plans = []
+    for x, (a, b) in zip(ins, outs):
+        plans.append(coll.Plan(lib, [
+            coll.make_desc(comm, coll.COLL_ALLREDUCE, "int32", n, rows(x), rows(a), 2, 0, keep),
+            coll.make_desc(comm, coll.COLL_ALLREDUCE, "int32", n, rows(shared), rows(b), 2, 0, keep),
+            coll.make_desc(comm, coll.COLL_ALLREDUCE, "int32", n, rows(x), rows(shared), 2, 0, keep),
+        ], threads=64, batched=False))
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def work(k):
+        with torch.cuda.stream(st):
+            for _ in range(rounds):
+                plans[k].launch(st.cuda_stream)
+
+    for _ in range(3):
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        assert coll.status(lib) is None
+        for k in range(2):
+            assert (outs[k][0] == p * (k + 1)).all()
+            b = outs[k][1].cpu().numpy()
+            assert (b == b[0, 0]).all() and b[0, 0] in (3 * p, p * p, 2 * p * p)
+        s = shared.cpu().numpy()
+        assert (s == s[0, 0]).all() and s[0, 0] in (p, 2 * p)
+    for plan in plans:
+        plan.close()
+    comm.close()
