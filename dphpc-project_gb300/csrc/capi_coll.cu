@@ -167,22 +167,27 @@ struct gpumpi_comm_s {
 // The calls of a plan in groups, for host-buffer calls that copy in, run and
 // copy out one group after another on three streams.
 struct HostPipe {
-    bool ok = false;                       // false: no two groups, or calls that share device memory
+    enum State { NEW, READY, NONE } state = NEW;   // NONE: no two groups, or calls that share device memory
     std::vector<std::vector<int>> groups;  // calls (creation order) of each group
     std::vector<SpreadArgs> tiles;
-    char* base = nullptr;                  // device copy of the groups' tile lists
     cudaStream_t in = nullptr, out = nullptr;
     cudaEvent_t begin = nullptr, end = nullptr;
     std::vector<cudaEvent_t> arrived, ran;
-    ~HostPipe() {
+    void drop() {
         for (auto e : arrived) cudaEventDestroy(e);
         for (auto e : ran) cudaEventDestroy(e);
         if (begin) cudaEventDestroy(begin);
         if (end) cudaEventDestroy(end);
         if (in) cudaStreamDestroy(in);
         if (out) cudaStreamDestroy(out);
-        if (base) cudaFree(base);
+        arrived.clear();
+        ran.clear();
+        groups.clear();
+        tiles.clear();
+        begin = end = nullptr;
+        in = out = nullptr;
     }
+    ~HostPipe() { drop(); }
 };
 
 struct gpumpi_plan_s {
@@ -212,7 +217,9 @@ struct gpumpi_plan_s {
     std::vector<char> plain_spread;
     std::vector<SpreadArgs> plain_tiles;
     std::mutex pipe_mu;                    // host-buffer calls of one plan enqueue one after another
-    HostPipe* pipe = nullptr;              // made by the first one
+    HostPipe pipe;                         // filled in by the first one
+    char* pipe_base = nullptr;             // part of `base` for the groups' tile lists
+    size_t pipe_bytes = 0;
 };
 
 namespace {
@@ -287,6 +294,17 @@ void desc_bytes(const gpumpi_coll_desc& d, int P, size_t* in, size_t* out) {
         default: *in = *out = 0;
     }
 }
+
+// Bytes a host-buffer call copies for a descriptor of P ranks, both ways.
+size_t host_bytes(const gpumpi_coll_desc& d, int P, size_t* in, size_t* out) {
+    desc_bytes(d, P, in, out);
+    if (d.op != GPUMPI_COLL_BCAST) *in *= P;
+    if (d.op != GPUMPI_COLL_REDUCE) *out *= P;
+    return *in + *out;
+}
+
+constexpr int PIPE_GROUPS = 8;
+constexpr size_t PIPE_MIN_BYTES = 4u << 20;   // below, the groups' launches and events cost more than the overlap gives
 
 // Levels of the calls of a list: a call is one level above the highest earlier
 // call that it shares memory with, one of the two writing it, so the calls of
@@ -586,8 +604,20 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     }
     size_t total = off_sp;
     for (const SpreadBuilder& b : spread) total += b.bytes() + 64;
-    CK(cudaMalloc(&p->base, total));
+    // Room for the tile lists of a host-buffer call's groups (make_pipe fills it in
+    // with the first of those calls, which therefore allocates no device memory).
+    if (p->batch_spread && nlevels == 1 && ndesc > 1) {
+        size_t moved = 0, in, out, room = 0;
+        for (int i = 0; i < ndesc; i++) {
+            moved += host_bytes(descs[i], descs[i].comm->n, &in, &out);
+            room += SpreadBuilder::max_bytes(descs[i].comm->n);
+        }
+        if (moved >= PIPE_MIN_BYTES) p->pipe_bytes = room + (PIPE_GROUPS + 1) * (SpreadBuilder::max_bytes(0) + 64);
+    }
+    const size_t off_pipe = (total + 63) & ~(size_t)63;
+    CK(cudaMalloc(&p->base, off_pipe + p->pipe_bytes));
     char* base = p->base;
+    p->pipe_base = base + off_pipe;
     std::vector<char> h(total, 0);
     DevDesc* hd = (DevDesc*)(h.data() + off_desc);
     void** hp = (void**)(h.data() + off_ptr);
@@ -889,13 +919,14 @@ int enqueue_copies(const std::vector<CopyRun>& runs, int desc, cudaMemcpyKind ki
     return GPUMPI_OK;
 }
 
-constexpr int PIPE_GROUPS = 8;
-constexpr size_t PIPE_MIN_BYTES = 4u << 20;   // below, the groups' launches and events cost more than the overlap gives
-
 // The groups of a plan, calls with the most output for their input first, so
-// that the way back is busy from the start.
-int make_pipe(gpumpi_plan_t p, HostPipe& pipe, cudaStream_t st) {
-    if (!p->batched || !p->batch_spread || p->batch_tiles.nlevels != 1 || p->ndesc < 2) return GPUMPI_OK;
+// that the way back is busy from the start.  On an error the pipe is as before
+// and the next call tries again.
+int make_pipe(gpumpi_plan_t p, HostPipe& pipe) {
+    if (!p->pipe_bytes) {
+        pipe.state = HostPipe::NONE;
+        return GPUMPI_OK;
+    }
     // the caller's address tables may be gone: the plan's own copies
     std::vector<gpumpi_coll_desc> descs(p->descs);
     for (int i = 0; i < p->ndesc; i++) {
@@ -903,19 +934,17 @@ int make_pipe(gpumpi_plan_t p, HostPipe& pipe, cudaStream_t st) {
         descs[i].recvbufs = p->rb[i].data();
     }
     std::vector<int> level;
-    if (plan_levels(descs.data(), p->ndesc, level, true) != 1) return GPUMPI_OK;
+    if (plan_levels(descs.data(), p->ndesc, level, true) != 1) {
+        pipe.state = HostPipe::NONE;
+        return GPUMPI_OK;
+    }
     std::vector<size_t> in(p->ndesc), out(p->ndesc);
     std::vector<int> order(p->ndesc);
     size_t total = 0;
     for (int i = 0; i < p->ndesc; i++) {
-        const int P = p->descs[i].comm->n;
-        desc_bytes(p->descs[i], P, &in[i], &out[i]);
-        if (p->descs[i].op != GPUMPI_COLL_BCAST) in[i] *= P;
-        if (p->descs[i].op != GPUMPI_COLL_REDUCE) out[i] *= P;
-        total += in[i] + out[i];
+        total += host_bytes(p->descs[i], p->descs[i].comm->n, &in[i], &out[i]);
         order[i] = i;
     }
-    if (total < PIPE_MIN_BYTES) return GPUMPI_OK;
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return in[a] / (out[a] + 1.0) < in[b] / (out[b] + 1.0); });
     size_t held = 0;
@@ -925,7 +954,10 @@ int make_pipe(gpumpi_plan_t p, HostPipe& pipe, cudaStream_t st) {
         held += in[i] + out[i];
         if (held >= total / PIPE_GROUPS) held = 0;
     }
-    if (pipe.groups.size() < 2) return GPUMPI_OK;
+    if (pipe.groups.size() < 2) {
+        pipe.state = HostPipe::NONE;
+        return GPUMPI_OK;
+    }
     std::vector<SpreadBuilder> tiles(pipe.groups.size());
     size_t bytes = 0;
     for (size_t g = 0; g < pipe.groups.size(); g++) {
@@ -935,17 +967,18 @@ int make_pipe(gpumpi_plan_t p, HostPipe& pipe, cudaStream_t st) {
         tiles[g].end_level();
         bytes += (tiles[g].bytes() + 63) & ~(size_t)63;
     }
+    if (bytes > p->pipe_bytes) {   // not reached: max_bytes() bounds every call
+        pipe.state = HostPipe::NONE;
+        return GPUMPI_OK;
+    }
     std::vector<char> image(bytes);
-    CK(cudaMalloc(&pipe.base, bytes));
     pipe.tiles.resize(tiles.size());
     size_t at = 0;
     for (size_t g = 0; g < tiles.size(); g++) {
-        tiles[g].image(image.data() + at, pipe.base + at, &pipe.tiles[g]);
+        tiles[g].image(image.data() + at, p->pipe_base + at, &pipe.tiles[g]);
         pipe.tiles[g].job = g_api.djob;
         at += (tiles[g].bytes() + 63) & ~(size_t)63;
     }
-    // returns once the pageable image has been staged
-    CK(cudaMemcpyAsync(pipe.base, image.data(), bytes, cudaMemcpyHostToDevice, st));
     CK(cudaStreamCreateWithFlags(&pipe.in, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&pipe.out, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&pipe.begin, cudaEventDisableTiming));
@@ -957,7 +990,11 @@ int make_pipe(gpumpi_plan_t p, HostPipe& pipe, cudaStream_t st) {
         CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         pipe.ran.push_back(e);
     }
-    pipe.ok = true;
+    // Ahead of every group's inputs on the stream that brings them, so a launch on
+    // any stream that waits for its inputs waits for its tiles too.  Returns once
+    // the pageable image has been staged.
+    CK(cudaMemcpyAsync(p->pipe_base, image.data(), bytes, cudaMemcpyHostToDevice, pipe.in));
+    pipe.state = HostPipe::READY;
     return GPUMPI_OK;
 }
 
@@ -1048,11 +1085,12 @@ extern "C" int gpumpi_plan_run_host(gpumpi_plan_t p, void* const* host_send, voi
     CK(cudaStreamIsCapturing(st, &capturing));
     if (bi + bo >= PIPE_MIN_BYTES && p->sync_mode == 0 && capturing == cudaStreamCaptureStatusNone) {
         std::lock_guard<std::mutex> lock(p->pipe_mu);
-        if (!p->pipe) {
-            p->pipe = new HostPipe();
-            if (make_pipe(p, *p->pipe, st)) cudaGetLastError();   // not ok: one after another, as below
+        if (p->pipe.state == HostPipe::NEW && make_pipe(p, p->pipe)) {   // one after another, as below
+            cudaGetLastError();
+            p->pipe.drop();
         }
-        if (p->pipe->ok && host_disjoint(to_dev, to_host)) return run_pipe(p, *p->pipe, to_dev, to_host, st);
+        if (p->pipe.state == HostPipe::READY && host_disjoint(to_dev, to_host))
+            return run_pipe(p, p->pipe, to_dev, to_host, st);
     }
     int rc = enqueue_copies(to_dev, -1, cudaMemcpyHostToDevice, st);
     if (!rc) rc = gpumpi_plan_launch(p, stream);
@@ -1064,7 +1102,6 @@ extern "C" int gpumpi_plan_destroy(gpumpi_plan_t p) {
     if (!p) return GPUMPI_EINVAL;
     if (p->exec) cudaGraphExecDestroy(p->exec);
     if (p->graph) cudaGraphDestroy(p->graph);
-    delete p->pipe;
     cudaFree(p->base);
     delete p;
     return GPUMPI_OK;

@@ -1374,6 +1374,11 @@ size_t SpreadBuilder::bytes() const {
            sizeof(void*) * ptrs.size();
 }
 
+size_t SpreadBuilder::max_bytes(int nranks) {
+    if (nranks == 0) return sizeof(u64) * 2 + sizeof(SpreadLevel);
+    return sizeof(SpreadCall) * SP_PARAM_CALLS + sizeof(void*) * 2 * (size_t)nranks;
+}
+
 void SpreadBuilder::image(char* host, char* dev, SpreadArgs* a) {
     const size_t calls_at = sizeof(u64) * 2, levels_at = calls_at + sizeof(SpreadCall) * calls.size(),
                  ptrs_at = levels_at + sizeof(SpreadLevel) * levels.size();

@@ -156,6 +156,8 @@ struct SpreadBuilder {
     void end_level();
     // Device image (calls, levels, counter, addresses) of bytes() bytes, and the launch arguments.
     size_t bytes() const;
+    // At most so many bytes of an image belong to one call; 0 ranks: to the rest of a one-level image.
+    static size_t max_bytes(int nranks);
     void image(char* host, char* dev, SpreadArgs* args);
     // The same as kernel parameters; false when they hold too few ranks.
     bool params(SpreadParams* p) const;

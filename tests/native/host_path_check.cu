@@ -1,0 +1,152 @@
+// Host side of the collective API on a fake CUDA runtime: what it enqueues, in
+// which order, what it allocates and what it leaves behind on errors.
+// Usage: host_path_check SCENARIO
+#include "fake_cuda.h"
+
+#include <chrono>
+#include <functional>
+
+#include "spread.cuh"
+using namespace gm;
+
+static int bad = 0;
+#define CHECK(x, ...)                                \
+    do {                                             \
+        if (!(x)) {                                  \
+            if (bad++ < 10) {                        \
+                printf("failed: %s: ", #x);          \
+                printf(__VA_ARGS__);                 \
+                printf("\n");                        \
+            }                                        \
+        }                                            \
+    } while (0)
+
+// Buffers of the calls of a test and what kernels other than tiles may touch.
+struct Job_ {
+    int P = 4;
+    gpumpi_comm_t comm = nullptr;
+    std::vector<std::vector<void*>> send, recv;
+    std::vector<std::vector<char>> hsend, hrecv;   // pinned, rank by rank
+    std::vector<void*> hs, hr;
+    std::vector<gpumpi_coll_desc> descs;
+    gpumpi_plan_t plan = nullptr;
+};
+static std::vector<fake::Span> g_buffers;   // device buffers of all jobs
+
+static std::vector<fake::Span> kernel_spans(const void* kernel, void** args) {
+    if (kernel != (const void*)gpumpi_spread_kernel) return g_buffers;
+    const SpreadArgs& a = *(const SpreadArgs*)args[0];
+    std::vector<fake::Span> v;
+    for (u32 i = 0; i < a.ncalls; i++) {
+        if (a.ncalls > 1) v.push_back({(const char*)(a.calls + i), sizeof(SpreadCall), false});
+        const SpreadCall& c = a.ncalls == 1 ? a.one : a.calls[i];
+        v.push_back({(const char*)c.src, c.nsrc * sizeof(void*), false});
+        v.push_back({(const char*)c.dst, c.ndst * sizeof(void*), false});
+        for (u32 q = 0; q < c.nsrc; q++) v.push_back({c.src[q] + c.off, 16, false});
+        for (u32 r = 0; r < c.ndst; r++) v.push_back({c.dst[r] + c.off, 16, true});
+    }
+    return v;
+}
+
+// A batched plan of `n` Allreduces of 4 ranks of `count` FP64 elements each, with pinned host buffers.
+static Job_* make(int n, size_t count) {
+    Job_* j = new Job_();
+    CHECK(gpumpi_comm_create(j->P, &j->comm) == 0, "comm");
+    j->send.resize(n);
+    j->recv.resize(n);
+    for (int i = 0; i < n; i++)
+        for (int r = 0; r < 2 * j->P; r++) {
+            void* d = nullptr;
+            cudaMalloc(&d, count * 8);
+            g_buffers.push_back({(char*)d, count * 8, true});
+            (r < j->P ? j->send : j->recv)[i].push_back(d);
+            std::vector<char> h(count * 8, (char)(r + i));
+            (r < j->P ? j->hsend : j->hrecv).push_back(h);
+        }
+    for (auto* side : {&j->hsend, &j->hrecv})
+        for (auto& h : *side) {
+            fake::state().pinned.push_back({h.data(), h.size()});
+            (side == &j->hsend ? j->hs : j->hr).push_back(h.data());
+        }
+    for (int i = 0; i < n; i++) {
+        gpumpi_coll_desc d;
+        memset(&d, 0, sizeof(d));
+        d.comm = j->comm;
+        d.op = GPUMPI_COLL_ALLREDUCE;
+        d.dtype = MPI_DOUBLE;
+        d.redop = GPUMPI_OP_SUM;
+        d.count = count;
+        d.sendbufs = j->send[i].data();
+        d.recvbufs = j->recv[i].data();
+        j->descs.push_back(d);
+    }
+    CHECK(gpumpi_plan_create(j->descs.data(), n, 64, 1, &j->plan) == 0, "plan: %s", gpumpi_last_error());
+    return j;
+}
+static int run_host(Job_* j, cudaStream_t st) {
+    return gpumpi_plan_run_host(j->plan, j->hs.data(), j->hr.data(), st, nullptr, nullptr);
+}
+static cudaStream_t stream() {
+    cudaStream_t st = nullptr;
+    cudaStreamCreateWithFlags(&st, 0);
+    return st;
+}
+static int streams_used(size_t from) {
+    std::set<void*> used;
+    for (size_t i = from; i < fake::state().ops.size(); i++) used.insert(fake::state().ops[i].stream);
+    return (int)used.size();
+}
+
+static const size_t LARGE = 1 << 16, SMALL = 1 << 10;   // elements: 4 MiB and more in 2 calls, less
+
+// A host-buffer call allocates no device memory, and its tile lists have arrived before a launch reads them.
+static void tables() {
+    Job_* j = make(3, LARGE);
+    const size_t from = fake::state().ops.size();
+    const int mallocs = fake::state().mallocs;
+    CHECK(run_host(j, stream()) == 0, "%s", gpumpi_last_error());
+    CHECK(fake::state().mallocs == mallocs, "%d allocations", fake::state().mallocs - mallocs);
+    CHECK(streams_used(from) == 3, "%d streams", streams_used(from));
+    CHECK(fake::races(from) == 0, "races");
+}
+
+// The tile lists have arrived before a launch reads them, also where the first
+// call does not use them (results over its inputs) and the next one is on
+// another stream.
+static bool in_tables(const fake::Span& a) {
+    for (const fake::Span& b : g_buffers)
+        if (a.lo >= b.lo && a.lo < b.lo + b.n) return false;
+    return fake::is_device(a.lo);
+}
+static void uploaded() {
+    Job_* j = make(3, LARGE);
+    const size_t from = fake::state().ops.size();
+    CHECK(gpumpi_plan_run_host(j->plan, j->hs.data(), j->hs.data(), stream(), nullptr, nullptr) == 0, "first");
+    CHECK(run_host(j, stream()) == 0, "%s", gpumpi_last_error());
+    CHECK(streams_used(from) == 4 && fake::races(from, in_tables) == 0, "%d streams", streams_used(from));
+}
+
+// Where the streams of the groups cannot be had, one after another; the next call tries again.
+static void retry() {
+    Job_* j = make(3, LARGE);
+    cudaStream_t st = stream();
+    fake::state().fail = "cudaStreamCreateWithFlags";
+    fake::state().fail_at = fake::state().calls["cudaStreamCreateWithFlags"] + 1;
+    const size_t streams = fake::state().live_streams.size(), events = fake::state().live_events.size();
+    size_t from = fake::state().ops.size();
+    CHECK(run_host(j, st) == 0, "%s", gpumpi_last_error());
+    CHECK(streams_used(from) == 1 && fake::races(from) == 0, "%d streams", streams_used(from));
+    CHECK(fake::state().live_streams.size() == streams && fake::state().live_events.size() <= events + 1, "left behind");
+    from = fake::state().ops.size();
+    CHECK(run_host(j, st) == 0, "%s", gpumpi_last_error());
+    CHECK(streams_used(from) == 3 && fake::races(from) == 0, "%d streams", streams_used(from));
+}
+
+int main(int argc, char** argv) {
+    const std::map<std::string, std::function<void()>> scenarios = {
+        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}};
+    fake::state().kernel_spans = kernel_spans;
+    scenarios.at(argc > 1 ? argv[1] : "")();
+    printf("%s bad %d\n", argv[1], bad);
+    return bad != 0;
+}
