@@ -220,6 +220,10 @@ struct gpumpi_plan_s {
     HostPipe pipe;                         // filled in by the first one
     char* pipe_base = nullptr;             // part of `base` for the groups' tile lists
     size_t pipe_bytes = 0;
+    cudaEvent_t host_done = nullptr;       // end of the last host-buffer call, the next one starts after it
+    ~gpumpi_plan_s() {
+        if (host_done) cudaEventDestroy(host_done);
+    }
 };
 
 namespace {
@@ -1050,6 +1054,14 @@ int run_pipe(gpumpi_plan_t p, HostPipe& pipe, const std::vector<CopyRun>& in, co
     return GPUMPI_OK;
 }
 
+// One after another on one stream.
+int host_enqueue(gpumpi_plan_t p, const std::vector<CopyRun>& in, const std::vector<CopyRun>& out, cudaStream_t st) {
+    int rc = enqueue_copies(in, -1, cudaMemcpyHostToDevice, st);
+    if (!rc) rc = gpumpi_plan_launch(p, st);
+    if (!rc) rc = enqueue_copies(out, -1, cudaMemcpyDeviceToHost, st);
+    return rc;
+}
+
 }  // namespace
 
 extern "C" int gpumpi_plan_run_host(gpumpi_plan_t p, void* const* host_send, void* const* host_recv,
@@ -1077,24 +1089,26 @@ extern "C" int gpumpi_plan_run_host(gpumpi_plan_t p, void* const* host_send, voi
     }
     if (h2d_bytes) *h2d_bytes = bi;
     if (d2h_bytes) *d2h_bytes = bo;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return host_enqueue(p, to_dev, to_host, st);
+    // The calls of a plan share its device buffers: each starts when the one
+    // before it has ended, whatever their streams.
+    std::lock_guard<std::mutex> lock(p->pipe_mu);
+    if (!p->host_done) CK(cudaEventCreateWithFlags(&p->host_done, cudaEventDisableTiming));
+    else CK(cudaStreamWaitEvent(st, p->host_done, 0));
     // Copies in, launches and copies out of groups of calls on three streams: the
     // link carries both directions at once (three communicators of 128, 88 and 40
     // ranks, 2^14 elements per rank: 1438 us one after another, 1010 us so; alone,
     // with a wait, 1.80 and 1.31 ms).
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    CK(cudaStreamIsCapturing(st, &capturing));
-    if (bi + bo >= PIPE_MIN_BYTES && p->sync_mode == 0 && capturing == cudaStreamCaptureStatusNone) {
-        std::lock_guard<std::mutex> lock(p->pipe_mu);
-        if (p->pipe.state == HostPipe::NEW && make_pipe(p, p->pipe)) {   // one after another, as below
-            cudaGetLastError();
-            p->pipe.drop();
-        }
-        if (p->pipe.state == HostPipe::READY && host_disjoint(to_dev, to_host))
-            return run_pipe(p, p->pipe, to_dev, to_host, st);
+    bool piped = bi + bo >= PIPE_MIN_BYTES && p->sync_mode == 0;
+    if (piped && p->pipe.state == HostPipe::NEW && make_pipe(p, p->pipe)) {
+        cudaGetLastError();
+        p->pipe.drop();
     }
-    int rc = enqueue_copies(to_dev, -1, cudaMemcpyHostToDevice, st);
-    if (!rc) rc = gpumpi_plan_launch(p, stream);
-    if (!rc) rc = enqueue_copies(to_host, -1, cudaMemcpyDeviceToHost, st);
+    piped = piped && p->pipe.state == HostPipe::READY && host_disjoint(to_dev, to_host);
+    const int rc = piped ? run_pipe(p, p->pipe, to_dev, to_host, st) : host_enqueue(p, to_dev, to_host, st);
+    CK(cudaEventRecord(p->host_done, st));
     return rc;
 }
 

@@ -142,9 +142,45 @@ static void retry() {
     CHECK(streams_used(from) == 3 && fake::races(from) == 0, "%d streams", streams_used(from));
 }
 
+// Calls of one plan on different streams: each ends before the next one starts.
+static void order() {
+    for (size_t count : {LARGE, SMALL}) {
+        Job_* j = make(3, count);
+        const size_t from = fake::state().ops.size();
+        for (int i = 0; i < 3; i++) CHECK(run_host(j, stream()) == 0, "%s", gpumpi_last_error());
+        CHECK(fake::races(from) == 0, "races of %zu elements", count);
+    }
+}
+
+// Calls of one plan from two threads on one stream do not mix, whatever their form.
+static void turns() {
+    for (size_t count : {LARGE, SMALL}) {
+        Job_* j = make(3, count);
+        cudaStream_t st = stream();
+        const size_t from = fake::state().ops.size();
+        fake::state().pause_us = 200;
+        std::vector<std::thread> threads;
+        for (int t = 0; t < 2; t++)
+            threads.emplace_back([&] {
+                for (int i = 0; i < 3; i++) CHECK(run_host(j, st) == 0, "%s", gpumpi_last_error());
+            });
+        for (auto& t : threads) t.join();
+        fake::state().pause_us = 0;
+        // a call's operations: the same number each, by one thread
+        const std::vector<fake::Op>& ops = fake::state().ops;
+        const size_t each = (ops.size() - from - (count == LARGE)) / 6;   // and the tile lists, with the first
+        for (size_t i = 0; i < 6; i++)
+            for (size_t k = 0; k < each; k++) {
+                const size_t at = from + (count == LARGE) + i * each;
+                CHECK(ops[at + k].thread == ops[at].thread, "call %zu of %zu elements", i, count);
+            }
+        CHECK(fake::races(from) == 0, "races of %zu elements", count);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
-        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}};
+        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}};
     fake::state().kernel_spans = kernel_spans;
     scenarios.at(argc > 1 ? argv[1] : "")();
     printf("%s bad %d\n", argv[1], bad);
