@@ -1027,31 +1027,43 @@ bool host_disjoint(const std::vector<CopyRun>& in, const std::vector<CopyRun>& o
     return true;
 }
 
-int run_pipe(gpumpi_plan_t p, HostPipe& pipe, const std::vector<CopyRun>& in, const std::vector<CopyRun>& out,
-             cudaStream_t st) {
+int pipe_groups(HostPipe& pipe, const std::vector<CopyRun>& in, const std::vector<CopyRun>& out, cudaStream_t st) {
     CK(cudaEventRecord(pipe.begin, st));
     CK(cudaStreamWaitEvent(pipe.in, pipe.begin, 0));
-    int rc = GPUMPI_OK;
-    for (size_t g = 0; g < pipe.groups.size() && !rc; g++) {
+    for (size_t g = 0; g < pipe.groups.size(); g++) {
+        int rc = GPUMPI_OK;
         for (int d : pipe.groups[g])
             if (!rc) rc = enqueue_copies(in, d, cudaMemcpyHostToDevice, pipe.in);
-        if (rc) break;
+        if (rc) return rc;
         CK(cudaEventRecord(pipe.arrived[g], pipe.in));
         CK(cudaStreamWaitEvent(st, pipe.arrived[g], 0));
         {
             std::lock_guard<std::mutex> turn(stream_lock(st));
             rc = launch_tiles((const void*)gpumpi_spread_kernel, &pipe.tiles[g], pipe.tiles[g].ntiles, st, false);
         }
-        if (rc) break;
+        if (rc) return rc;
         CK(cudaEventRecord(pipe.ran[g], st));
         CK(cudaStreamWaitEvent(pipe.out, pipe.ran[g], 0));
         for (int d : pipe.groups[g])
             if (!rc) rc = enqueue_copies(out, d, cudaMemcpyDeviceToHost, pipe.out);
+        if (rc) return rc;
     }
-    if (rc) return rc;
     CK(cudaEventRecord(pipe.end, pipe.out));
     CK(cudaStreamWaitEvent(st, pipe.end, 0));
     return GPUMPI_OK;
+}
+
+int run_pipe(HostPipe& pipe, const std::vector<CopyRun>& in, const std::vector<CopyRun>& out, cudaStream_t st) {
+    const int rc = pipe_groups(pipe, in, out, st);
+    if (!rc) return rc;
+    // copies that are under way still use the caller's memory: the caller, who
+    // knows of `st` only, waits for them there, or here if that cannot be had
+    for (cudaStream_t s : {pipe.in, pipe.out})
+        if (cudaEventRecord(pipe.end, s) != cudaSuccess || cudaStreamWaitEvent(st, pipe.end, 0) != cudaSuccess) {
+            cudaGetLastError();
+            cudaStreamSynchronize(s);
+        }
+    return rc;
 }
 
 // One after another on one stream.
@@ -1107,8 +1119,9 @@ extern "C" int gpumpi_plan_run_host(gpumpi_plan_t p, void* const* host_send, voi
         p->pipe.drop();
     }
     piped = piped && p->pipe.state == HostPipe::READY && host_disjoint(to_dev, to_host);
-    const int rc = piped ? run_pipe(p, p->pipe, to_dev, to_host, st) : host_enqueue(p, to_dev, to_host, st);
-    CK(cudaEventRecord(p->host_done, st));
+    const int rc = piped ? run_pipe(p->pipe, to_dev, to_host, st) : host_enqueue(p, to_dev, to_host, st);
+    if (rc) cudaEventRecord(p->host_done, st);   // the message is that of rc
+    else CK(cudaEventRecord(p->host_done, st));
     return rc;
 }
 

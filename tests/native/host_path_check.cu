@@ -178,9 +178,35 @@ static void turns() {
     }
 }
 
+// A call that fails half way reports it, and nothing that it put on other streams outlives a wait for the caller's.
+static void errors() {
+    int failed = 0;
+    for (const char* what : {"cudaMemcpyAsync", "cudaLaunchKernelExC", "cudaEventRecord", "cudaStreamWaitEvent"}) {
+        Job_* j = make(3, LARGE);
+        cudaStream_t st = stream();
+        CHECK(run_host(j, st) == 0, "%s", gpumpi_last_error());
+        const int first = fake::state().calls[what];
+        CHECK(run_host(j, st) == 0, "%s", gpumpi_last_error());
+        const int n = fake::state().calls[what] - first;
+        for (int k = 0; k < n; k++) {
+            const size_t from = fake::state().ops.size();
+            fake::state().fail = what;
+            fake::state().fail_at = fake::state().calls[what] + k;
+            const int rc = run_host(j, st);
+            fake::state().fail_at = -1;
+            failed += rc != 0;
+            CHECK(rc == GPUMPI_ECUDA, "%s call %d: %d", what, k, rc);
+            const fake::Ops done = fake::state().stream[st] | fake::state().host;
+            for (size_t i = from; i < fake::state().ops.size(); i++) CHECK(done[i], "%s call %d: operation %zu", what, k, i);
+            CHECK(run_host(j, st) == 0 && fake::races(from) == 0, "%s call %d: the next call", what, k);
+        }
+    }
+    CHECK(failed > 30, "%d", failed);
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
-        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}};
+        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}, {"errors", errors}};
     fake::state().kernel_spans = kernel_spans;
     scenarios.at(argc > 1 ? argv[1] : "")();
     printf("%s bad %d\n", argv[1], bad);
