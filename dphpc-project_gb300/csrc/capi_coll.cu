@@ -210,10 +210,10 @@ struct gpumpi_plan_s {
     int independent = 0;                   // calls touch disjoint memory and include no barrier
     int sync_mode = 0;                     // 0 automatic, 1 flag rounds for every call
     std::vector<int> plain_op;             // collective of each plain launch
-    // spread form of the launch-ordered launches (spread.cuh); ntiles 0 in a
-    // launch it does not cover
+    // spread form (spread.cuh) of a batched launch, one launch for each level of
+    // its calls, and of the launch-ordered plain launches that it covers
     bool batch_spread = false;
-    SpreadArgs batch_tiles;
+    std::vector<SpreadArgs> batch_tiles;
     std::vector<char> plain_spread;
     std::vector<SpreadArgs> plain_tiles;
     std::mutex pipe_mu;                    // host-buffer calls of one plan enqueue one after another
@@ -406,8 +406,7 @@ int launch(const void* kern, int grid, int threads, size_t smem, void* args, cud
 }
 
 int spread_attributes() {
-    for (const void* k : {(const void*)gpumpi_spread_kernel, (const void*)gpumpi_spread_levels_kernel,
-                          (const void*)gpumpi_spread_params_kernel}) {
+    for (const void* k : {(const void*)gpumpi_spread_kernel, (const void*)gpumpi_spread_params_kernel}) {
         CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
         CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM));
     }
@@ -444,8 +443,6 @@ std::mutex& stream_lock(cudaStream_t st) {
 }
 
 int launch_spread(SpreadArgs* args, cudaStream_t st) {
-    if (args->nlevels > 1)   // a barrier between levels: every block resident
-        return launch((const void*)gpumpi_spread_levels_kernel, (int)args->blocks, SP_T, SP_SMEM, args, st);
     return launch_tiles((const void*)gpumpi_spread_kernel, args, args->ntiles, st);
 }
 
@@ -616,7 +613,7 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
             moved += host_bytes(descs[i], descs[i].comm->n, &in, &out);
             room += SpreadBuilder::max_bytes(descs[i].comm->n);
         }
-        if (moved >= PIPE_MIN_BYTES) p->pipe_bytes = room + (PIPE_GROUPS + 1) * (SpreadBuilder::max_bytes(0) + 64);
+        if (moved >= PIPE_MIN_BYTES) p->pipe_bytes = room + (PIPE_GROUPS + 1) * 64;
     }
     const size_t off_pipe = (total + 63) & ~(size_t)63;
     CK(cudaMalloc(&p->base, off_pipe + p->pipe_bytes));
@@ -682,10 +679,13 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     size_t at = off_sp;
     for (size_t k = 0; k < spread.size(); k++) {
         at = (at + 63) & ~(size_t)63;
-        SpreadArgs& a = batched ? p->batch_tiles : p->plain_tiles[k];
-        spread[k].image(h.data() + at, base + at, &a);
-        a.job = g_api.djob;
-        a.overlap = !batched && overlap[k];
+        if (batched) p->batch_tiles.resize(spread[k].levels.size());
+        SpreadArgs* a = batched ? p->batch_tiles.data() : &p->plain_tiles[k];
+        spread[k].image(h.data() + at, base + at, a);
+        for (size_t l = 0; l < spread[k].levels.size(); l++) {
+            a[l].job = g_api.djob;
+            a[l].overlap = !batched && overlap[k];
+        }
         at += spread[k].bytes();
     }
     CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));
@@ -728,10 +728,6 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     int per = 0, sms = 0, dev = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (p->batch_spread && nlevels > 1) {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)gpumpi_spread_levels_kernel, SP_T, SP_SMEM));
-        p->batch_tiles.blocks = std::max(1u, std::min((u32)(per * sms), p->batch_tiles.blocks));
-    }
     p->plain_smem.assign(ndesc, rank_smem_bytes(0));
     for (int k = 0; k <= ndesc; k++) {
         // k < ndesc: each plain launch at its own thread count; k == ndesc: the batched launch
@@ -761,7 +757,18 @@ static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
     const void* k = (const void*)gpumpi_plan_kernel;
     std::lock_guard<std::mutex> lock(stream_lock(st));
     if (p->batched) {
-        if (p->batch_spread && p->sync_mode == 0) return launch_spread(&p->batch_tiles, st);
+        if (p->batch_spread && p->sync_mode == 0) {
+            // A launch for each level.  One launch with a barrier of all its blocks
+            // between two levels needs them all on the GPU at once, so it waits for
+            // every kernel that holds some of it, and is slower: five dependent calls
+            // of 4 ranks of 200 FP64 22.7 us, so 11.6; of 48 of 20000 38.4, 28.3; of 200
+            // of 131072 517, 463; 400 calls of 8 ranks of one element 1481, 824.
+            for (SpreadArgs& a : p->batch_tiles) {
+                int rc = launch_spread(&a, st);
+                if (rc) return rc;
+            }
+            return GPUMPI_OK;
+        }
         return launch(k, p->total_slots, p->threads, p->smem, &p->batch_args, st);
     }
     for (int i = 0; i < p->ndesc; i++) {
@@ -778,7 +785,7 @@ extern "C" int gpumpi_plan_launch(gpumpi_plan_t p, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     if (p->exec) {
         CK(cudaGraphLaunch(p->exec, st));
-        g_launches += p->batched ? 1 : p->ndesc;
+        g_launches += !p->batched ? p->ndesc : p->batch_spread && p->sync_mode == 0 ? p->batch_tiles.size() : 1;
         return GPUMPI_OK;
     }
     return plan_enqueue(p, st);
@@ -808,7 +815,7 @@ extern "C" int gpumpi_plan_capture(gpumpi_plan_t p, void* stream) {
     // One launch of independent tiles: replaying it as a graph would keep it from
     // overlapping the launch before it (the 16-communicator batch at 1 element per
     // rank, back to back: 16.4 us as a graph, 12.9 us launched; alone 22.5 and 23.9).
-    if (p->batched && p->batch_spread && p->sync_mode == 0 && p->batch_tiles.nlevels == 1) return GPUMPI_OK;
+    if (p->batched && p->batch_spread && p->sync_mode == 0 && p->batch_tiles.size() == 1) return GPUMPI_OK;
     (void)stream;   // captured on a private stream; replays go to the stream given to gpumpi_plan_launch
     cudaStream_t cap;
     CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));

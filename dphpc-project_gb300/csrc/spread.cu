@@ -691,7 +691,7 @@ static __device__ __noinline__ void move_tile(const SpreadCall& c, u32 tile, cha
         if (i + c.stages < n && !*(volatile u32*)&ring.failed) issue(i + c.stages, stage);
         if (++stage == c.stages) stage = 0;
     }
-    // the results are in global memory before a level ends
+    // the results are in global memory before the launch ends
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.global;" ::: "memory");
 }
@@ -825,10 +825,8 @@ static __device__ __forceinline__ void set_tables(Block& b, void* const* ptrs) {
 
 // The call of this block's first tile and its addresses.  They are the plan's
 // own and do not change, so this runs before the block waits for the launches
-// or the level ahead of it: three dependent loads from L2 that the tile no
-// longer waits for (16 communicators of 4..256 ranks, 301 elements each, 18.8 ->
-// 17.1 us; five dependent calls of 48 ranks 55.6 -> 53.3; ten calls of 64 ranks
-// one after another 132 -> 125).
+// ahead of it: three dependent loads from L2 that the tile no longer waits for
+// (16 communicators of 4..256 ranks, 301 elements each, 18.8 -> 17.1 us).
 static __device__ __forceinline__ void first_call(Block& b, const SpreadCall* one, const SpreadCall* calls, u32 ncalls,
                                                   u32 ntiles, char* smem, void* const* ptrs = nullptr) {
     if (blockIdx.x >= ntiles) return;
@@ -861,46 +859,6 @@ static __device__ __forceinline__ void run_tiles(Block& b, const SpreadCall* one
         run_tile(b.c, t - b.c.first_tile, smem, b.ring, phases, job);
         __syncthreads();
     }
-}
-
-// Every block of the launch has finished its tiles and sees the results of
-// all; between, `ahead` prepares the next level.  `arrived` counts blocks over
-// all barriers of all launches of the plan (each block adds `left` once it
-// gives up, so that the count stays a whole number of barriers).  Returns false
-// when the wait ran out.
-template <class F>
-static __device__ bool grid_barrier(Block& b, u64* arrived, u32 left, Job* job, F ahead) {
-    __syncthreads();
-    u64 old = 0;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        old = atomicAdd(arrived, 1ull);
-    }
-    ahead();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const u64 target = (old / gridDim.x + 1) * gridDim.x;
-        u32 ok = 1;
-        if (ld_acquire(arrived) < target) {
-            const u64 t0 = gtime();
-            for (u32 i = 1; ld_acquire(arrived) < target; i++) {
-                if ((i & 255) == 0 && gtime() - t0 > job->timeout_ns) {
-                    job_fail(job, (int)blockIdx.x, GPUMPI_ERR_TIMEOUT, "a level of a plan did not complete");
-                    atomicAdd(arrived, (u64)left);
-                    ok = 0;
-                    break;
-                }
-            }
-        }
-        __threadfence();
-        b.found = ok;
-    }
-    __syncthreads();
-    const bool ok = b.found != 0;
-    // the next level's bulk loads read what ordinary stores of this level wrote
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    __syncthreads();
-    return ok;
 }
 
 }  // namespace gm
@@ -938,30 +896,6 @@ extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
     grid_wait();
     grid_trigger();
     run_tiles(b, nullptr, A.calls, A.ncalls, A.ntiles, sp_smem, phases, nullptr, A.ptrs);
-    block_end(b);
-}
-
-// Calls that depend on each other: the levels one after another, a barrier of
-// all blocks (a cooperative launch) between two.
-extern "C" __global__ void __launch_bounds__(SP_T, SP_BLOCKS_PER_SM)
-    gpumpi_spread_levels_kernel(const __grid_constant__ SpreadArgs A) {
-    extern __shared__ __align__(16) char sp_smem[];
-    __shared__ Block b;
-    u32 phases = 0;
-    block_begin(b);
-    SpreadLevel L = A.levels[0];
-    first_call(b, nullptr, A.calls + L.first_call, L.ncalls, L.ntiles, sp_smem);
-    grid_wait();
-    grid_trigger();
-    for (u32 l = 0; l < A.nlevels; l++) {
-        run_tiles(b, nullptr, A.calls + L.first_call, L.ncalls, L.ntiles, sp_smem, phases, A.job);
-        if (l + 1 == A.nlevels) break;
-        L = A.levels[l + 1];
-        if (!grid_barrier(b, A.arrived, A.nlevels - 2 - l, A.job, [&]() {
-                first_call(b, nullptr, A.calls + L.first_call, L.ncalls, L.ntiles, sp_smem);
-            }))
-            break;
-    }
     block_end(b);
 }
 
@@ -1369,39 +1303,29 @@ bool SpreadBuilder::params(SpreadParams* p) const {
     return true;
 }
 
-size_t SpreadBuilder::bytes() const {
-    return sizeof(u64) * 2 + sizeof(SpreadCall) * calls.size() + sizeof(SpreadLevel) * levels.size() +
-           sizeof(void*) * ptrs.size();
-}
+size_t SpreadBuilder::bytes() const { return sizeof(SpreadCall) * calls.size() + sizeof(void*) * ptrs.size(); }
 
 size_t SpreadBuilder::max_bytes(int nranks) {
-    if (nranks == 0) return sizeof(u64) * 2 + sizeof(SpreadLevel);
     return sizeof(SpreadCall) * SP_PARAM_CALLS + sizeof(void*) * 2 * (size_t)nranks;
 }
 
-void SpreadBuilder::image(char* host, char* dev, SpreadArgs* a) {
-    const size_t calls_at = sizeof(u64) * 2, levels_at = calls_at + sizeof(SpreadCall) * calls.size(),
-                 ptrs_at = levels_at + sizeof(SpreadLevel) * levels.size();
+void SpreadBuilder::image(char* host, char* dev, SpreadArgs* args) {
+    const size_t ptrs_at = sizeof(SpreadCall) * calls.size();
     for (SpreadCall& c : calls) {
         c.src = (const char* const*)(dev + ptrs_at + (size_t)c.src * sizeof(void*));
         c.dst = (char* const*)(dev + ptrs_at + (size_t)c.dst * sizeof(void*));
     }
-    memset(a, 0, sizeof(*a));
-    memset(host, 0, sizeof(u64) * 2);
     if (!calls.empty()) {
-        a->one = calls[0];
-        memcpy(host + calls_at, calls.data(), sizeof(SpreadCall) * calls.size());
+        memcpy(host, calls.data(), sizeof(SpreadCall) * calls.size());
         memcpy(host + ptrs_at, ptrs.data(), sizeof(void*) * ptrs.size());
     }
-    memcpy(host + levels_at, levels.data(), sizeof(SpreadLevel) * levels.size());
-    a->arrived = (u64*)dev;
-    a->calls = (const SpreadCall*)(dev + calls_at);
-    a->levels = (const SpreadLevel*)(dev + levels_at);
-    a->nlevels = (u32)levels.size();
-    a->ncalls = (u32)calls.size();
-    for (const SpreadLevel& l : levels) {
-        a->ntiles = l.ntiles;
-        a->blocks = std::max(a->blocks, l.ntiles);
+    for (size_t l = 0; l < levels.size(); l++) {
+        SpreadArgs& a = args[l];
+        memset(&a, 0, sizeof(a));
+        if (levels[l].ncalls) a.one = calls[levels[l].first_call];
+        a.calls = (const SpreadCall*)dev + levels[l].first_call;
+        a.ncalls = levels[l].ncalls;
+        a.ntiles = levels[l].ntiles;
     }
 }
 

@@ -88,22 +88,18 @@ struct alignas(16) SpreadCall {
     u32 cold;                   // SP_MOVE to several destinations: the results do not fit L2
 };
 
-// The tiles of a launch, level by level: the calls of a level touch disjoint
-// memory, those of the next may use their results.
+// The tiles of a plan, level by level: the calls of a level touch disjoint
+// memory, those of the next may use their results.  A level is a launch.
 struct SpreadLevel {
-    u32 first_call, ncalls, ntiles, pad;
+    u32 first_call, ncalls, ntiles;
 };
 
 struct SpreadArgs {
     SpreadCall one;             // the call of a launch with a single SpreadCall
     Job* job;                   // error words and the limit of every wait
     const SpreadCall* calls;
-    const SpreadLevel* levels;  // [nlevels], for more than one
-    u64* arrived;               // blocks that reached the end of a level, over all launches
-    u32 ncalls;                 // one level: its calls and tiles
+    u32 ncalls;
     u32 ntiles;
-    u32 nlevels;
-    u32 blocks;                 // more than one level: blocks of the launch
     u32 overlap;                // touches nothing that the launches since the last one without this mark touch
 };
 
@@ -154,10 +150,9 @@ struct SpreadBuilder {
     // Append the call's tiles, sized for the level it is part of.
     void add(const gpumpi_coll_desc& d, int nranks, int esize, const SpreadLoad& level);
     void end_level();
-    // Device image (calls, levels, counter, addresses) of bytes() bytes, and the launch arguments.
+    // Device image (calls, addresses) of bytes() bytes, and the arguments of each level's launch.
     size_t bytes() const;
-    // At most so many bytes of an image belong to one call; 0 ranks: to the rest of a one-level image.
-    static size_t max_bytes(int nranks);
+    static size_t max_bytes(int nranks);   // at most so many of them belong to one call
     void image(char* host, char* dev, SpreadArgs* args);
     // The same as kernel parameters; false when they hold too few ranks.
     bool params(SpreadParams* p) const;
@@ -167,4 +162,3 @@ struct SpreadBuilder {
 
 extern "C" __global__ void gpumpi_spread_kernel(const __grid_constant__ gm::SpreadArgs A);
 extern "C" __global__ void gpumpi_spread_params_kernel(const __grid_constant__ gm::SpreadParams A);
-extern "C" __global__ void gpumpi_spread_levels_kernel(const __grid_constant__ gm::SpreadArgs A);

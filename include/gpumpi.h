@@ -222,13 +222,14 @@ int gpumpi_comm_size(gpumpi_comm_t comm, int* nranks);
 int gpumpi_coll_plain(const gpumpi_coll_desc* descs, int ndesc, int threads_per_rank, void* stream);
 
 /* Batched form: every descriptor in one launch.  As tiles, calls that use one
- * another's results run level by level; as rank blocks, the blocks of each
- * communicator run that communicator's calls in order.  Synchronises the
- * stream and reports device errors. */
+ * another's results run level by level, a launch for each level; as rank
+ * blocks, the blocks of each communicator run that communicator's calls in
+ * order.  Synchronises the stream and reports device errors. */
 int gpumpi_coll_batched(const gpumpi_coll_desc* descs, int ndesc, int threads_per_rank, void* stream);
 
 /* Reusable plan of collective calls (descriptors are copied to the device
- * once).  batched = 0: one launch per descriptor; 1: one launch in total.
+ * once).  batched = 0: one launch per descriptor; 1: one launch in total
+ * (tiles of calls that depend on each other: one for each level).
  * threads_per_rank 0 = 128 (rank blocks; tiles have their own).  A launch of
  * tiles may start while the one before it on the stream ends, and plain
  * launches of calls without a common buffer may run together; none reads or
@@ -249,9 +250,9 @@ int gpumpi_plan_launch(gpumpi_plan_t plan, void* stream);
  * inputs were complete when the launch started and the end of the launch
  * orders the results.  A plain launch holds one call and is always
  * launch-ordered in mode 0.  A batched plan whose calls depend on each other
- * runs as levels of independent tiles with a barrier of the launch between
- * two, or, where a call is not covered by tiles, with flag rounds.  mode 1: every call synchronises its ranks with
- * arrive/depart flags, as the device MPI_* calls do.  Drops a captured graph
+ * runs as levels of independent tiles, one launch after another, or, where a
+ * call is not covered by tiles, with flag rounds.  mode 1: every call
+ * synchronises its ranks with arrive/depart flags, as the device MPI_* calls do.  Drops a captured graph
  * (capture again to replay).  No counterpart in the reference. */
 int gpumpi_plan_set_sync(gpumpi_plan_t plan, int mode);
 /* 1 when the plan's launches run the launch-ordered forms, else 0. */

@@ -204,9 +204,28 @@ static void errors() {
     CHECK(failed > 30, "%d", failed);
 }
 
+// A plan of calls that use each other's results: a launch for each level, none of which needs all its blocks
+// on the GPU at once.
+static void levels() {
+    Job_* j = make(1, SMALL);
+    std::vector<gpumpi_coll_desc> d(5, j->descs[0]);
+    for (int i = 1; i < 5; i += 2) std::swap(d[i].sendbufs, d[i].recvbufs);
+    gpumpi_plan_t p = nullptr;
+    CHECK(gpumpi_plan_create(d.data(), 5, 64, 1, &p) == 0, "%s", gpumpi_last_error());
+    cudaStream_t st = stream();
+    const size_t from = fake::state().ops.size();
+    const uint64_t counted = gpumpi_kernel_launches();
+    CHECK(gpumpi_plan_launch(p, st) == 0, "%s", gpumpi_last_error());
+    CHECK(fake::state().ops.size() - from == 5 && gpumpi_kernel_launches() - counted == 5, "%zu launches",
+          fake::state().ops.size() - from);
+    for (size_t i = from; i < fake::state().ops.size(); i++)
+        CHECK(!fake::state().ops[i].cooperative && fake::state().ops[i].stream == st, "launch %zu", i - from);
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
-        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}, {"errors", errors}};
+        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}, {"errors", errors},
+        {"levels", levels}};
     fake::state().kernel_spans = kernel_spans;
     scenarios.at(argc > 1 ? argv[1] : "")();
     printf("%s bad %d\n", argv[1], bad);

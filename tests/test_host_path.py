@@ -39,7 +39,8 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["tables", "uploaded", "retry", "order", "turns", "errors"])
+@pytest.mark.parametrize("scenario", ["tables", "uploaded", "retry", "order", "turns", "errors",
+                                      "levels"])
 def test_host_path(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr
