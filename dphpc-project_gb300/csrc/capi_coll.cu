@@ -315,12 +315,20 @@ constexpr size_t PIPE_MIN_BYTES = 4u << 20;   // below, the groups' launches and
 // one level touch disjoint memory.  Each call's spans: the bytes each rank
 // reads and writes (Bcast: the root's buffer is read, the others written).
 // Spans of one call never conflict with each other here (in-place forms are
-// the schedules' concern); spans are sorted by start and compared with the
-// spans still open.  Returns the number of levels, or 0 when the list holds a
-// barrier or is too long to be levelled.  One level means that the plan kernel
-// may run every call in its launch-ordered form.  fill_inputs: what a call
-// reads counts as written (a host-buffer call copies it in).
+// the schedules' concern).  Spans are sorted by start and compared with the
+// spans still open, up to the first conflict: lists without one are done.  In
+// the others the spans' ends cut memory into pieces, and each call in turn
+// comes after the last writer of every piece it uses and after the readers
+// since then of every piece it writes.  That takes time in proportion to the
+// spans, where all pairs of conflicting calls take its square (creating a plan
+// of 2000 Allreduces of 256 ranks that ping-pong between two buffers: 7.2 s by
+// pairs, 0.18 s so, 0.11 s when they are independent).  Returns the number of levels, or 0
+// when the list holds a barrier or is too long to be levelled.  One level means
+// that the plan kernel may run every call in its launch-ordered form.
+// fill_inputs: what a call reads counts as written (a host-buffer call copies
+// it in).
 constexpr int MAX_LEVEL_CALLS = 2048;
+constexpr size_t MAX_LEVEL_PIECES = 1u << 26;   // pieces of all spans, 0.2 s
 int plan_levels(const gpumpi_coll_desc* descs, int ndesc, std::vector<int>& level, bool fill_inputs = false) {
     struct Span {
         uintptr_t lo, hi;
@@ -360,29 +368,63 @@ int plan_levels(const gpumpi_coll_desc* descs, int ndesc, std::vector<int>& leve
         }
     }
     std::sort(v.begin(), v.end(), [](const Span& a, const Span& b) { return a.lo < b.lo; });
-    std::vector<std::vector<char>> after;   // after[i][j], j < i: call i comes after call j
+    level.assign(ndesc, 0);
+    bool conflict = false;
     std::vector<Span> open;
-    for (const Span& x : v) {
+    for (size_t i = 0; i < v.size() && !conflict; i++) {
+        const Span& x = v[i];
         size_t k = 0;
         for (size_t j = 0; j < open.size(); j++)
             if (open[j].hi > x.lo) open[k++] = open[j];
         open.resize(k);
-        for (const Span& o : open) {
-            if (o.call == x.call || !(o.w || x.w)) continue;
-            if (ndesc > MAX_LEVEL_CALLS) return 0;
-            if (after.empty()) after.resize(ndesc);
-            const int i = std::max(o.call, x.call), j = std::min(o.call, x.call);
-            if (after[i].empty()) after[i].assign(i, 0);
-            after[i][j] = 1;
-        }
+        for (const Span& o : open) conflict = conflict || (o.call != x.call && (o.w || x.w));
         open.push_back(x);
     }
-    level.assign(ndesc, 0);
+    if (!conflict) return 1;
+    if (ndesc > MAX_LEVEL_CALLS) return 0;
+    // where pieces start and end; most spans are those of other calls again
+    std::vector<uintptr_t> cut;
+    for (size_t i = 0; i < v.size(); i++) {
+        if (i == 0 || v[i].lo != v[i - 1].lo) cut.push_back(v[i].lo);
+        if (i == 0 || v[i].lo != v[i - 1].lo || v[i].hi != v[i - 1].hi) cut.push_back(v[i].hi);
+    }
+    std::sort(cut.begin(), cut.end());
+    cut.erase(std::unique(cut.begin(), cut.end()), cut.end());
+    struct Pieces {
+        u32 first, end;
+        int w;
+    };
+    std::vector<size_t> first(ndesc + 1, 0);   // of each call's spans
+    for (const Span& x : v) first[x.call + 1]++;
+    for (int i = 0; i < ndesc; i++) first[i + 1] += first[i];
+    std::vector<size_t> next(first.begin(), first.end() - 1);
+    std::vector<Pieces> spans(v.size());
+    size_t lo = 0, pieces = 0;
+    for (const Span& x : v) {
+        while (cut[lo] != x.lo) lo++;
+        const size_t hi = cut[lo + 1] == x.hi ? lo + 1 : std::lower_bound(cut.begin() + lo, cut.end(), x.hi) - cut.begin();
+        pieces += hi - lo;
+        spans[next[x.call]++] = {(u32)lo, (u32)hi, x.w};
+    }
+    if (pieces > MAX_LEVEL_PIECES) return 0;
+    struct Piece {
+        int written = 0, read = 0;   // level + 1 of its last writer and of its readers since
+    };
+    std::vector<Piece> piece(cut.size());
     int n = 1;
-    for (size_t i = 0; i < after.size(); i++) {
-        for (size_t j = 0; j < after[i].size(); j++)
-            if (after[i][j]) level[i] = std::max(level[i], level[j] + 1);
-        n = std::max(n, level[i] + 1);
+    for (int i = 0; i < ndesc; i++) {
+        int l = 0;
+        for (size_t k = first[i]; k < first[i + 1]; k++)
+            for (u32 c = spans[k].first; c < spans[k].end; c++)
+                l = std::max(l, spans[k].w ? std::max(piece[c].written, piece[c].read) : piece[c].written);
+        for (int w : {0, 1})
+            for (size_t k = first[i]; k < first[i + 1]; k++)
+                for (u32 c = spans[k].first; spans[k].w == w && c < spans[k].end; c++) {
+                    if (w) piece[c] = {l + 1, 0};
+                    else piece[c].read = std::max(piece[c].read, l + 1);
+                }
+        level[i] = l;
+        n = std::max(n, l + 1);
     }
     return n;
 }

@@ -33,9 +33,17 @@ struct Job_ {
 };
 static std::vector<fake::Span> g_buffers;   // device buffers of all jobs
 
+typedef std::set<std::pair<const void*, const void*>> CallSet;
+static std::vector<CallSet> g_launched;   // the calls of each launch, by their first rank's buffers
+
 static std::vector<fake::Span> kernel_spans(const void* kernel, void** args) {
     if (kernel != (const void*)gpumpi_spread_kernel) return g_buffers;
     const SpreadArgs& a = *(const SpreadArgs*)args[0];
+    g_launched.emplace_back();
+    for (u32 i = 0; i < a.ncalls; i++) {
+        const SpreadCall& c = a.ncalls == 1 ? a.one : a.calls[i];
+        g_launched.back().insert({c.src[0], c.dst[0]});
+    }
     std::vector<fake::Span> v;
     for (u32 i = 0; i < a.ncalls; i++) {
         if (a.ncalls > 1) v.push_back({(const char*)(a.calls + i), sizeof(SpreadCall), false});
@@ -222,10 +230,92 @@ static void levels() {
         CHECK(!fake::state().ops[i].cooperative && fake::state().ops[i].stream == st, "launch %zu", i - from);
 }
 
+// The levels of random lists of Allreduces over one piece of memory: as few as their conflicts allow.
+static void random_levels() {
+    unsigned long long x = 12345;
+    auto rnd = [&](int n) { return (int)((x = x * 6364136223846793005ull + 1442695040888963407ull) >> 33) % n; };
+    void* mem = nullptr;
+    cudaMalloc(&mem, 1 << 16);
+    gpumpi_comm_t comm = nullptr;
+    CHECK(gpumpi_comm_create(2, &comm) == 0, "comm");
+    for (int it = 0; it < 300; it++) {
+        const int n = 1 + rnd(12), room = 8 << rnd(9);
+        std::vector<std::vector<void*>> at(2 * n);
+        std::vector<gpumpi_coll_desc> d(n);
+        for (int i = 0; i < n; i++) {
+            memset(&d[i], 0, sizeof(d[i]));
+            d[i].comm = comm;
+            d[i].op = GPUMPI_COLL_ALLREDUCE;
+            d[i].dtype = MPI_DOUBLE;
+            d[i].redop = GPUMPI_OP_SUM;
+            d[i].count = 1 + rnd(1 + room / 8);
+            for (int k = 0; k < 4; k++) at[2 * i + k / 2].push_back((char*)mem + 8 * rnd(room));
+            d[i].sendbufs = at[2 * i].data();
+            d[i].recvbufs = at[2 * i + 1].data();
+        }
+        auto conflict = [&](int i, int j) {
+            for (int a = 0; a < 4; a++)
+                for (int b = 0; b < 4; b++) {
+                    const char *p = (char*)at[2 * i + a / 2][a % 2], *q = (char*)at[2 * j + b / 2][b % 2];
+                    if ((a >= 2 || b >= 2) && p < q + 8 * d[j].count && q < p + 8 * d[i].count) return true;
+                }
+            return false;
+        };
+        std::vector<int> level(n, 0);
+        std::vector<CallSet> want;
+        for (int i = 0; i < n; i++) {
+            for (int j = 0; j < i; j++)
+                if (conflict(i, j)) level[i] = std::max(level[i], level[j] + 1);
+            if ((int)want.size() <= level[i]) want.resize(level[i] + 1);
+            want[level[i]].insert({at[2 * i][0], at[2 * i + 1][0]});
+        }
+        gpumpi_plan_t p = nullptr;
+        CHECK(gpumpi_plan_create(d.data(), n, 64, 1, &p) == 0, "%s", gpumpi_last_error());
+        g_launched.clear();
+        CHECK(gpumpi_plan_launch(p, nullptr) == 0, "%s", gpumpi_last_error());
+        CHECK(g_launched == want, "list %d: %zu levels, %zu expected", it, g_launched.size(), want.size());
+        gpumpi_plan_destroy(p);
+    }
+}
+
+// Creating a long plan of dependent calls takes no more than a few times as long as one of independent calls.
+static void long_plans() {
+    const int P = 256, n = 2000;
+    void* mem = nullptr;
+    cudaMalloc(&mem, (size_t)P * (n + 1) * 8);
+    gpumpi_comm_t comm = nullptr;
+    CHECK(gpumpi_comm_create(P, &comm) == 0, "comm");
+    double took[2];
+    for (int dependent = 0; dependent < 2; dependent++) {
+        std::vector<std::vector<void*>> at(n + 1);
+        for (int i = 0; i <= n; i++)
+            for (int r = 0; r < P; r++) at[i].push_back((char*)mem + ((size_t)(dependent ? i % 2 : i) * P + r) * 8);
+        std::vector<gpumpi_coll_desc> d(n);
+        for (int i = 0; i < n; i++) {
+            memset(&d[i], 0, sizeof(d[i]));
+            d[i].comm = comm;
+            d[i].op = GPUMPI_COLL_ALLREDUCE;
+            d[i].dtype = MPI_DOUBLE;
+            d[i].redop = GPUMPI_OP_SUM;
+            d[i].count = 1;
+            d[i].sendbufs = dependent ? at[i].data() : nullptr;
+            d[i].recvbufs = at[i + 1].data();
+        }
+        gpumpi_plan_t p = nullptr;
+        const auto t0 = std::chrono::steady_clock::now();
+        CHECK(gpumpi_plan_create(d.data(), n, 64, 1, &p) == 0, "%s", gpumpi_last_error());
+        took[dependent] = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        CHECK(gpumpi_plan_launch_ordered(p) == !dependent, "form");
+        gpumpi_plan_destroy(p);
+    }
+    printf("independent %.3f s, dependent %.3f s\n", took[0], took[1]);
+    CHECK(took[1] < 10 * took[0] + 0.2, "%.3f s, %.3f s", took[0], took[1]);
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
         {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}, {"errors", errors},
-        {"levels", levels}};
+        {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans}};
     fake::state().kernel_spans = kernel_spans;
     scenarios.at(argc > 1 ? argv[1] : "")();
     printf("%s bad %d\n", argv[1], bad);
