@@ -251,13 +251,13 @@ ApiJob g_api;
 int spread_attributes();
 
 int api_job() {
+    int rc = spread_attributes();
+    if (rc) return rc;
     if (g_api.djob) return GPUMPI_OK;
     // the plan kernel streams through L2 (ld.global.cg) and stages bulk copies
     // in shared memory: prefer the largest shared-memory carve-out
     CK(cudaFuncSetAttribute((const void*)gpumpi_plan_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
                             (int)cudaSharedmemCarveoutMaxShared));
-    int rc = spread_attributes();
-    if (rc) return rc;
     Job hj;
     memset(&hj, 0, sizeof(hj));
     char* mem = nullptr;
@@ -447,11 +447,19 @@ int launch(const void* kern, int grid, int threads, size_t smem, void* args, cud
     return GPUMPI_OK;
 }
 
+// Kernel attributes belong to a device: once for each that plans are made on.
 int spread_attributes() {
+    static std::mutex mu;
+    static std::vector<int> done;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    if (std::find(done.begin(), done.end(), dev) != done.end()) return GPUMPI_OK;
     for (const void* k : {(const void*)gpumpi_spread_kernel, (const void*)gpumpi_spread_params_kernel}) {
         CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
         CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM));
     }
+    done.push_back(dev);
     return GPUMPI_OK;
 }
 

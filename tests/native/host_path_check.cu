@@ -312,10 +312,20 @@ static void long_plans() {
     CHECK(took[1] < 10 * took[0] + 0.2, "%.3f s, %.3f s", took[0], took[1]);
 }
 
+// A plan made on a second device raises the kernels' shared memory limit there too.
+static void devices() {
+    for (int dev : {0, 1, 0, 2}) {
+        fake::state().current_device = dev;
+        make(1, SMALL);
+        CHECK(fake::state().attributes.count({(const void*)gpumpi_spread_kernel, dev}) == 1, "device %d", dev);
+    }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
         {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}, {"errors", errors},
-        {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans}};
+        {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans},
+        {"devices", devices}};
     fake::state().kernel_spans = kernel_spans;
     scenarios.at(argc > 1 ? argv[1] : "")();
     printf("%s bad %d\n", argv[1], bad);
