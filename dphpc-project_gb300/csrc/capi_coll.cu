@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -196,7 +197,7 @@ struct gpumpi_plan_s {
     int batched;
     int threads;
     size_t smem;
-    char* base;                       // device allocation
+    char* base = nullptr;             // device allocation
     PlanArgs batch_args;              // batched launch
     std::vector<PlanArgs> plain_args; // one per descriptor
     std::vector<int> plain_grid;
@@ -222,7 +223,10 @@ struct gpumpi_plan_s {
     size_t pipe_bytes = 0;
     cudaEvent_t host_done = nullptr;       // end of the last host-buffer call, the next one starts after it
     ~gpumpi_plan_s() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
         if (host_done) cudaEventDestroy(host_done);
+        if (base) cudaFree(base);
     }
 };
 
@@ -613,7 +617,7 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     size_t off_pubt = (off_ptr + sizeof(void*) * ptrs + 63) & ~(size_t)63;   // Pub tables, one entry per rank
     const size_t off_sp = off_pubt + sizeof(Pub) * (ptrs / 2);   // SpreadCalls, then their address tables
     // the spread form: the whole batched launch, or each plain launch it covers
-    gpumpi_plan_s* p = new gpumpi_plan_s();
+    std::unique_ptr<gpumpi_plan_s> p(new gpumpi_plan_s());   // gone with its memory on any error below
     std::vector<int> level;
     const int nlevels = plan_levels(descs, ndesc, level);
     p->independent = nlevels == 1;
@@ -794,12 +798,10 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
             snprintf(m, sizeof(m), "%d rank blocks of %d threads cannot be co-resident (max %d)", need, t,
                      per * sms);
             set_last_error(m);
-            cudaFree(p->base);
-            delete p;
             return GPUMPI_ENORES;
         }
     }
-    *out = p;
+    *out = p.release();
     return GPUMPI_OK;
 }
 
@@ -1184,9 +1186,6 @@ extern "C" int gpumpi_plan_run_host(gpumpi_plan_t p, void* const* host_send, voi
 
 extern "C" int gpumpi_plan_destroy(gpumpi_plan_t p) {
     if (!p) return GPUMPI_EINVAL;
-    if (p->exec) cudaGraphExecDestroy(p->exec);
-    if (p->graph) cudaGraphDestroy(p->graph);
-    cudaFree(p->base);
     delete p;
     return GPUMPI_OK;
 }

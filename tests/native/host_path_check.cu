@@ -321,11 +321,37 @@ static void devices() {
     }
 }
 
+// A plan that cannot be made leaves no device memory behind.
+static void failed_plans() {
+    Job_* j = make(3, SMALL);
+    for (const char* what : {"cudaMalloc", "cudaMemcpy", "cudaStreamSynchronize", "cudaGetDevice",
+                             "cudaOccupancyMaxActiveBlocksPerMultiprocessor"})
+        for (int batched : {0, 1}) {
+            const size_t before = fake::state().device.size();
+            gpumpi_plan_t p = nullptr;
+            int first = fake::state().calls[what];
+            CHECK(gpumpi_plan_create(j->descs.data(), 3, 64, batched, &p) == 0, "%s", gpumpi_last_error());
+            gpumpi_plan_destroy(p);
+            const int n = fake::state().calls[what] - first;
+            CHECK(n > 0, "%s is not called", what);
+            fake::state().fail = what;
+            for (int k = 0; k < n; k++) {
+                fake::state().fail_at = fake::state().calls[what] + k;
+                p = nullptr;
+                const int rc = gpumpi_plan_create(j->descs.data(), 3, 64, batched, &p);
+                fake::state().fail_at = -1;
+                CHECK(rc == 0 || p == nullptr, "%s call %d", what, k);
+                if (rc == 0) gpumpi_plan_destroy(p);   // the rank blocks' staging is sized without it
+                CHECK(fake::state().device.size() == before, "%s call %d: memory left", what, k);
+            }
+        }
+}
+
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
         {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}, {"errors", errors},
         {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans},
-        {"devices", devices}};
+        {"devices", devices}, {"failed_plans", failed_plans}};
     fake::state().kernel_spans = kernel_spans;
     scenarios.at(argc > 1 ? argv[1] : "")();
     printf("%s bad %d\n", argv[1], bad);
