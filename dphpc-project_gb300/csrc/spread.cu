@@ -369,20 +369,35 @@ static __device__ __noinline__ void stream_tile(const SpreadCall& c, u32 tile, c
 // rows), which 512-byte rows only just afford.
 constexpr int SP_GROUPS = 3;
 
-template <class T, class O>
+//
+// MANY: more than SP_TAB ranks.  The sources' addresses are needed over and
+// over, each before a load can start, and the shared memory that the blocks of
+// an SM take leaves L1 no room for them: they lie at its end.  Of the
+// destinations' addresses each lane reads one of 32 ahead of the stores before
+// them, since a load from global memory cannot move above a store that may
+// change it.  (Allreduce of 1024 ranks of 60001 FP64, chunks of 256 bytes, with
+// all addresses in global memory 430 us, so 378; of 257 ranks 131 and 102.)
+template <class T, class O, bool MANY>
 static __device__ __noinline__ void rows_tile(const SpreadCall& c, u32 tile, char* smem) {
     constexpr int K = 16 / sizeof(T);    // elements a lane holds of a chunk of 512 bytes
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const char* const* st;
     char* const* dt;
-    tables(c, smem, st, dt);
+    if constexpr (MANY) {
+        const char** ts = reinterpret_cast<const char**>(smem + fold_table(c.nsrc));
+        for (u32 q = threadIdx.x; q < c.nsrc; q += SP_T) ts[q] = ld_ptr(c.src, q);
+        st = ts;
+        dt = c.dst;
+    } else {
+        tables(c, smem, st, dt);
+    }
     const u32 all = (u32)((c.nu + c.per - 1) / c.per);
     const u32 w0 = tile * c.rows + warp, w1 = min(tile * c.rows + c.rows, all);
     const u32 chunks = w1 > w0 ? (w1 - w0 + SP_WARPS - 1) / SP_WARPS : 0;   // this warp's
     const u32 groups = (c.nsrc + c.batch - 1) / c.batch;
     const u32 steps = chunks * groups;
     const u32 pitch = c.ub, units = pitch / 16, group_bytes = c.batch * pitch;
-    char* part = smem + warp * SP_PART;
+    char* part = smem + warp * (MANY ? rows_part(c.nsrc) : SP_PART);
     const u32 part_s = smem_addr(part);
     // unit `lane` of a group, and how units 32 further on lie
     const u32 j0 = lane / units, u0 = lane - j0 * units;
@@ -447,22 +462,143 @@ static __device__ __noinline__ void rows_tile(const SpreadCall& c, u32 tile, cha
             for (; j < n; j++) fold(j, false);
             if (++cg == SP_GROUPS) cg = 0;
         }
+        if constexpr (MANY) {
+            u64 next = lane < c.ndst ? (u64)ld_ptr(dt, lane) : 0;
+            for (u32 r0 = 0; r0 < c.ndst; r0 += 32) {
+                const u64 now = next;
+                if (r0 + 32 + lane < c.ndst) next = (u64)ld_ptr(dt, r0 + 32 + lane);
+                const u32 n = min(32u, c.ndst - r0);
 #pragma unroll 4
-        for (u32 r = 0; r < c.ndst; r++) {
-            T* d = reinterpret_cast<T*>(dt[r] + at) + lane;
+                for (u32 r = 0; r < n; r++) {
+                    T* d = reinterpret_cast<T*>(__shfl_sync(~0u, now, r) + at) + lane;
 #pragma unroll
-            for (int k = 0; k < K; k++)
-                if (k * 32 + lane < m) d[k * 32] = acc[k];
+                    for (int k = 0; k < K; k++)
+                        if (k * 32 + lane < m) d[k * 32] = acc[k];
+                }
+            }
+        } else {
+#pragma unroll 4
+            for (u32 r = 0; r < c.ndst; r++) {
+                T* d = reinterpret_cast<T*>(dt[r] + at) + lane;
+#pragma unroll
+                for (int k = 0; k < K; k++)
+                    if (k * 32 + lane < m) d[k * 32] = acc[k];
+            }
         }
     }
     cp_wait<0>();
+}
+
+// n units of V of each of nsrc sources, one after another in g, SP_T units at a time.
+template <class V>
+static __device__ __forceinline__ void passes_load(const char* const* src, u32 nsrc, u64 at, u32 n, char* g) {
+    const u32 total = n * nsrc;
+    const u32 d_q = SP_T / n, d_i = SP_T % n;
+    u32 q = threadIdx.x / n, i = threadIdx.x % n;
+    const u32 g_s = smem_addr(g);
+    for (u32 k = threadIdx.x; k < total; k += SP_T) {
+        const char* p = src[q] + at + (u64)i * sizeof(V);
+        if constexpr (sizeof(V) >= 4) cp_async<sizeof(V)>(g_s + k * (u32)sizeof(V), p);
+        else reinterpret_cast<V*>(g)[k] = ld_unit<V>(p);
+        q += d_q;
+        i += d_i;
+        if (i >= n) {
+            i -= n;
+            q++;
+        }
+    }
+}
+
+// The n units of V at `res` to each of ndst destinations.
+template <class V>
+static __device__ __forceinline__ void passes_store(char* const* dst, u32 ndst, u64 at, u32 n, const char* res) {
+    const u32 total = n * ndst;
+    const u32 d_r = SP_T / n, d_i = SP_T % n;
+    u32 r = threadIdx.x / n, i = threadIdx.x % n;
+    for (u32 k = threadIdx.x; k < total; k += SP_T) {
+        reinterpret_cast<V*>(dst[r] + at)[i] = reinterpret_cast<const V*>(res)[i];
+        r += d_r;
+        i += d_i;
+        if (i >= n) {
+            i -= n;
+            r++;
+        }
+    }
+}
+
+// acc folded with n elements at g, `pitch` elements apart.
+template <class T, class O>
+static __device__ __forceinline__ T fold_column(T acc, const T* g, u32 n, u32 pitch) {
+    u32 q = 0;
+    for (; q + 8 <= n; q += 8) {
+        T x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) x[k] = g[(q + k) * pitch];
+#pragma unroll
+        for (int k = 0; k < 8; k++) acc = O::f(x[k], acc);
+    }
+    for (; q < n; q++) acc = O::f(g[q * pitch], acc);
+    return acc;
+}
+
+// One chunk by the whole block (SP_ROWS with `group` 1): a gather tile in passes
+// over the sources, each loaded into one half of the ring while the one before
+// it is folded from the other.  More ranks than the ring holds 32 elements of
+// would leave a gather tile with less than a warp's lanes to add, and an FP64
+// addition takes a warp as long for one lane as for 32; a warp with a chunk of
+// its own takes five times as long for each source, finding its address and
+// its element there, and a call of few chunks has few warps.
+template <class T, class O>
+static __device__ __noinline__ void passes_tile(const SpreadCall& c, u32 tile, char* smem) {
+    const u32 m = (u32)min((u64)c.per, c.nu - (u64)tile * c.per);
+    const u64 at = c.off + (u64)tile * c.per * sizeof(T);
+    const u32 batch = passes_half(c.nsrc) / (c.per * (u32)sizeof(T));   // sources of a pass
+    const bool units16 = c.ub == c.per * sizeof(T);
+    const char** ts = reinterpret_cast<const char**>(smem + fold_table(c.nsrc));
+    for (u32 q = threadIdx.x; q < c.nsrc; q += SP_T) ts[q] = ld_ptr(c.src, q);
+    __syncthreads();
+    const u32 half = passes_half(c.nsrc);
+    u32 q1 = 0, into = 0;   // the next pass to load and its half
+    auto issue = [&]() {
+        const u32 n = min(batch, c.nsrc - q1);
+        if (n) {
+            if (units16) passes_load<uint4>(ts + q1, n, at, m * (u32)sizeof(T) / 16, smem + into * half);
+            else passes_load<T>(ts + q1, n, at, m, smem + into * half);
+        }
+        cp_commit();
+        q1 += n;
+        into ^= 1;
+    };
+    issue();
+    T acc{};
+    u32 from = 0;
+    for (u32 q = 0; q < c.nsrc; q += batch) {
+        issue();
+        cp_wait<1>();
+        __syncthreads();   // every thread's part of the pass has arrived
+        const T* g = reinterpret_cast<const T*>(smem + from * half) + threadIdx.x;
+        const u32 n = min(batch, c.nsrc - q);
+        if (threadIdx.x < m) acc = q ? fold_column<T, O>(acc, g, n, m) : fold_column<T, O>(g[0], g + m, n - 1, m);
+        from ^= 1;
+        __syncthreads();   // before its half is loaded again
+    }
+    cp_wait<0>();
+    // the results and the destinations' addresses take the ring's place
+    char** td = reinterpret_cast<char**>(smem + SP_T * sizeof(T));
+    if (threadIdx.x < m) reinterpret_cast<T*>(smem)[threadIdx.x] = acc;
+    for (u32 r = threadIdx.x; r < c.ndst; r += SP_T) td[r] = ld_ptr(c.dst, r);
+    __syncthreads();
+    if (units16) passes_store<uint4>(td, c.ndst, at, m * (u32)sizeof(T) / 16, smem);
+    else passes_store<T>(td, c.ndst, at, m, smem);
 }
 
 template <class T, class O>
 static __device__ __forceinline__ void fold_tile(const SpreadCall& c, u32 tile, char* smem) {
     if (c.kind == SP_GATHER) gather_tile<T, O>(c, tile, smem);
     else if (c.kind == SP_STREAM) stream_tile<T, O, uint4>(c, tile, smem);
-    else rows_tile<T, O>(c, tile, smem);
+    else if (c.group) passes_tile<T, O>(c, tile, smem);
+    else if (c.nsrc > SP_TAB) rows_tile<T, O, true>(c, tile, smem);
+    else rows_tile<T, O, false>(c, tile, smem);
 }
 
 // ---- bulk copies into the ring
@@ -1098,6 +1234,22 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         const double fits = (double)SP_RING / ((double)P * esize);
         const u64 most = (u64)fits / step * step;   // elements of the largest gather tile
         const u64 nrows = split(hi / V, SP_T);
+        // Above SP_TAB ranks gather tiles stay where they all run at once, which is
+        // short calls; then SP_ROWS in passes, with as few elements a tile as keep the SMs
+        // busy (512 bytes at most); from 1 MiB chunks of a warp, whose loads never pause
+        // (from 96 KiB for odd buffers of 1- and 2-byte types, which passes load one by one).
+        // One call, Reduce of FP64 unless named, gather / passes of 32, 64, 128 elements
+        // / a warp's chunks of 512 bytes, us: 1024 ranks of 2000 48 / 51, 58, 73 / 240,
+        // of 20000 298 / 107, 86, 107 / 254, of 60000 835 / 216, 174, 166 / 257, of
+        // 150000 1897 / 443, 344, 324 / 312; 512 of 60000 256 / 115, 92, 86 / 131, of
+        // 150000 525 / 237, 181, 168 / 158; Allreduce of 60001 int32, 1024 ranks 279 /
+        // 156, 147, 142 / 175, of 150001 448 / 354, 320, 292 / 277; of 512 ranks of
+        // 150001 uint8 320 / -, -, 244 / 206.
+        // (Rank blocks: Reduce of 60000, 512 ranks 145, 1024 277.)  Among other calls
+        // the warps' chunks start earlier (Allreduce and Reduce of FP64 and int32 by
+        // communicators of 1024, 512, 256 and 64 ranks, passes / chunks from 128 KiB:
+        // 20001 elements 384 / 559, 60001 1010 / 801).
+        const bool many = P > SP_TAB;
         if (lone) {
             const u64 m = lone_gather(n, step, most);
             if (m) {
@@ -1108,7 +1260,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         // A lone fold that does not fit streams when that gives two tiles for each
         // SM (4 ranks of 10^6 FP64: rows 13.7, stream 12.3, gather 14.6 us; 64 of
         // 62496, 122 rows: 23.0, 19.3, 18.7; 200 of 20000, 39 rows: 52, 52, 26)
-        if (aligned && (lone ? nrows >= 2 * SP_SMS : row * SP_T * 16 <= 2 * target) && hi >= SP_T * V) {
+        if (aligned && !many && (lone ? nrows >= 2 * SP_SMS : row * SP_T * 16 <= 2 * target) && hi >= SP_T * V) {
             c.kind = SP_STREAM;
             c.nu = hi;
             c.per = (u32)std::max(1.0, std::min((double)nrows, target / (row * SP_T * 16)));
@@ -1121,16 +1273,32 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         }
         // a lone fold of buffers aligned to their elements (4 ranks of 2 * 10^6 int32:
         // gather 19.4, rows 13.7 us; 64 of 62497 FP64, 500 KB each: 20.0, 24.6 us)
-        if (hi > lo && (lone ? !aligned && (hi - lo) * esize >= 524288
-                             : (hi - lo) * esize >= rows_min(aligned, total))) {
+        const u64 inner = hi > lo ? (hi - lo) * esize : 0;
+        const bool alone = level.calls == 1;
+        const u64 least = many && alone ? aligned || esize >= 4 ? 1048576 : 98304
+                          : lone        ? aligned ? ~0ull : 524288
+                          : many        ? std::max<u64>(32768 * esize, rows_min(aligned, total))
+                                        : rows_min(aligned, total);
+        const bool passes = many && inner && inner < least && (aligned || esize > 1) &&
+                            (lone || (level.folded > 4.0 * SP_SMS * most && (alone || n > SP_SMS / 2 * most)));
+        if (passes || (inner && inner >= least)) {
             c.kind = SP_ROWS;
             c.off = lo * esize;
             c.nu = hi - lo;
             u32 chunk = 512;
-            while (chunk > 32 * (u32)esize && row * chunk * SP_WARPS > 4 * target) chunk /= 2;
+            if (passes) {
+                const u32 per = level.folded <= 2.0 * SP_SMS * 32    ? 32
+                                : level.folded <= 4.0 * SP_SMS * 64  ? 64
+                                : level.folded <= 4.0 * SP_SMS * 128 ? 128
+                                                                     : 256;
+                chunk = std::min(512u, per * (u32)esize);
+                c.group = 1;
+            }
+            while (many && alone && !passes && chunk > 128 && inner < 580ull * chunk) chunk /= 2;
+            while (!(many && alone) && !passes && chunk > 32 * (u32)esize && row * chunk * SP_WARPS > 4 * target) chunk /= 2;
             c.per = chunk / esize;
             c.ub = chunk + (aligned ? 0 : 16);
-            c.batch = std::min(c.nsrc, SP_PART / (SP_GROUPS * c.ub));
+            c.batch = std::min(c.nsrc, rows_part(c.nsrc) / (SP_GROUPS * c.ub));
             const u64 chunks = (c.nu + c.per - 1) / c.per;
             c.rows = (u32)std::min((double)chunks, SP_WARPS * std::max(1.0, target / (row * chunk * SP_WARPS)));
             if (lone) {
@@ -1140,6 +1308,8 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
                 const u32 k = c.nsrc < 16 || (c.nsrc < 32 && total >= 1e8) ? 2 : 4;
                 c.rows = (u32)round_up(split(chunks, k * SP_SMS), SP_WARPS);
             }
+            if (lone && many) c.rows = (u32)split(chunks, 4 * SP_SMS);
+            if (passes) c.rows = 1;
             c.ntiles = (u32)((chunks + c.rows - 1) / c.rows);
             c.tile_bytes = (u32)(row * chunk * c.rows);
             calls.push_back(c);

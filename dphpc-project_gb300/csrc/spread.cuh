@@ -35,6 +35,13 @@ constexpr u32 SP_SMEM = SP_RING + 2 * SP_TAB * (u32)sizeof(char*);
 constexpr int SP_WARPS = SP_T / 32;
 constexpr u32 SP_PART = SP_RING / SP_WARPS;   // a warp's part of the ring
 constexpr u32 SP_CHUNK = 128;
+// With more than SP_TAB ranks a fold keeps the sources' addresses at the end of
+// its shared memory; that leaves each warp this much of the ring.
+__host__ __device__ constexpr u32 fold_table(u32 nsrc) { return SP_SMEM - nsrc * (u32)sizeof(char*); }
+__host__ __device__ constexpr u32 rows_part(u32 nsrc) {
+    return nsrc <= 2 * SP_TAB ? SP_PART : fold_table(nsrc) / SP_WARPS / 16 * 16;
+}
+__host__ __device__ constexpr u32 passes_half(u32 nsrc) { return fold_table(nsrc) / 32 * 16; }
 constexpr int SP_MAX_STAGES = 8;
 constexpr int SP_BLOCKS_PER_SM = 4;     // 208 KiB of shared memory, 64 registers a thread
 
@@ -65,7 +72,8 @@ enum SpreadKind : int {
     SP_MOVE = 4,
     // The fold again, of buffers aligned to their elements only or in finer
     // pieces.  Each warp folds chunks of `per` elements, a tile is `rows`
-    // chunks; `batch` sources are loaded at a time, `ub` bytes apart.
+    // chunks; `batch` sources are loaded at a time, `ub` bytes apart.  With `group`
+    // 1 a tile is one chunk, folded by the whole block in passes over the sources.
     SP_ROWS = 5,
 };
 
