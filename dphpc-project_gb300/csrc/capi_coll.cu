@@ -899,18 +899,15 @@ namespace {
 typedef int (*AddrRangeFn)(unsigned long long* base, size_t* size, unsigned long long ptr);
 
 AddrRangeFn addr_range() {
-    static AddrRangeFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static AddrRangeFn fn = [] {
         void* f = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
             q == cudaDriverEntryPointSuccess)
-            fn = (AddrRangeFn)f;
-        else
-            cudaGetLastError();
-    }
+            return (AddrRangeFn)f;
+        cudaGetLastError();
+        return (AddrRangeFn) nullptr;
+    }();
     return fn;
 }
 

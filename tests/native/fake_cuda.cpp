@@ -140,6 +140,7 @@ static int fake_address_range(unsigned long long* base, size_t* size, unsigned l
 }
 cudaError_t cudaGetDriverEntryPointByVersion(const char* name, void** f, unsigned, unsigned long long,
                                              cudaDriverEntryPointQueryResult* q) {
+    if (fake::state().pause_us) std::this_thread::sleep_for(std::chrono::microseconds(fake::state().pause_us));
     *f = !strcmp(name, "cuMemGetAddressRange") ? (void*)fake_address_range : nullptr;
     *q = *f ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
     return cudaSuccess;

@@ -48,7 +48,7 @@ struct State {
     std::map<std::string, int> calls;      // calls of each function
     std::string fail;                      // this function ...
     int fail_at = -1;                      // ... fails at this call (counted from 0; -1: never)
-    int pause_us = 0;                      // length of a copy call
+    int pause_us = 0;                      // length of a copy call and of a look-up of a driver function
     // bytes that a kernel launch touches
     std::vector<Span> (*kernel_spans)(const void* kernel, void** args) = nullptr;
 };

@@ -186,6 +186,23 @@ static void turns() {
     }
 }
 
+// The first calls of a process, of two plans from two threads: both go in groups.
+static void first_calls() {
+    Job_* jobs[2] = {make(3, LARGE), make(3, LARGE)};
+    cudaStream_t streams[2] = {stream(), stream()};
+    const size_t from = fake::state().ops.size();
+    fake::state().pause_us = 2000;
+    std::vector<std::thread> threads;
+    for (int t = 0; t < 2; t++)
+        threads.emplace_back([&, t] {
+            std::this_thread::sleep_for(std::chrono::microseconds(1000 * t));
+            CHECK(run_host(jobs[t], streams[t]) == 0, "%s", gpumpi_last_error());
+        });
+    for (auto& t : threads) t.join();
+    fake::state().pause_us = 0;
+    CHECK(streams_used(from) == 6, "%d streams", streams_used(from));
+}
+
 // A call that fails half way reports it, and nothing that it put on other streams outlives a wait for the caller's.
 static void errors() {
     int failed = 0;
@@ -349,7 +366,8 @@ static void failed_plans() {
 
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
-        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns}, {"errors", errors},
+        {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns},
+        {"first_calls", first_calls}, {"errors", errors},
         {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans},
         {"devices", devices}, {"failed_plans", failed_plans}};
     fake::state().kernel_spans = kernel_spans;
