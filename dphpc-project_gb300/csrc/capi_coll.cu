@@ -832,10 +832,43 @@ static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
     return GPUMPI_OK;
 }
 
+// One launch of independent tiles, which may start while the launch before it ends.
+static bool one_launch(gpumpi_plan_t p) {
+    return p->batched && p->batch_spread && p->sync_mode == 0 && p->batch_tiles.size() == 1;
+}
+
+// True when everything that `st` was given has run.  By the driver's function,
+// which leaves the runtime's last error alone, in the relaxed mode, which no
+// capture of another thread minds; a stream under capture is not asked.
+static bool stream_idle(cudaStream_t st) {
+    typedef int (*QueryFn)(cudaStream_t);
+    static QueryFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuStreamQuery", &f, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            return (QueryFn)f;
+        cudaGetLastError();
+        return (QueryFn) nullptr;
+    }();
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusActive;
+    if (!fn || cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone)
+        return false;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return false;
+    const bool idle = fn(st) == 0;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return idle;
+}
+
 extern "C" int gpumpi_plan_launch(gpumpi_plan_t p, void* stream) {
     if (!p) return GPUMPI_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
-    if (p->exec) {
+    // A graph cannot overlap the launch before it, so that of a single launch of
+    // tiles is for a stream that has nothing else to do (the 16-communicator batch at
+    // 1 element per rank, graph / launched: with a wait after each 22.0 / 23.4 us, back
+    // to back 16.4 / 13.1).
+    if (p->exec && (!one_launch(p) || stream_idle(st))) {
         CK(cudaGraphLaunch(p->exec, st));
         g_launches += !p->batched ? p->ndesc : p->batch_spread && p->sync_mode == 0 ? p->batch_tiles.size() : 1;
         return GPUMPI_OK;
@@ -864,10 +897,6 @@ extern "C" int gpumpi_plan_launch_ordered(gpumpi_plan_t p) {
 
 extern "C" int gpumpi_plan_capture(gpumpi_plan_t p, void* stream) {
     if (!p) return GPUMPI_EINVAL;
-    // One launch of independent tiles: replaying it as a graph would keep it from
-    // overlapping the launch before it (the 16-communicator batch at 1 element per
-    // rank, back to back: 16.4 us as a graph, 12.9 us launched; alone 22.5 and 23.9).
-    if (p->batched && p->batch_spread && p->sync_mode == 0 && p->batch_tiles.size() == 1) return GPUMPI_OK;
     (void)stream;   // captured on a private stream; replays go to the stream given to gpumpi_plan_launch
     cudaStream_t cap;
     CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));

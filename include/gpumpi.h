@@ -260,8 +260,9 @@ int gpumpi_plan_launch_ordered(gpumpi_plan_t plan);
 /* Capture the plan's launches once as a CUDA graph; later launches replay it
  * on the stream given to gpumpi_plan_launch.  `stream` is not used (the
  * capture runs on a private stream).  A batched plan that is one launch of
- * independent tiles is left as it is: launched directly it can overlap its
- * neighbours, which a graph cannot. */
+ * independent tiles replays the graph only on a stream that is idle, where
+ * that is quicker; behind other work it is launched directly, so that it can
+ * overlap its neighbours, which a graph cannot. */
 int gpumpi_plan_capture(gpumpi_plan_t plan, void* stream);
 /* Host-buffer form: per-rank host->device copies of the send data, the plan,
  * device->host copies of the results, ordered on `stream`.  A batched plan of

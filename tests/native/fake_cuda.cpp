@@ -63,9 +63,44 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t e, unsigned) {
     s.stream[st] |= s.event[e];
     return cudaSuccess;
 }
-cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* c) {
+cudaError_t cudaStreamIsCapturing(cudaStream_t st, cudaStreamCaptureStatus* c) {
     FAKE_CALL("cudaStreamIsCapturing");
-    *c = cudaStreamCaptureStatusNone;
+    *c = s.capturing.count(st) ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* mode) {
+    FAKE_CALL("cudaThreadExchangeStreamCaptureMode");
+    static thread_local cudaStreamCaptureMode now = cudaStreamCaptureModeGlobal;
+    std::swap(now, *mode);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamBeginCapture(cudaStream_t st, cudaStreamCaptureMode) {
+    FAKE_CALL("cudaStreamBeginCapture");
+    s.capturing.insert(st);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamEndCapture(cudaStream_t st, cudaGraph_t* g) {
+    FAKE_CALL("cudaStreamEndCapture");
+    s.capturing.erase(st);
+    *g = (cudaGraph_t)malloc(64);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long long) {
+    FAKE_CALL("cudaGraphInstantiate");
+    *e = (cudaGraphExec_t)malloc(64);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) {
+    FAKE_CALL("cudaGraphLaunch");
+    fake::enqueue("graph", st, {});
+    return cudaSuccess;
+}
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) {
+    free(e);
+    return cudaSuccess;
+}
+cudaError_t cudaGraphDestroy(cudaGraph_t g) {
+    free(g);
     return cudaSuccess;
 }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
@@ -138,10 +173,17 @@ static int fake_address_range(unsigned long long* base, size_t* size, unsigned l
     *size = it->second;
     return 0;
 }
+// a query of a stream under capture would end the capture
+static int fake_stream_query(cudaStream_t st) {
+    if (fake::state().capturing.count(st)) abort();
+    return fake::state().busy.count(st) ? 600 : 0;
+}
 cudaError_t cudaGetDriverEntryPointByVersion(const char* name, void** f, unsigned, unsigned long long,
                                              cudaDriverEntryPointQueryResult* q) {
     if (fake::state().pause_us) std::this_thread::sleep_for(std::chrono::microseconds(fake::state().pause_us));
-    *f = !strcmp(name, "cuMemGetAddressRange") ? (void*)fake_address_range : nullptr;
+    *f = !strcmp(name, "cuMemGetAddressRange") ? (void*)fake_address_range
+         : !strcmp(name, "cuStreamQuery")      ? (void*)fake_stream_query
+                                               : nullptr;
     *q = *f ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
     return cudaSuccess;
 }

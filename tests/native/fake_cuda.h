@@ -41,6 +41,7 @@ struct State {
     std::map<void*, Ops> stream, event;    // what the next operation of a stream / a waiter of an event comes after
     Ops host;                              // what the host has waited for
     std::set<void*> live_streams, live_events;
+    std::set<void*> busy, capturing;       // streams that report work, that are under capture
     std::map<char*, size_t> device;        // allocations
     std::vector<std::pair<const char*, size_t>> pinned;
     int mallocs = 0, current_device = 0;

@@ -203,6 +203,41 @@ static void first_calls() {
     CHECK(streams_used(from) == 6, "%d streams", streams_used(from));
 }
 
+// A captured plan of one launch replays its graph on an idle stream and is
+// launched behind other work or under capture; one of several launches is a graph always.
+static void captured() {
+    Job_* j = make(3, SMALL);
+    cudaStream_t st = stream();
+    auto launched = [&](gpumpi_plan_t p) {
+        const size_t from = fake::state().ops.size();
+        const uint64_t count = gpumpi_kernel_launches();
+        CHECK(gpumpi_plan_launch(p, st) == 0, "%s", gpumpi_last_error());
+        CHECK(gpumpi_kernel_launches() > count, "launches");
+        return fake::state().ops.size() == from + 1 ? fake::state().ops[from].what : std::string("?");
+    };
+    CHECK(launched(j->plan) == "launch", "before the capture");
+    const uint64_t count = gpumpi_kernel_launches();
+    CHECK(gpumpi_plan_capture(j->plan, nullptr) == 0 && gpumpi_kernel_launches() == count, "%s", gpumpi_last_error());
+    CHECK(launched(j->plan) == "graph", "idle");
+    fake::state().busy.insert(st);
+    CHECK(launched(j->plan) == "launch", "busy");
+    fake::state().busy.clear();
+    fake::state().capturing.insert(st);
+    CHECK(launched(j->plan) == "launch", "under capture");
+    fake::state().capturing.clear();
+    CHECK(launched(j->plan) == "graph", "idle again");
+    CHECK(gpumpi_plan_set_sync(j->plan, 1) == 0 && gpumpi_plan_set_sync(j->plan, 0) == 0, "set_sync");
+    CHECK(launched(j->plan) == "launch", "the graph has been dropped");
+    j->descs[1].sendbufs = j->descs[0].recvbufs;   // a second level
+    gpumpi_plan_t p = nullptr;
+    CHECK(gpumpi_plan_create(j->descs.data(), 3, 64, 1, &p) == 0 && gpumpi_plan_capture(p, nullptr) == 0, "%s",
+          gpumpi_last_error());
+    CHECK(launched(p) == "graph", "levels, idle");
+    fake::state().busy.insert(st);
+    CHECK(launched(p) == "graph", "levels, busy");
+    gpumpi_plan_destroy(p);
+}
+
 // A call that fails half way reports it, and nothing that it put on other streams outlives a wait for the caller's.
 static void errors() {
     int failed = 0;
@@ -367,7 +402,7 @@ static void failed_plans() {
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
         {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns},
-        {"first_calls", first_calls}, {"errors", errors},
+        {"first_calls", first_calls}, {"captured", captured}, {"errors", errors},
         {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans},
         {"devices", devices}, {"failed_plans", failed_plans}};
     fake::state().kernel_spans = kernel_spans;
