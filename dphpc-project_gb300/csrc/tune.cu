@@ -14,8 +14,10 @@
 // Timing: two untimed launches, then `reps` launches between CUDA events on
 // a stream of its own.  Plain results are cached, one line per shape, thread
 // count and GPU:
-//   <gpu name>|<op> <dtype> <redop> <ranks> <count> <threads>|<algo> <us>
-// so a later run with the same shapes skips those measurements.
+//   <gpu name>|tiles <op> <dtype> <redop> <ranks> <count> <threads>|<algo> <us>
+// so a later run with the same shapes skips those measurements.  The word before
+// the shape stands for what the schedules' numbers mean: lines without it are
+// from before some of them ran as tiles, and are measured again.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>
@@ -47,7 +49,7 @@ std::string shape_key(const gpumpi_coll_desc& d) {
     int n = 0;
     gpumpi_comm_size(d.comm, &n);
     std::ostringstream k;
-    k << d.op << ' ' << d.dtype << ' ' << d.redop << ' ' << n << ' ' << d.count;
+    k << "tiles " << d.op << ' ' << d.dtype << ' ' << d.redop << ' ' << n << ' ' << d.count;
     return k.str();
 }
 

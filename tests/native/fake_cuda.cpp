@@ -103,6 +103,16 @@ cudaError_t cudaGraphDestroy(cudaGraph_t g) {
     free(g);
     return cudaSuccess;
 }
+cudaError_t cudaGetDeviceProperties(cudaDeviceProp* p, int) {
+    memset(p, 0, sizeof(*p));
+    strcpy(p->name, "fake GPU");
+    return cudaSuccess;
+}
+cudaError_t cudaEventCreate(cudaEvent_t* e) { return cudaEventCreateWithFlags(e, 0); }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
+    *ms = 1.0f;
+    return cudaSuccess;
+}
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) {
     FAKE_CALL("cudaEventCreateWithFlags");
     *e = (cudaEvent_t)malloc(64);

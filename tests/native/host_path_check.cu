@@ -3,6 +3,8 @@
 // Usage: host_path_check SCENARIO
 #include "fake_cuda.h"
 
+#include <unistd.h>
+
 #include <chrono>
 #include <functional>
 
@@ -238,6 +240,25 @@ static void captured() {
     gpumpi_plan_destroy(p);
 }
 
+// The tuner measures again what a file has from before some schedules ran as
+// tiles, and reads what it wrote itself.
+static void tuner_file() {
+    Job_* j = make(1, SMALL);
+    char path[] = "/tmp/host_path_tuneXXXXXX";
+    FILE* f = fdopen(mkstemp(path), "w");
+    for (int t : {64, 128, 256, 512, 1024}) fprintf(f, "fake GPU|3 13 2 4 %zu %d|2 0.01\n", SMALL, t);
+    fclose(f);
+    gpumpi_tune_opts opts = {1, path, 0};
+    const uint64_t before = gpumpi_kernel_launches();
+    int threads = 0, algo = 0;
+    CHECK(gpumpi_autotune(j->descs.data(), 1, &opts, nullptr, &threads, &algo) == 0, "%s", gpumpi_last_error());
+    CHECK(algo == 1 && gpumpi_kernel_launches() > before, "schedule %d", algo);   // all take as long: the first
+    const uint64_t once = gpumpi_kernel_launches();
+    CHECK(gpumpi_autotune(j->descs.data(), 1, &opts, nullptr, &threads, &algo) == 0, "%s", gpumpi_last_error());
+    CHECK(algo == 1 && gpumpi_kernel_launches() == once, "schedule %d", algo);
+    remove(path);
+}
+
 // A call that fails half way reports it, and nothing that it put on other streams outlives a wait for the caller's.
 static void errors() {
     int failed = 0;
@@ -402,7 +423,7 @@ static void failed_plans() {
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
         {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns},
-        {"first_calls", first_calls}, {"captured", captured}, {"errors", errors},
+        {"first_calls", first_calls}, {"captured", captured}, {"tuner_file", tuner_file}, {"errors", errors},
         {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans},
         {"devices", devices}, {"failed_plans", failed_plans}};
     fake::state().kernel_spans = kernel_spans;

@@ -39,7 +39,7 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["tables", "uploaded", "retry", "order", "turns", "first_calls", "captured",
+@pytest.mark.parametrize("scenario", ["tables", "uploaded", "retry", "order", "turns", "first_calls", "captured", "tuner_file",
                                       "errors", "levels", "random_levels", "long_plans", "devices", "failed_plans"])
 def test_host_path(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=120)
