@@ -1172,7 +1172,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     // 32768 with 2 / 3 / 4 362, 319, 345).  At most 2 MB: 2^20 with 0.5 MiB 10.18 ms, 1
     // MiB 9.90, 2 MB 9.79, 8 MB 9.92.
     const double total = level.bytes;
-    const bool lone = level.calls == 1 && total <= SP_LONE_BYTES;
+    const bool alone = level.calls == 1, lone = alone && total <= SP_LONE_BYTES, large = alone && !lone;
     const double waves = level.calls == 1 || total >= 1.1e9 ? 3 : total < 3.2e8 ? 1.75 : 2;
     const double target = lone ? total / (SP_SMS * 2)
                                : std::min(2e6, std::max(16384.0, total / (SP_SMS * SP_BLOCKS_PER_SM * waves)));
@@ -1236,8 +1236,10 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         const u64 nrows = split(hi / V, SP_T);
         // Above SP_TAB ranks gather tiles stay where they all run at once, which is
         // short calls; then SP_ROWS in passes, with as few elements a tile as keep the SMs
-        // busy (512 bytes at most); from 1 MiB chunks of a warp, whose loads never pause
-        // (from 96 KiB for odd buffers of 1- and 2-byte types, which passes load one by one).
+        // busy (512 bytes at most); from 576 KiB chunks of a warp, whose loads never pause
+        // (1- and 2-byte types from 1 MiB, from 96 KiB in odd buffers, which passes load one by one;
+        // Reduce of FP64, passes / chunks: 512 ranks of 63476 95 / 124, of 97656 138 / 127
+        // us, 320 of 50780 75 / 102, of 101560 93 / 83).
         // One call, Reduce of FP64 unless named, gather / passes of 32, 64, 128 elements
         // / a warp's chunks of 512 bytes, us: 1024 ranks of 2000 48 / 51, 58, 73 / 240,
         // of 20000 298 / 107, 86, 107 / 254, of 60000 835 / 216, 174, 166 / 257, of
@@ -1274,8 +1276,11 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         // a lone fold of buffers aligned to their elements (4 ranks of 2 * 10^6 int32:
         // gather 19.4, rows 13.7 us; 64 of 62497 FP64, 500 KB each: 20.0, 24.6 us)
         const u64 inner = hi > lo ? (hi - lo) * esize : 0;
-        const bool alone = level.calls == 1;
-        const u64 least = many && alone ? aligned || esize >= 4 ? 1048576 : 98304
+        // From 250 MB a single call always goes by rows: even of 256 ranks it has 1000
+        // chunks, a gather tile of many ranks a few elements (Reduce of 256 ranks of
+        // 1015624 uint8: gather 682, rows 93 us; Allreduce of 160 of 812500 446, 96).
+        const u64 least = many && alone ? esize >= 4 ? 589824 : aligned ? 1048576 : 98304
+                          : large      ? 0
                           : lone        ? aligned ? ~0ull : 524288
                           : many        ? std::max<u64>(32768 * esize, rows_min(aligned, total))
                                         : rows_min(aligned, total);
@@ -1295,7 +1300,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
                 c.group = 1;
             }
             while (many && alone && !passes && chunk > 128 && inner < 580ull * chunk) chunk /= 2;
-            while (!(many && alone) && !passes && chunk > 32 * (u32)esize && row * chunk * SP_WARPS > 4 * target) chunk /= 2;
+            while (!(many && alone) && !large && !passes && chunk > 32 * (u32)esize && row * chunk * SP_WARPS > 4 * target) chunk /= 2;
             c.per = chunk / esize;
             c.ub = chunk + (aligned ? 0 : 16);
             c.batch = std::min(c.nsrc, rows_part(c.nsrc) / (SP_GROUPS * c.ub));
@@ -1309,6 +1314,12 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
                 c.rows = (u32)round_up(split(chunks, k * SP_SMS), SP_WARPS);
             }
             if (lone && many) c.rows = (u32)split(chunks, 4 * SP_SMS);
+            // a large call: equal tiles in whole waves, at most a chunk for each warp (chunks
+            // that are halved until they make three tiles for each block, as among other
+            // calls / so, us: Reduce of FP64, 256 ranks of 126952 132 / 81, of 195312 226 /
+            // 119, 320 of 156248 202 / 124, 64 of 1562501 229 / 209; Allreduce of 256 of 97656
+            // 172 / 96; the rank blocks took 121, 156, 186, 480 and 152)
+            if (large && c.nsrc >= 16) c.rows = (u32)split(chunks, 4 * SP_SMS * split(chunks, 4 * SP_SMS * SP_WARPS));
             if (passes) c.rows = 1;
             c.ntiles = (u32)((chunks + c.rows - 1) / c.rows);
             c.tile_bytes = (u32)(row * chunk * c.rows);
@@ -1359,6 +1370,12 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         // MB 41 / 45), unless 4-byte units have to go one at a time (64 MB 23.8 / 17.1)
         move = bytes >= SP_MOVE_BYTES && (c.ub < 4 || (c.ub == 4 && !chunks && total >= 8e6));
         if (move) even = total < 4e6 ? SP_SMS : total < 3e7 ? 2 * SP_SMS : 4 * SP_SMS;
+    } else if (large && a2a && c.ub == 16) {
+        // The same holds for 16-byte units of larger calls, in tiles of 128 KiB (FP64, 128
+        // ranks, SP_MOVE / SP_COPY: 400 MB 90 / 68 us, 1.6 GB 281 / 252, 4 GB 666 / 622; 200
+        // ranks, 4 GB 670 / 641; tiles of 300 KB 71, 259, 638, of 2 MB 78, 298, 632).
+        // Rank blocks took 254 and 606 us for the second and the third.
+        move = false;
     } else if (lone) {
         // Bulk copies need the call to be large and a few hundred pieces (Allgather of
         // 64 ranks, 100 MB: SP_MOVE 18.1, SP_FAN 26, SP_COPY 23.5 us; 32 MB 8.7, 9.0, 8.6;
@@ -1371,7 +1388,9 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         if (move && units16) even = SP_SMS;
     }
     if (move) {
-        const u64 longest = a2a ? SP_PIECE : SP_FAN_PIECE;
+        // a large call has warps enough for one long row each (Alltoall of odd FP64 buffers,
+        // pieces of 1920 / 6016 bytes: 128 ranks, 800 MB 165 / 150, 4 GB 722 / 646 us)
+        const u64 longest = a2a && !large ? SP_PIECE : SP_FAN_PIECE;
         c.kind = SP_MOVE;
         c.cold = total >= 1e8;
         c.nu = bytes;
@@ -1433,6 +1452,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         const u64 items = (u64)c.ndst * c.nsrc * split(units, item);
         u64 per = step * (u64)std::max(1.0, target / (2.0 * step * item * c.ub));
         if (lone) per = round_up(split(items, even), step);
+        if (large && a2a && c.ub == 16) per = 4096;
         c.per = (u32)per;
         c.ntiles = (u32)split(items, per);
     }

@@ -1,0 +1,162 @@
+"""Forms of tiles that it takes a large call or an odd length to reach.
+
+Each call runs as tiles and is compared, byte for byte, with the same fold or
+copy by PyTorch on the device; the bytes around every buffer stay untouched.
+tests/test_spread_cover.py checks on the CPU that these sizes reach the form
+they are meant for.
+"""
+import importlib.util
+import os
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GUARD = 64   # bytes around each buffer
+
+
+@pytest.fixture(scope="module")
+def api(gpu_built):
+    spec = importlib.util.spec_from_file_location("gpumpi_coll", os.path.join(gpu_built.PKG, "gpumpi_coll.py"))
+    mod = importlib.util.module_from_spec(spec)
+    sys.modules[spec.name] = mod
+    spec.loader.exec_module(mod)
+    return mod, mod.bind(gpu_built.load_library())
+
+
+class Rows:
+    """P buffers of n elements in one allocation, buffer r starting r * skew elements past a 16-byte boundary."""
+
+    def __init__(self, p, n, dt, skew, seed=None):
+        import torch
+
+        self.dt = getattr(torch, dt)
+        es = torch.empty(0, dtype=self.dt).element_size()
+        self.bytes = n * es
+        step = (self.bytes + 15) // 16 * 16 + 2 * GUARD + 16
+        self.mem = torch.empty(p * step, dtype=torch.uint8, device="cuda")
+        self.mem.fill_(0xA5)
+        self.at = [r * step + GUARD + r * skew * es % 16 for r in range(p)]
+        if seed is not None:
+            g = torch.Generator(device="cuda").manual_seed(seed)
+            for r in range(p):
+                row = self.row(r)
+                if dt.startswith("float"):
+                    row.uniform_(-1.5, 1.5, generator=g)
+                else:
+                    row.random_(0, 200, generator=g)
+        self.ptrs = [self.mem.data_ptr() + a for a in self.at]
+
+    def row(self, r):
+        m = self.mem[self.at[r]:self.at[r] + self.bytes]
+        if m.data_ptr() % m.new_empty(0, dtype=self.dt).element_size():
+            raise AssertionError("alignment")
+        return _typed(m, self.dt)
+
+    def outside_untouched(self):
+        end = 0
+        for a in self.at + [len(self.mem)]:
+            assert (self.mem[end:a] == 0xA5).all(), "bytes around the buffers changed"
+            end = a + self.bytes
+
+
+def _typed(m, dt):
+    """Bytes as elements of dt; the storage offset is a multiple of the element's size."""
+    import torch
+
+    if dt == torch.uint8:
+        return m
+    es = torch.empty(0, dtype=dt).element_size()
+    whole = torch.empty(0, dtype=dt, device="cuda").set_(m.untyped_storage(), m.storage_offset() // es, (len(m) // es,))
+    assert whole.data_ptr() == m.data_ptr()
+    return whole
+
+
+def _same(a, b):
+    import torch
+
+    return torch.equal(a.contiguous().view(torch.uint8), b.contiguous().view(torch.uint8))
+
+
+def _fold(xs, p, op):
+    import torch
+
+    acc = xs(0).clone()
+    for q in range(1, p):
+        x = xs(q)
+        acc = {"sum": lambda: x + acc, "max": lambda: torch.where(x > acc, x, acc),
+               "min": lambda: torch.where(x > acc, acc, x)}[op]()
+    return acc
+
+
+def _launch(api, descs, batched):
+    import torch
+
+    coll, lib = api
+    plan = coll.Plan(lib, descs, threads=64, batched=batched)
+    plan.launch()
+    torch.cuda.synchronize()
+    assert coll.status(lib) is None
+    plan.close()
+
+
+class Call:
+    def __init__(self, api, kind, p, n, dt, skew, op="sum", values=None):
+        coll, lib = api
+        self.kind, self.p, self.n, self.op, self.root = kind, p, n, op, p // 2
+        self.keep = []
+        self.comm = coll.Comm(lib, p)
+        ns = n * p if kind == "alltoall" else n
+        nr = n * p if kind in ("alltoall", "allgather") else n
+        self.send = Rows(p, ns, dt, skew, seed=p + n) if kind != "bcast" else None
+        # of a Reduce only the root's buffer is used
+        self.recv = Rows(p if kind != "reduce" else 1, nr, dt, 3 * skew, seed=n if kind == "bcast" else None)
+        if values is not None:
+            values(self.send)
+        if kind == "bcast":
+            self.want = self.recv.row(self.root).clone()
+        code = {"bcast": coll.COLL_BCAST, "reduce": coll.COLL_REDUCE, "allreduce": coll.COLL_ALLREDUCE,
+                "alltoall": coll.COLL_ALLTOALL, "allgather": coll.COLL_ALLGATHER}[kind]
+        red = {"sum": coll.OP_SUM, "max": coll.OP_MAX, "min": coll.OP_MIN}[op]
+        self.desc = coll.make_desc(self.comm, code, dt, n, self.send.ptrs if self.send else None,
+                                   self.recv.ptrs if kind != "reduce" else self.recv.ptrs * p, red, self.root, self.keep)
+
+    def check(self):
+        p, n = self.p, self.n
+        if self.kind == "bcast":
+            for r in range(p):
+                assert _same(self.recv.row(r), self.want), "rank %d" % r
+        elif self.kind in ("reduce", "allreduce"):
+            want = _fold(self.send.row, p, self.op)
+            for r in range(len(self.recv.at)):
+                assert _same(self.recv.row(r), want), "rank %d" % r
+        else:
+            import torch
+
+            sent = [self.send.row(q) for q in range(p)]
+            for r in range(p):
+                want = torch.cat([x[r * n:(r + 1) * n] for x in sent] if self.kind == "alltoall" else sent)
+                assert _same(self.recv.row(r), want), "rank %d" % r
+        self.recv.outside_untouched()
+        if self.send:
+            self.send.outside_untouched()
+        self.comm.close()
+
+
+# calls alone in their launch
+ALONE = [
+    # more than 250 MB
+    ("reduce", 256, 126952, "float64", 0), ("reduce", 256, 126953, "float64", 1), ("reduce", 256, 1015624, "uint8", 0),
+    ("allreduce", 160, 812500, "uint8", 0), ("allreduce", 256, 97656, "float64", 0), ("reduce", 320, 101560, "float64", 0),
+    ("allreduce", 17, 2000001, "int32", 1), ("reduce", 512, 97657, "float64", 1),
+    ("alltoall", 128, 1524, "float64", 0), ("alltoall", 31, 60000, "int32", 0), ("alltoall", 128, 1525, "float64", 1),
+    ("alltoall", 31, 60001, "int32", 1), ("alltoall", 7, 2500001, "uint8", 1), ("alltoall", 128, 20, "float64", 0),
+]
+
+
+@pytest.mark.parametrize("kind,p,n,dt,skew", ALONE)
+def test_large_calls(api, kind, p, n, dt, skew):
+    call = Call(api, kind, p, n, dt, skew, "max" if dt == "uint8" and "reduce" in kind else "sum")
+    _launch(api, [call.desc], True)
+    call.check()

@@ -48,6 +48,13 @@ FORMS = [
     ("allreduce", 512, 20001, "i4", 1, "passes"), ("allreduce", 640, 700000, "u1", 0, "passes"),
     ("allreduce", 640, 700001, "u1", 1, "rows-many"), ("allreduce", 257, 160003, "f8", 1, "rows-many"),
     ("allreduce", 769, 165000, "f8", 0, "rows-many"), ("allreduce", 2048, 130001, "i4", 1, "passes"),
+    ("reduce", 256, 126952, "f8", 0, "rows"), ("reduce", 256, 126953, "f8", 1, "rows"),
+    ("reduce", 256, 1015624, "u1", 0, "rows"), ("allreduce", 160, 812500, "u1", 0, "rows"),
+    ("allreduce", 256, 97656, "f8", 0, "rows"), ("reduce", 320, 101560, "f8", 0, "rows-many"),
+    ("allreduce", 17, 2000001, "i4", 1, "rows"), ("reduce", 512, 97657, "f8", 1, "rows-many"),
+    ("alltoall", 128, 1524, "f8", 0, "copy"), ("alltoall", 31, 60000, "i4", 0, "copy"),
+    ("alltoall", 128, 1525, "f8", 1, "move-alltoall"), ("alltoall", 31, 60001, "i4", 1, "move-alltoall"),
+    ("alltoall", 7, 2500001, "u1", 1, "move-alltoall"), ("alltoall", 128, 20, "f8", 0, "copy"),
 ]
 
 
