@@ -1134,6 +1134,12 @@ static u64 lone_gather(u64 n, u64 step, u64 fits) {
     return 0;
 }
 
+// Elements from which the rest of a fold of 1- or 2-byte elements goes on its own
+// (Reduce of uint8 of odd lengths, rank blocks / single elements / so, us: 3 ranks of
+// 3001, four calls 55 / 10.3 / 3.5; 64 of 600001 66 / 57 / 12; 256 of 40001 96 / 29 / 5.3,
+// of 600001 651 / 382 / 41).
+constexpr u64 GATHER_REST = 1024;
+
 static bool is_fold(int op) { return op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE; }
 
 bool SpreadBuilder::covers(const gpumpi_coll_desc& d, int P, int esize) {
@@ -1230,7 +1236,14 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         };
         // whole vectors, or what lies 16 bytes and more from both ends of the buffers
         const u64 lo = aligned ? 0 : V, hi = aligned ? n / V * V : n > 2 * V ? n - V : 0;
-        const u64 step = aligned && n % V == 0 ? V : 1;
+        // 1- and 2-byte types take gather tiles of whole vectors and one of the rest: loaded
+        // one by one their elements are most of a tile's work
+        const bool rest = aligned && esize < 4 && n % V && n >= GATHER_REST;
+        const u64 step = aligned && (rest || n % V == 0) ? V : 1;
+        auto gather_all = [&](u64 per) {
+            gather(0, rest ? hi : n, per, per);
+            if (rest) gather(hi, n - hi, n - hi, n - hi);
+        };
         const double fits = (double)SP_RING / ((double)P * esize);
         const u64 most = (u64)fits / step * step;   // elements of the largest gather tile
         const u64 nrows = split(hi / V, SP_T);
@@ -1255,7 +1268,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         if (lone) {
             const u64 m = lone_gather(n, step, most);
             if (m) {
-                gather(0, n, m, m);
+                gather_all(m);
                 return;
             }
         }
@@ -1334,7 +1347,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
             // of 124992 float32, 64 elements 40.4, 52 44.5 us)
             const u64 m = round_up(split(n, 8 * SP_SMS), step);
             const u64 per = m >= 48 && m <= most ? m : most;
-            gather(0, n, per, per);
+            gather_all(per);
             return;
         }
         // A warp's addition takes the same time however many lanes add: fill it as
@@ -1343,7 +1356,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         const double fill = std::min(32.0, std::ceil(level.folded / (152 * SP_BLOCKS_PER_SM * 2)));
         const double per = std::min(fits, std::max(target / 2 / ((double)P * esize), fill));
         const u64 m = std::max(step, (u64)std::min(per, (double)n) / step * step);
-        gather(0, n, m, m);
+        gather_all(m);
         return;
     }
     const bool a2a = d.op == GPUMPI_COLL_ALLTOALL;

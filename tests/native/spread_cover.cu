@@ -235,6 +235,11 @@ static void check(int op, int P, u64 n, int dtype, int es, int skew, int calls, 
     // than two tiles for each block (FP64 additions cost the same for 2 lanes as for 32)
     if (P > SP_TAB && (op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE) && es > 1)
         for (const SpreadCall& c : b.calls) CHECK(c.kind != SP_GATHER || c.per >= 32 || c.ntiles <= 2 * 4 * 152);
+    // whole buffers of 1- and 2-byte elements on 16-byte boundaries do not go element by
+    // element, whatever their length: at most their last 15 bytes do
+    const bool fold = op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE;
+    if (skew == 0 && es < 4 && fold && n >= 1024)
+        for (const SpreadCall& c : b.calls) CHECK(c.kind != SP_GATHER || c.ub == 16 || c.nu * es < 16);
 }
 
 int main(int argc, char** argv) {

@@ -152,6 +152,9 @@ ALONE = [
     ("allreduce", 17, 2000001, "int32", 1), ("reduce", 512, 97657, "float64", 1),
     ("alltoall", 128, 1524, "float64", 0), ("alltoall", 31, 60000, "int32", 0), ("alltoall", 128, 1525, "float64", 1),
     ("alltoall", 31, 60001, "int32", 1), ("alltoall", 7, 2500001, "uint8", 1), ("alltoall", 128, 20, "float64", 0),
+    # whole vectors of 1-byte elements and a rest
+    ("reduce", 3, 1025, "uint8", 0), ("reduce", 128, 600001, "uint8", 0),
+    ("allreduce", 256, 40001, "uint8", 0), ("allreduce", 64, 150001, "uint8", 0),
 ]
 
 

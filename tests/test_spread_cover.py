@@ -55,6 +55,7 @@ FORMS = [
     ("alltoall", 128, 1524, "f8", 0, "copy"), ("alltoall", 31, 60000, "i4", 0, "copy"),
     ("alltoall", 128, 1525, "f8", 1, "move-alltoall"), ("alltoall", 31, 60001, "i4", 1, "move-alltoall"),
     ("alltoall", 7, 2500001, "u1", 1, "move-alltoall"), ("alltoall", 128, 20, "f8", 0, "copy"),
+    ("reduce", 3, 1025, "u1", 0, "gather"), ("reduce", 128, 600001, "i2", 0, "gather"),
 ]
 
 
