@@ -1139,6 +1139,7 @@ static u64 lone_gather(u64 n, u64 step, u64 fits) {
 // 3001, four calls 55 / 10.3 / 3.5; 64 of 600001 66 / 57 / 12; 256 of 40001 96 / 29 / 5.3,
 // of 600001 651 / 382 / 41).
 constexpr u64 GATHER_REST = 1024;
+constexpr u64 RAGGED_BYTES = 4096;   // the same for the end of a Bcast
 
 static bool is_fold(int op) { return op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE; }
 
@@ -1212,7 +1213,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     ptrs.insert(ptrs.end(), dst.begin(), dst.end());
     c.nsrc = (u32)src.size();
     c.ndst = (u32)dst.size();
-    const u64 bytes = d.count * (u64)esize;
+    u64 bytes = d.count * (u64)esize;
     if (is_fold(d.op)) {
         int ft = fold_type(d.dtype);
         if (d.redop == GPUMPI_OP_SUM || d.redop == GPUMPI_OP_PROD) {
@@ -1361,6 +1362,24 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     }
     const bool a2a = d.op == GPUMPI_COLL_ALLTOALL;
     c.rs = a2a ? bytes : 0;
+    // The end alone of a Bcast's block would make its units 1 or 2 bytes: it goes as a
+    // gather tile of one source (uint8 to 128 ranks, rank blocks / with its own units /
+    // so, us: 600001 elements 21 / 26 / 15, 2400001 60 / 164 / 56; to 256 ranks 35 / 83 /
+    // 35, 107 / 326 / 104; 10001 to 64 ranks 6.2 / 4.1 / 2.6).
+    if (c.nsrc == 1 && bits % 16 == 0 && bytes % 4 && bytes >= RAGGED_BYTES) {
+        SpreadCall end = c;
+        end.kind = SP_GATHER;
+        end.fn = (esize == 1 ? FT_I8 : FT_I16) * 4 + GPUMPI_OP_MAX;
+        end.off = bytes / 16 * 16;
+        end.nu = bytes % 16 / esize;
+        end.per = (u32)end.nu;
+        end.rs = 0;
+        end.ub = esize;
+        end.ntiles = 1;
+        end.tile_bytes = (u32)((1 + c.ndst) * (bytes % 16));
+        calls.push_back(end);
+        bytes = end.off;
+    }
     bits |= bytes;
     const bool units16 = bits % 16 == 0;
     c.ub = units16 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;

@@ -240,6 +240,8 @@ static void check(int op, int P, u64 n, int dtype, int es, int skew, int calls, 
     const bool fold = op == GPUMPI_COLL_REDUCE || op == GPUMPI_COLL_ALLREDUCE;
     if (skew == 0 && es < 4 && fold && n >= 1024)
         for (const SpreadCall& c : b.calls) CHECK(c.kind != SP_GATHER || c.ub == 16 || c.nu * es < 16);
+    if (skew == 0 && es < 4 && op == GPUMPI_COLL_BCAST && n * es >= 4096)
+        for (const SpreadCall& c : b.calls) CHECK((c.kind != SP_FAN && c.kind != SP_COPY) || c.ub >= 4);
 }
 
 int main(int argc, char** argv) {

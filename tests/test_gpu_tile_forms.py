@@ -155,6 +155,9 @@ ALONE = [
     # whole vectors of 1-byte elements and a rest
     ("reduce", 3, 1025, "uint8", 0), ("reduce", 128, 600001, "uint8", 0),
     ("allreduce", 256, 40001, "uint8", 0), ("allreduce", 64, 150001, "uint8", 0),
+    # a Bcast whose length is odd
+    ("bcast", 200, 4097, "uint8", 0), ("bcast", 128, 2400001, "uint8", 0),
+    ("bcast", 256, 957025, "uint8", 0),
 ]
 
 

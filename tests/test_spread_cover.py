@@ -56,6 +56,7 @@ FORMS = [
     ("alltoall", 128, 1525, "f8", 1, "move-alltoall"), ("alltoall", 31, 60001, "i4", 1, "move-alltoall"),
     ("alltoall", 7, 2500001, "u1", 1, "move-alltoall"), ("alltoall", 128, 20, "f8", 0, "copy"),
     ("reduce", 3, 1025, "u1", 0, "gather"), ("reduce", 128, 600001, "i2", 0, "gather"),
+    ("bcast", 200, 4097, "u1", 0, "gather"), ("bcast", 128, 2400001, "u1", 0, "move-fan"),
 ]
 
 
