@@ -1066,6 +1066,13 @@ static int fold_type(int dtype) {
 // bytes cannot take the ring and do so from 512 bytes.
 constexpr u64 SP_MOVE_UNITS = 8192;
 constexpr u64 SP_MOVE_BYTES = 512;
+// Units of 1 byte of many ranks sooner: their rows fill every warp, and cost as much
+// as some 250 units (odd uint8 Alltoall, SP_COPY / SP_MOVE, us: 64 ranks, blocks of 385
+// bytes 6.3 / 6.8, 501 7.4 / 7.1; 256 ranks, 193 34 / 42, 257 44 / 43, 501 84 / 50; 1000
+// ranks, 65 266 / 526, 129 387 / 404, 257 820 / 427, 501 1641 / 470, rank blocks 885).
+static u64 move_bytes(u32 unit, u64 blocks) {
+    return unit > 1 || blocks < 65536 ? SP_MOVE_BYTES : blocks < 524288 ? 257 : 144;
+}
 constexpr u64 SP_PIECE = 1920;       // longest piece: three fit a warp's part of the ring
 
 // Bytes of a rank's vector from which a fold goes by rows instead of gather
@@ -1383,7 +1390,8 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     bits |= bytes;
     const bool units16 = bits % 16 == 0;
     c.ub = units16 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
-    bool move = bytes >= (a2a ? c.ub >= 4 ? SP_MOVE_UNITS : SP_MOVE_BYTES : fan_min(units16, total));
+    const u64 move_min = c.ub >= 4 ? SP_MOVE_UNITS : move_bytes(c.ub, (u64)c.nsrc * c.ndst);
+    bool move = bytes >= (a2a ? move_min : fan_min(units16, total));
     bool fan = !a2a && bytes / c.ub >= 2 * SP_T;
     // SP_COPY by chunks, where at most a quarter of the lanes' turns is empty: for
     // 4-byte units (int32 Alltoall of the 16 communicators, 30001 per rank 73.9 ->
@@ -1400,7 +1408,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         // bytes and more (64 ranks, SP_COPY / SP_MOVE: 16-byte units, 16 MB 4.1 / 8.1 us,
         // 64 MB 8.6 / 14.3; 8-byte units 200 MB 40 / 45; 4-byte units 64 MB 11.1 / 17.1, 200
         // MB 41 / 45), unless 4-byte units have to go one at a time (64 MB 23.8 / 17.1)
-        move = bytes >= SP_MOVE_BYTES && (c.ub < 4 || (c.ub == 4 && !chunks && total >= 8e6));
+        move = bytes >= move_bytes(c.ub, (u64)c.nsrc * c.ndst) && (c.ub < 4 || (c.ub == 4 && !chunks && total >= 8e6));
         if (move) even = total < 4e6 ? SP_SMS : total < 3e7 ? 2 * SP_SMS : 4 * SP_SMS;
     } else if (large && a2a && c.ub == 16) {
         // The same holds for 16-byte units of larger calls, in tiles of 128 KiB (FP64, 128

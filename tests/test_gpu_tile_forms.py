@@ -158,6 +158,9 @@ ALONE = [
     # a Bcast whose length is odd
     ("bcast", 200, 4097, "uint8", 0), ("bcast", 128, 2400001, "uint8", 0),
     ("bcast", 256, 957025, "uint8", 0),
+    # short odd blocks
+    ("alltoall", 256, 257, "uint8", 1), ("alltoall", 256, 256, "uint8", 1),
+    ("alltoall", 730, 145, "uint8", 1),
 ]
 
 

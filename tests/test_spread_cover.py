@@ -57,6 +57,8 @@ FORMS = [
     ("alltoall", 7, 2500001, "u1", 1, "move-alltoall"), ("alltoall", 128, 20, "f8", 0, "copy"),
     ("reduce", 3, 1025, "u1", 0, "gather"), ("reduce", 128, 600001, "i2", 0, "gather"),
     ("bcast", 200, 4097, "u1", 0, "gather"), ("bcast", 128, 2400001, "u1", 0, "move-fan"),
+    ("alltoall", 256, 257, "u1", 1, "move-alltoall"), ("alltoall", 256, 256, "u1", 1, "copy"),
+    ("alltoall", 730, 145, "u1", 1, "move-alltoall"), ("alltoall", 256, 255, "i2", 1, "copy"),
 ]
 
 
