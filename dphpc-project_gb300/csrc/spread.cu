@@ -1104,7 +1104,7 @@ static u64 rows_min(bool aligned, double total) {
 // and 420 MB 87.5 against 76.5; the 16-communicator batch at 500001 per rank 5364
 // against 5104, at 50001 561 against 565.  (Lone calls up to SP_LONE_BYTES have
 // their own rule in add().)
-constexpr u64 SP_FAN_PIECE = 6272;
+constexpr u64 SP_FAN_PIECE = 6272, SP_HALF_PIECE = 3072;
 constexpr double SP_FAN_ALIGNED = 1024, SP_FAN_ODD = 8;
 static u64 fan_min(bool units16, double total) {
     if (units16) return total >= 2e8 ? 8192 : ~0ull;
@@ -1392,7 +1392,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     c.ub = units16 ? 16 : bits % 8 == 0 ? 8 : bits % 4 == 0 ? 4 : bits % 2 == 0 ? 2 : 1;
     const u64 move_min = c.ub >= 4 ? SP_MOVE_UNITS : move_bytes(c.ub, (u64)c.nsrc * c.ndst);
     bool move = bytes >= (a2a ? move_min : fan_min(units16, total));
-    bool fan = !a2a && bytes / c.ub >= 2 * SP_T;
+    bool fan = !a2a && bytes / c.ub >= 2 * SP_T, halves = false;
     // SP_COPY by chunks, where at most a quarter of the lanes' turns is empty: for
     // 4-byte units (int32 Alltoall of the 16 communicators, 30001 per rank 73.9 ->
     // 53.4 us, 100003 182 -> 160; the whole batch at 50000 511 -> 505) and lone calls
@@ -1423,14 +1423,20 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         // once for several destinations, which pays once the stores no longer fit the
         // same few tiles (Bcast of 16-byte units to 16 ranks, SP_FAN / SP_COPY: 8 MB 6.1 /
         // 4.0 us, 32 MB 7.6 / 8.3; of 8-byte units 8 MB 3.6 / 5.2, 32 MB 7.0 / 12.6).
+        // (From 160 MB a Bcast of fewer goes in pieces of half the length: 200 ranks of
+        // 900000 bytes SP_FAN 37.4, SP_MOVE 29.6, half 29.8; of 1225000 49.0, 44.4, 39.6; 256
+        // of 957024 58.3, 54.5, 42.3; 512 of 410144 49.1, 48.0, 34.3; rank blocks 256 of
+        // 957024 49 us.)
         move = total >= 8e7 && bytes >= 2048 && split(bytes, SP_FAN_PIECE) * c.nsrc >= 200;
+        halves = !move && units16 && c.nsrc == 1 && total >= 1.6e8;
+        move = move || halves;
         fan = fan && (!units16 || total >= 1.6e7);
         if (move && units16) even = SP_SMS;
     }
     if (move) {
         // a large call has warps enough for one long row each (Alltoall of odd FP64 buffers,
         // pieces of 1920 / 6016 bytes: 128 ranks, 800 MB 165 / 150, 4 GB 722 / 646 us)
-        const u64 longest = a2a && !large ? SP_PIECE : SP_FAN_PIECE;
+        const u64 longest = a2a && !large ? SP_PIECE : halves ? SP_HALF_PIECE : SP_FAN_PIECE;
         c.kind = SP_MOVE;
         c.cold = total >= 1e8;
         c.nu = bytes;

@@ -161,6 +161,8 @@ ALONE = [
     # short odd blocks
     ("alltoall", 256, 257, "uint8", 1), ("alltoall", 256, 256, "uint8", 1),
     ("alltoall", 730, 145, "uint8", 1),
+    # pieces of half the length
+    ("bcast", 512, 51268, "float64", 0),
 ]
 
 

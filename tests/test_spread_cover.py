@@ -59,6 +59,7 @@ FORMS = [
     ("bcast", 200, 4097, "u1", 0, "gather"), ("bcast", 128, 2400001, "u1", 0, "move-fan"),
     ("alltoall", 256, 257, "u1", 1, "move-alltoall"), ("alltoall", 256, 256, "u1", 1, "copy"),
     ("alltoall", 730, 145, "u1", 1, "move-alltoall"), ("alltoall", 256, 255, "i2", 1, "copy"),
+    ("bcast", 256, 957025, "u1", 0, "move-fan"), ("bcast", 512, 51268, "f8", 0, "move-fan"),
 ]
 
 
