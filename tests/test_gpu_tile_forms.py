@@ -1,4 +1,4 @@
-"""Forms of tiles that it takes a large call or an odd length to reach.
+"""Forms of tiles that it takes a large call to reach, and values that a fold must not change.
 
 Each call runs as tiles and is compared, byte for byte, with the same fold or
 copy by PyTorch on the device; the bytes around every buffer stay untouched.
@@ -146,23 +146,23 @@ class Call:
 
 # calls alone in their launch
 ALONE = [
+    # vectors streamed, and rows of odd buffers
+    ("allreduce", 4, 1000000, "float64", 0), ("allreduce", 4, 1000001, "float64", 1), ("reduce", 64, 62497, "float64", 1),
+    ("reduce", 64, 70001, "float64", 1), ("allreduce", 20, 600001, "int32", 1),
+    # bulk copies to several destinations
+    ("bcast", 16, 750000, "float64", 0), ("bcast", 16, 750001, "float64", 1), ("bcast", 16, 6000001, "uint8", 1),
+    ("allgather", 100, 1000, "float64", 0), ("allgather", 100, 1001, "float64", 1), ("allgather", 100, 8001, "uint8", 1),
     # more than 250 MB
     ("reduce", 256, 126952, "float64", 0), ("reduce", 256, 126953, "float64", 1), ("reduce", 256, 1015624, "uint8", 0),
     ("allreduce", 160, 812500, "uint8", 0), ("allreduce", 256, 97656, "float64", 0), ("reduce", 320, 101560, "float64", 0),
     ("allreduce", 17, 2000001, "int32", 1), ("reduce", 512, 97657, "float64", 1),
     ("alltoall", 128, 1524, "float64", 0), ("alltoall", 31, 60000, "int32", 0), ("alltoall", 128, 1525, "float64", 1),
     ("alltoall", 31, 60001, "int32", 1), ("alltoall", 7, 2500001, "uint8", 1), ("alltoall", 128, 20, "float64", 0),
-    # whole vectors of 1-byte elements and a rest
-    ("reduce", 3, 1025, "uint8", 0), ("reduce", 128, 600001, "uint8", 0),
+    # 1-byte types: whole vectors and a rest, pieces of half the length, short odd blocks
+    ("bcast", 200, 4097, "uint8", 0), ("bcast", 128, 2400001, "uint8", 0), ("bcast", 256, 957025, "uint8", 0),
+    ("bcast", 512, 51268, "float64", 0), ("reduce", 3, 1025, "uint8", 0), ("reduce", 128, 600001, "uint8", 0),
     ("allreduce", 256, 40001, "uint8", 0), ("allreduce", 64, 150001, "uint8", 0),
-    # a Bcast whose length is odd
-    ("bcast", 200, 4097, "uint8", 0), ("bcast", 128, 2400001, "uint8", 0),
-    ("bcast", 256, 957025, "uint8", 0),
-    # short odd blocks
-    ("alltoall", 256, 257, "uint8", 1), ("alltoall", 256, 256, "uint8", 1),
-    ("alltoall", 730, 145, "uint8", 1),
-    # pieces of half the length
-    ("bcast", 512, 51268, "float64", 0),
+    ("alltoall", 256, 257, "uint8", 1), ("alltoall", 256, 256, "uint8", 1), ("alltoall", 730, 145, "uint8", 1),
 ]
 
 
@@ -171,3 +171,91 @@ def test_large_calls(api, kind, p, n, dt, skew):
     call = Call(api, kind, p, n, dt, skew, "max" if dt == "uint8" and "reduce" in kind else "sum")
     _launch(api, [call.desc], True)
     call.check()
+
+
+@pytest.mark.parametrize("skew", [0, 1])
+def test_bulk_copies_among_other_calls(api, skew):
+    """A level of more than 1 GB, in which odd buffers go by bulk copies too."""
+    calls = [Call(api, "bcast", 64, 1000000 + skew, "float64", skew), Call(api, "allgather", 24, 70000 + skew, "float64", skew),
+             Call(api, "allreduce", 5, 33333, "int32", skew)]
+    _launch(api, [c.desc for c in calls], True)
+    for c in calls:
+        c.check()
+
+
+BEYOND = (1 << 32) + 12345
+
+
+@pytest.mark.parametrize("kind,p,n,skew", [("bcast", 3, BEYOND, 1), ("bcast", 2, BEYOND // 16 * 16, 0),
+                                           ("allreduce", 2, BEYOND, 1), ("allreduce", 2, BEYOND // 16 * 16, 0),
+                                           ("alltoall", 2, BEYOND // 2, 1), ("alltoall", 2, BEYOND // 32 * 16, 0),
+                                           ("allgather", 2, BEYOND // 2, 1)])
+def test_buffers_beyond_4_gib(api, kind, p, n, skew):
+    call = Call(api, kind, p, n, "uint8", skew, "max")
+    _launch(api, [call.desc], False)
+    call.check()
+
+
+# gather tiles, vectors streamed, rows, passes over the sources, rows of many ranks
+SPECIAL = [(5, 1000, 0), (4, 1000000, 0), (4, 1000001, 1), (512, 20001, 1), (300, 160003, 1)]
+
+
+@pytest.mark.parametrize("p,n,skew", SPECIAL)
+@pytest.mark.parametrize("op", ["max", "min", "sum"])
+@pytest.mark.parametrize("dt", ["float64", "float32"])
+def test_special_values_through_folds(api, p, n, skew, op, dt):
+    """NaN, infinities, signed zeros and subnormals, in any order of ranks.  For
+    MAX and MIN an operand stays or goes as `x > acc` says, and the kept one's
+    bits are kept.  A NaN that is a sum has no sign of its own (rank blocks of
+    two schedules differ in it): sums have theirs in the same places, and the
+    same bits elsewhere."""
+    import torch
+
+    def values(rows):
+        tiny = torch.finfo(getattr(torch, dt)).tiny / 4
+        v = torch.tensor([float("nan"), float("inf"), -float("inf"), 0.0, -0.0, tiny, -tiny, 1.0, -1.0],
+                         dtype=getattr(torch, dt), device="cuda")
+        g = torch.Generator(device="cuda").manual_seed(n)
+        for r in range(p):
+            rows.row(r).copy_(v[torch.randint(0, len(v), (n,), device="cuda", generator=g)])
+
+    call = Call(api, "allreduce", p, n, dt, skew, op, values)
+    _launch(api, [call.desc], False)
+    if op != "sum":
+        call.check()
+        return
+    want = _fold(call.send.row, p, op)
+    none = torch.isnan(want)
+    for r in range(p):
+        got = call.recv.row(r)
+        assert torch.equal(torch.isnan(got), none) and _same(got[~none], want[~none]), "rank %d" % r
+    call.recv.outside_untouched()
+    call.comm.close()
+
+
+def test_dependent_calls_with_another_schedule(api):
+    """One call whose schedule tiles do not carry out keeps a plan of dependent
+    calls in rank blocks, in one launch, with flag rounds between the calls."""
+    import torch
+
+    coll, lib = api
+    p, n = 24, 5000
+    comm, keep = coll.Comm(lib, p), []
+    x, y, z = (Rows(p, n, "float64", 0, seed=s) for s in (1, None, None))
+    descs = [coll.make_desc(comm, coll.COLL_ALLREDUCE, "float64", n, a.ptrs, b.ptrs, coll.OP_SUM, 0, keep, algo)
+             for a, b, algo in ((x, y, 0), (y, z, 2))]
+    plan = coll.Plan(lib, descs, threads=128, batched=True)
+    assert not plan.launch_ordered
+    before = lib.gpumpi_kernel_launches()
+    plan.launch()
+    torch.cuda.synchronize()
+    assert coll.status(lib) is None
+    assert lib.gpumpi_kernel_launches() == before + 1
+    mid = _fold(x.row, p, "sum")
+    out = _fold(lambda q: mid, p, "sum")
+    for r in range(p):
+        assert _same(y.row(r), mid) and _same(z.row(r), out)
+    for t in (x, y, z):
+        t.outside_untouched()
+    plan.close()
+    comm.close()
