@@ -906,10 +906,13 @@ extern "C" int gpumpi_plan_capture(gpumpi_plan_t p, void* stream) {
     g_launches = before;
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(cap, &g);
+    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&p->exec, g, 0);
+    // its first replay need not bring it to the device (31.8 us launched, 33.3 without)
+    if (!rc && e == cudaSuccess && (cudaGraphUpload(p->exec, cap) != cudaSuccess || cudaStreamSynchronize(cap) != cudaSuccess))
+        cudaGetLastError();
     cudaStreamDestroy(cap);
     if (rc) return rc;
     CK(e);
-    CK(cudaGraphInstantiate(&p->exec, g, 0));
     p->graph = g;
     return GPUMPI_OK;
 }

@@ -90,6 +90,10 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long 
     *e = (cudaGraphExec_t)malloc(64);
     return cudaSuccess;
 }
+cudaError_t cudaGraphUpload(cudaGraphExec_t, cudaStream_t) {
+    FAKE_CALL("cudaGraphUpload");
+    return cudaSuccess;
+}
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t st) {
     FAKE_CALL("cudaGraphLaunch");
     fake::enqueue("graph", st, {});
