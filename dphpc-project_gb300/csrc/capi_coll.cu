@@ -496,8 +496,8 @@ std::mutex& stream_lock(cudaStream_t st) {
     return mu[(h >> 4 ^ h >> 10) % 64];
 }
 
-int launch_spread(SpreadArgs* args, cudaStream_t st) {
-    return launch_tiles((const void*)gpumpi_spread_kernel, args, args->ntiles, st);
+int launch_spread(SpreadArgs* args, cudaStream_t st, bool overlap = true) {
+    return launch_tiles((const void*)gpumpi_spread_kernel, args, args->ntiles, st, overlap);
 }
 
 }  // namespace
@@ -568,8 +568,10 @@ extern "C" int gpumpi_plan_create(const gpumpi_coll_desc* descs, int ndesc, int 
     return gpumpi_plan_create_ex(descs, ndesc, threads, batched, nullptr, out);
 }
 
-extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, int threads, int batched,
-                                     const int* plain_threads, gpumpi_plan_t* out) {
+// upload: the stream whose work brings the tables, for a plan that is launched
+// there only, first by plan_enqueue(p, st, true); null: they have arrived on return.
+static int create_plan(const gpumpi_coll_desc* descs, int ndesc, int threads, int batched, const int* plain_threads,
+                       const cudaStream_t* upload, gpumpi_plan_t* out) {
     if (!descs || ndesc <= 0 || !out) return GPUMPI_EINVAL;
     if (threads == 0) threads = 128;
     if (threads < 64 || threads > 1024 || threads % 32) return GPUMPI_EINVAL;
@@ -742,10 +744,14 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
         }
         at += spread[k].bytes();
     }
-    CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));
-    // a copy from pageable memory may return before it has arrived, and launches on
-    // any stream read the tables before they wait for anything
-    CK(cudaStreamSynchronize(cudaStreamLegacy));
+    if (upload) {
+        CK(cudaMemcpyAsync(base, h.data(), total, cudaMemcpyHostToDevice, *upload));   // staged on return
+    } else {
+        CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));
+        // a copy from pageable memory may return before it has arrived, and launches on
+        // any stream read the tables before they wait for anything
+        CK(cudaStreamSynchronize(cudaStreamLegacy));
+    }
     p->ndesc = ndesc;
     p->ncomm = ncomm;
     p->batched = batched;
@@ -805,7 +811,14 @@ extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, i
     return GPUMPI_OK;
 }
 
-static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
+extern "C" int gpumpi_plan_create_ex(const gpumpi_coll_desc* descs, int ndesc, int threads, int batched,
+                                     const int* plain_threads, gpumpi_plan_t* out) {
+    return create_plan(descs, ndesc, threads, batched, plain_threads, nullptr, out);
+}
+
+// first: the plan's tables arrive on `st` just before, so its first launch may not
+// start ahead of that; the later ones start when the first has.
+static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st, bool first = false) {
     const void* k = (const void*)gpumpi_plan_kernel;
     std::lock_guard<std::mutex> lock(stream_lock(st));
     if (p->batched) {
@@ -816,8 +829,9 @@ static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
             // of 4 ranks of 200 FP64 22.7 us, so 11.6; of 48 of 20000 38.4, 28.3; of 200
             // of 131072 517, 463; 400 calls of 8 ranks of one element 1481, 824.
             for (SpreadArgs& a : p->batch_tiles) {
-                int rc = launch_spread(&a, st);
+                int rc = launch_spread(&a, st, !first);
                 if (rc) return rc;
+                first = false;
             }
             return GPUMPI_OK;
         }
@@ -825,9 +839,10 @@ static int plan_enqueue(gpumpi_plan_t p, cudaStream_t st) {
     }
     for (int i = 0; i < p->ndesc; i++) {
         int rc = p->plain_spread[i] && p->plain_args[i].ordered
-                     ? launch_spread(&p->plain_tiles[i], st)
+                     ? launch_spread(&p->plain_tiles[i], st, !first)
                      : launch(k, p->plain_grid[i], p->plain_threads[i], p->plain_smem[i], &p->plain_args[i], st);
         if (rc) return rc;
+        first = false;
     }
     return GPUMPI_OK;
 }
@@ -1221,10 +1236,13 @@ extern "C" int gpumpi_plan_destroy(gpumpi_plan_t p) {
 
 extern "C" int gpumpi_api_status(char* msg, int len);
 static int one_shot(const gpumpi_coll_desc* descs, int ndesc, int threads, void* stream, int batched) {
+    // The tables come in the stream's order: a wait for them alone would be 7 us of a
+    // single call's 43 (rank blocks, which did without, 34).
     gpumpi_plan_t p = nullptr;
-    int rc = gpumpi_plan_create(descs, ndesc, threads, batched, &p);
+    cudaStream_t st = (cudaStream_t)stream;
+    int rc = create_plan(descs, ndesc, threads, batched, nullptr, &st, &p);
     if (rc) return rc;
-    rc = gpumpi_plan_launch(p, stream);
+    rc = plan_enqueue(p, st, true);
     cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
     gpumpi_plan_destroy(p);
     if (rc) return rc;

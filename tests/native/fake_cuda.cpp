@@ -136,11 +136,14 @@ cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t st) {
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* kernel, void** args) {
     FAKE_CALL("cudaLaunchKernelExC");
-    bool cooperative = false;
+    bool cooperative = false, overlap = false;
     for (unsigned i = 0; i < c->numAttrs; i++)
         cooperative = cooperative || (c->attrs[i].id == cudaLaunchAttributeCooperative && c->attrs[i].val.cooperative);
+    for (unsigned i = 0; i < c->numAttrs; i++)
+        overlap = overlap || (c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization &&
+                              c->attrs[i].val.programmaticStreamSerializationAllowed);
     fake::enqueue("launch", c->stream, s.kernel_spans ? s.kernel_spans(kernel, args) : std::vector<fake::Span>(),
-                  cooperative);
+                  cooperative, overlap);
     return cudaSuccess;
 }
 cudaError_t cudaFuncSetAttribute(const void* k, cudaFuncAttribute a, int) {

@@ -33,6 +33,7 @@ struct Op {
     Ops before;
     std::vector<Span> spans;
     bool cooperative;
+    bool overlap;      // may start before the operation ahead of it on the stream has ended
 };
 
 struct State {
@@ -66,11 +67,12 @@ inline bool fails(const char* name) {
     return s.fail == name && s.fail_at == n;
 }
 
-inline void enqueue(const char* what, void* st, std::vector<Span> spans, bool cooperative = false) {
+inline void enqueue(const char* what, void* st, std::vector<Span> spans, bool cooperative = false,
+                    bool overlap = false) {
     State& s = state();
     std::lock_guard<std::recursive_mutex> lock(s.mu);
     if (s.ops.size() >= MAX_OPS) abort();
-    Op op{what, st, std::this_thread::get_id(), s.stream[st] | s.host, spans, cooperative};
+    Op op{what, st, std::this_thread::get_id(), s.stream[st] | s.host, spans, cooperative, overlap};
     s.stream[st] = op.before;
     s.stream[st].set(s.ops.size());
     s.ops.push_back(op);

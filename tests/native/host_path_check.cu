@@ -259,6 +259,31 @@ static void tuner_file() {
     remove(path);
 }
 
+// A call without a plan waits once, for its results; its tables arrive in the
+// stream's order, ahead of its first launch, which does not overlap them.
+static void one_shot_calls() {
+    Job_* j = make(3, SMALL);
+    for (int dependent : {0, 1}) {
+        if (dependent) j->descs[1].sendbufs = j->descs[0].recvbufs;
+        for (auto call : {gpumpi_coll_plain, gpumpi_coll_batched}) {
+            cudaStream_t st = stream();
+            const size_t from = fake::state().ops.size();
+            const int waits = fake::state().calls["cudaStreamSynchronize"];
+            CHECK(call(j->descs.data(), 3, 64, st) == 0, "%s", gpumpi_last_error());
+            CHECK(fake::state().calls["cudaStreamSynchronize"] == waits + 1, "%d waits",
+                  fake::state().calls["cudaStreamSynchronize"] - waits);
+            bool first = true;
+            for (size_t i = from; i < fake::state().ops.size(); i++) {
+                const fake::Op& op = fake::state().ops[i];
+                if (op.what != "launch") continue;
+                CHECK(op.stream == st && op.before[from] && op.overlap == !first, "launch %zu", i - from);
+                first = false;
+            }
+            CHECK(!first && fake::races(from) == 0, "dependent %d", dependent);
+        }
+    }
+}
+
 // A call that fails half way reports it, and nothing that it put on other streams outlives a wait for the caller's.
 static void errors() {
     int failed = 0;
@@ -423,7 +448,8 @@ static void failed_plans() {
 int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
         {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns},
-        {"first_calls", first_calls}, {"captured", captured}, {"tuner_file", tuner_file}, {"errors", errors},
+        {"first_calls", first_calls}, {"captured", captured}, {"tuner_file", tuner_file},
+        {"one_shot_calls", one_shot_calls}, {"errors", errors},
         {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans},
         {"devices", devices}, {"failed_plans", failed_plans}};
     fake::state().kernel_spans = kernel_spans;

@@ -39,8 +39,9 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["tables", "uploaded", "retry", "order", "turns", "first_calls", "captured", "tuner_file",
-                                      "errors", "levels", "random_levels", "long_plans", "devices", "failed_plans"])
+@pytest.mark.parametrize("scenario", ["tables", "uploaded", "retry", "order", "turns", "first_calls", "captured",
+                                      "tuner_file", "one_shot_calls", "errors", "levels", "random_levels",
+                                      "long_plans", "devices", "failed_plans"])
 def test_host_path(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout[-3000:] + r.stderr
