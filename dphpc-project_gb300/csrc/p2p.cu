@@ -443,8 +443,9 @@ static __device__ __forceinline__ void copy_batch16(uint4* d, const uint4* s, u3
 
 template <bool cg>
 static __device__ __forceinline__ void copy_vec16(uint4* d, const uint4* s, u64 nv) {
-    for (u64 i = 0; i < nv; i += BATCH16)
-        copy_batch16<cg>(d + i, s + i, nv - i < BATCH16 ? (u32)(nv - i) : BATCH16);
+    u64 i = 0;
+    for (; i + BATCH16 <= nv; i += BATCH16) copy_batch16<cg>(d + i, s + i, BATCH16);
+    if (i < nv) copy_batch16<cg>(d + i, s + i, (u32)(nv - i));
 }
 
 static __device__ void leader_copy(void* dst, const void* src, u64 n) {
