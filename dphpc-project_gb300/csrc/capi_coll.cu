@@ -1,10 +1,10 @@
-// Host-driven collectives: communicators whose ranks are thread blocks, and
-// plans that run a list of collective calls either as one kernel launch per
-// call ("plain") or as one persistent cooperative launch in which the blocks
-// of every communicator run their communicator's calls in order ("batched").
-// Both forms execute the same device schedules as the MPI_* calls of
-// converted programs (coll.cu), so their results are identical and their
-// speed differs only by launch structure.
+// Host-driven collectives: communicators and plans that run a list of
+// collective calls with one kernel launch per call ("plain") or with as few as
+// their dependences allow ("batched").  Calls that need no flag rounds run as
+// independent tiles over the whole GPU (spread.cuh); the others as thread
+// blocks, one for each rank, which run the device schedules of the MPI_* calls
+// of converted programs (coll.cu), a batched list in one cooperative launch.
+// Results are the same bits in every form.
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include <string.h>

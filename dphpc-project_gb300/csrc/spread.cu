@@ -54,7 +54,7 @@ static __device__ __noinline__ void fan_tile(const SpreadCall& c, u32 tile) {
     const u32 r1 = min(r0 + c.group, c.ndst);
     const u64 o0 = (u64)piece * c.per;
     const u64 o1 = min(o0 + c.per, c.nu);
-    const char* s = ld_ptr(c.src, q) + c.rs * r0;
+    const char* s = ld_ptr(c.src, q);
     const u64 row = (u64)q * c.nu * sizeof(V);
     for (u64 o = o0 + threadIdx.x; o < o1; o += U * SP_T) {
         V v[U];
@@ -915,7 +915,7 @@ struct Block {
 // in the SMs: with three, blocks went wherever one had just ended, several to
 // one SM (Allreduce of 200 ranks of 50000 FP64 134 us, two launches 78 us).
 // Back to back, an Allreduce of one FP64 value over 16 ranks takes 2.6 us instead
-// of 5.1, ten calls of 64 ranks 135 instead of 153.
+// of 5.1; alone, with a wait after each, 12.8 us either way.
 static __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 static __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -1124,11 +1124,11 @@ static u64 fan_min(bool units16, double total) {
 // first loads) than it takes to keep loads under way.  Three tiles for each
 // block that fits, as in a level of many calls, leave a tail and are short.
 // Measured with 152, 304, 608 and 1216 tiles for each kind, 4..200 ranks, 0.1 to
-// 200 MB, three tiles -> here, us: Allreduce of 64 ranks of 15616 FP64 10.4 -> 6.4,
+// 200 MB, three tiles / these, us: Allreduce of 64 ranks of 15616 FP64 10.4 -> 6.4,
 // of 124992 float32 16.6 -> 12.4; of 200 of 4992 FP64 32 -> 12.5; Reduce of 16 of
 // 124992 float32 6.3 -> 3.6; Alltoall of 4 of 1 MB blocks 24.3 -> 8.6, of 64 of
 // 7.8 KB 14.2 -> 8.6; Bcast of 32 MB to 64 ranks 10.5 -> 7.1.  The same for 200 MB
-// (Alltoall 50 -> 36) but not much beyond: large calls want tiles of 2 MB.
+// (Alltoall 50 -> 36) but not much beyond.
 constexpr double SP_LONE_BYTES = 2.5e8;
 constexpr u32 SP_SMS = 152;
 
@@ -1368,7 +1368,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         // A warp's addition takes the same time however many lanes add: fill it as
         // far as that leaves two tiles for each block (the 16-communicator batch at
         // 301 per rank 20.7 -> 18.2 us, at 1024 28.7 -> 23.4 us)
-        const double fill = std::min(32.0, std::ceil(level.folded / (152 * SP_BLOCKS_PER_SM * 2)));
+        const double fill = std::min(32.0, std::ceil(level.folded / (SP_SMS * SP_BLOCKS_PER_SM * 2)));
         const double per = std::min(fits, std::max(target / 2 / ((double)P * esize), fill));
         const u64 m = std::max(step, (u64)std::min(per, (double)n) / step * step);
         gather_all(m);
@@ -1493,7 +1493,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
         u64 per = c.ub == 16 && target < 262144.0 ? 4 * SP_T : 8 * SP_T;
         const double sets = std::min(8.0, std::max(4.0, stored / ((double)per * c.ub)));
         c.group = (u32)std::min((double)c.ndst, sets);
-        while (per > 2 * SP_T && (double)c.nu * c.nsrc * c.ndst < 152.0 * per * c.group) per /= 2;
+        while (per > 2 * SP_T && (double)c.nu * c.nsrc * c.ndst < (double)SP_SMS * per * c.group) per /= 2;
         const u64 pieces = (c.nu + per - 1) / per;
         per = ((c.nu + pieces - 1) / pieces + SP_T - 1) / SP_T * SP_T;
         c.per = (u32)per;
@@ -1512,7 +1512,7 @@ void SpreadBuilder::add(const gpumpi_coll_desc& d, int P, int esize, const Sprea
     calls.push_back(c);
 }
 
-// Bytes that a tile moves, for a fold weighted by the length of its chain.
+// Bytes that a tile moves.
 static double tile_cost(const SpreadCall& c) {
     switch (c.kind) {
         case SP_FAN: return (double)c.per * c.ub * (1 + c.group);

@@ -10,11 +10,11 @@
 // may do any piece of any call.  The results are those of the rank form, bit
 // for bit: copies are copies, and a fold takes its inputs in rank order.
 //
-// Measured (rank form -> spread form, one launch): Allreduce of 8 ranks of 16
-// MiB 2515 -> 52 us; the 16-communicator batch of Bcast, Allreduce and Alltoall
-// at 1 element per rank 81 -> 16 us, at 301 326 -> 27 us, at 2^15 477 -> 379
-// us, at 100003 (rank buffers aligned to their elements only) 1909 -> 1202 us,
-// at 2^20 11.55 -> 10.29 ms.
+// Measured (rank form -> spread form, one launch, back to back): Allreduce of 8
+// ranks of 16 MiB 2515 -> 46 us; the 16-communicator batch of Bcast, Allreduce and
+// Alltoall at 1 element per rank 81 -> 13.3 us (with a wait after each 86 -> 22), at
+// 301 326 -> 17.3 us, at 2^15 477 -> 319 us, at 100003 (rank buffers aligned to their
+// elements only) 1909 -> 1047 us, at 2^20 11.55 -> 9.81 ms.
 #pragma once
 
 #include <stdint.h>
@@ -43,14 +43,13 @@ __host__ __device__ constexpr u32 rows_part(u32 nsrc) {
 }
 __host__ __device__ constexpr u32 passes_half(u32 nsrc) { return fold_table(nsrc) / 32 * 16; }
 constexpr int SP_MAX_STAGES = 8;
-constexpr int SP_BLOCKS_PER_SM = 4;     // 208 KiB of shared memory, 64 registers a thread
+constexpr int SP_BLOCKS_PER_SM = 4;     // 216 KiB of dynamic shared memory, 64 registers a thread
 
 // What the tiles of one SpreadCall do.  Units of a copy are `ub` bytes.
 enum SpreadKind : int {
     // Blocks of `nu` units: block q of every destination row comes from source
     // q.  A tile is `per` units of one block for `group` rows: loaded once,
-    // stored to each (Bcast: one source; Allgather; Alltoall with group = 1,
-    // whose source block lies `rs` bytes further for each row).
+    // stored to each (Bcast: one source; Allgather).
     SP_FAN = 0,
     // The same blocks when they are short: a tile is `per` units of the
     // sequence of all rows, each loaded and stored by one thread; with `group` 1,
@@ -60,7 +59,7 @@ enum SpreadKind : int {
     // destination.  A tile is `per` elements: the block loads them from all
     // sources into shared memory at once, then thread i folds element i.
     SP_GATHER = 2,
-    // The same fold for long vectors: a tile is `per` rows of one `ub`-byte
+    // The same fold for long vectors: a tile is `per` rows of one 16-byte
     // vector per thread, every thread streams its own vectors of one source
     // after another through its part of a ring in shared memory.
     SP_STREAM = 3,
@@ -70,8 +69,8 @@ enum SpreadKind : int {
     // 16-byte units they touch, `stages` rows ahead, and stores them from the
     // ring, shifted to each destination's alignment.  `nu` is in bytes.
     SP_MOVE = 4,
-    // The fold again, of buffers aligned to their elements only or in finer
-    // pieces.  Each warp folds chunks of `per` elements, a tile is `rows`
+    // The fold again, of buffers aligned to their elements only, of very many
+    // ranks or in finer pieces.  Each warp folds chunks of `per` elements, a tile is `rows`
     // chunks; `batch` sources are loaded at a time, `ub` bytes apart.  With `group`
     // 1 a tile is one chunk, folded by the whole block in passes over the sources.
     SP_ROWS = 5,
@@ -81,7 +80,7 @@ struct alignas(16) SpreadCall {
     const char* const* src;     // [nsrc]
     char* const* dst;           // [ndst]
     u64 nu;
-    u64 rs;                     // SP_GATHER: bytes between the starts of two tiles
+    u64 rs;                     // SP_GATHER: bytes between the starts of two tiles; Alltoall: between a source's blocks
     u64 off;                    // folds: bytes added to every address
     u32 first_tile, ntiles;
     int kind;

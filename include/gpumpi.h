@@ -12,10 +12,10 @@
  *
  *  2. Host-driven collectives on device buffers, one call per collective
  *     ("plain": one kernel launch per call) or many communicators and calls
- *     in one persistent launch ("batched"), optionally captured as a CUDA
- *     graph.  These have no counterpart in the reference, which only offered
- *     the device-side MPI_* calls; they expose the same device schedules
- *     (mpi.cu:77-408 in the reference) to host code.
+ *     in as few launches as their dependences allow ("batched"), optionally
+ *     captured as a CUDA graph.  These have no counterpart in the reference,
+ *     which only offered the device-side MPI_* calls (mpi.cu:77-408 there);
+ *     the results are those of the same calls in device code.
  *
  * All pointers are plain device or host addresses; streams are cudaStream_t
  * passed as void*.  Every function returns 0 on success or a nonzero
