@@ -171,6 +171,7 @@ struct HostPipe {
     enum State { NEW, READY, NONE } state = NEW;   // NONE: no two groups, or calls that share device memory
     std::vector<std::vector<int>> groups;  // calls (creation order) of each group
     std::vector<SpreadArgs> tiles;
+    std::vector<char> image;               // of the tile lists, which a copy from it may still read
     cudaStream_t in = nullptr, out = nullptr;
     cudaEvent_t begin = nullptr, end = nullptr;
     std::vector<cudaEvent_t> arrived, ran;
@@ -185,6 +186,7 @@ struct HostPipe {
         ran.clear();
         groups.clear();
         tiles.clear();
+        image.clear();
         begin = end = nullptr;
         in = out = nullptr;
     }
@@ -198,6 +200,7 @@ struct gpumpi_plan_s {
     int threads;
     size_t smem;
     char* base = nullptr;             // device allocation
+    std::vector<char> image;          // what a stream's copy to it may still read
     PlanArgs batch_args;              // batched launch
     std::vector<PlanArgs> plain_args; // one per descriptor
     std::vector<int> plain_grid;
@@ -745,7 +748,8 @@ static int create_plan(const gpumpi_coll_desc* descs, int ndesc, int threads, in
         at += spread[k].bytes();
     }
     if (upload) {
-        CK(cudaMemcpyAsync(base, h.data(), total, cudaMemcpyHostToDevice, *upload));   // staged on return
+        p->image = std::move(h);
+        CK(cudaMemcpyAsync(base, p->image.data(), total, cudaMemcpyHostToDevice, *upload));
     } else {
         CK(cudaMemcpy(base, h.data(), total, cudaMemcpyHostToDevice));
         // a copy from pageable memory may return before it has arrived, and launches on
@@ -1078,11 +1082,11 @@ int make_pipe(gpumpi_plan_t p, HostPipe& pipe) {
         pipe.state = HostPipe::NONE;
         return GPUMPI_OK;
     }
-    std::vector<char> image(bytes);
+    pipe.image.resize(bytes);
     pipe.tiles.resize(tiles.size());
     size_t at = 0;
     for (size_t g = 0; g < tiles.size(); g++) {
-        tiles[g].image(image.data() + at, p->pipe_base + at, &pipe.tiles[g]);
+        tiles[g].image(pipe.image.data() + at, p->pipe_base + at, &pipe.tiles[g]);
         pipe.tiles[g].job = g_api.djob;
         at += (tiles[g].bytes() + 63) & ~(size_t)63;
     }
@@ -1098,9 +1102,8 @@ int make_pipe(gpumpi_plan_t p, HostPipe& pipe) {
         pipe.ran.push_back(e);
     }
     // Ahead of every group's inputs on the stream that brings them, so a launch on
-    // any stream that waits for its inputs waits for its tiles too.  Returns once
-    // the pageable image has been staged.
-    CK(cudaMemcpyAsync(p->pipe_base, image.data(), bytes, cudaMemcpyHostToDevice, pipe.in));
+    // any stream that waits for its inputs waits for its tiles too.
+    CK(cudaMemcpyAsync(p->pipe_base, pipe.image.data(), bytes, cudaMemcpyHostToDevice, pipe.in));
     pipe.state = HostPipe::READY;
     return GPUMPI_OK;
 }

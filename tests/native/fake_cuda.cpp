@@ -56,6 +56,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t st) {
 cudaError_t cudaStreamSynchronize(cudaStream_t st) {
     FAKE_CALL("cudaStreamSynchronize");
     s.host |= s.stream[st == cudaStreamLegacy ? nullptr : st];
+    fake::waited();
     return cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t st, cudaEvent_t e, unsigned) {

@@ -51,6 +51,10 @@ struct State {
     std::string fail;                      // this function ...
     int fail_at = -1;                      // ... fails at this call (counted from 0; -1: never)
     int pause_us = 0;                      // length of a copy call and of a look-up of a driver function
+    // pageable sources of copies that nobody has waited for, and what was in them:
+    // where the device reads such memory itself, a copy may do so until then
+    std::vector<std::pair<const char*, std::string>> unread;
+    int gone = 0;                          // of them, those that were no longer the same when waited for
     // bytes that a kernel launch touches
     std::vector<Span> (*kernel_spans)(const void* kernel, void** args) = nullptr;
 };
@@ -96,6 +100,12 @@ inline int races(size_t from, bool (*counts)(const Span&) = nullptr) {
     return n;
 }
 
+// The host waits for what was enqueued.
+inline void waited() {
+    for (auto& r : state().unread) state().gone += memcmp(r.first, r.second.data(), r.second.size()) != 0;
+    state().unread.clear();
+}
+
 inline bool is_device(const void* p) {
     State& s = state();
     auto it = s.device.upper_bound((char*)p);
@@ -112,6 +122,7 @@ inline void copy(const char* what, void* dst, const void* src, size_t n, void* s
     bool pinned = is_device(src);
     for (auto& r : s.pinned) pinned = pinned || ((const char*)src >= r.first && (const char*)src < r.first + r.second);
     if (pinned) v.push_back({(const char*)src, n, false});
+    else s.unread.push_back({(const char*)src, std::string((const char*)src, n)});
     enqueue(what, st, v);
 }
 

@@ -284,6 +284,22 @@ static void one_shot_calls() {
     }
 }
 
+// What copies to the device read from pageable memory stays as it is until the
+// stream has been waited for.
+static void images() {
+    Job_* j = make(3, LARGE);
+    cudaStream_t st = stream();
+    fake::state().unread.clear();   // the communicator's and the plan's, waited for by what came after
+    fake::state().gone = 0;
+    CHECK(run_host(j, st) == 0, "%s", gpumpi_last_error());
+    CHECK(fake::state().unread.size() == 1, "%zu pageable copies", fake::state().unread.size());   // the tile lists
+    cudaStreamSynchronize(st);
+    CHECK(fake::state().gone == 0, "a group's tile lists");
+    fake::state().gone = 0;
+    CHECK(gpumpi_coll_batched(j->descs.data(), 3, 64, st) == 0, "%s", gpumpi_last_error());
+    CHECK(fake::state().gone == 0 && fake::state().unread.empty(), "a call's tables");
+}
+
 // A call that fails half way reports it, and nothing that it put on other streams outlives a wait for the caller's.
 static void errors() {
     int failed = 0;
@@ -449,7 +465,7 @@ int main(int argc, char** argv) {
     const std::map<std::string, std::function<void()>> scenarios = {
         {"tables", tables}, {"uploaded", uploaded}, {"retry", retry}, {"order", order}, {"turns", turns},
         {"first_calls", first_calls}, {"captured", captured}, {"tuner_file", tuner_file},
-        {"one_shot_calls", one_shot_calls}, {"errors", errors},
+        {"one_shot_calls", one_shot_calls}, {"images", images}, {"errors", errors},
         {"levels", levels}, {"random_levels", random_levels}, {"long_plans", long_plans},
         {"devices", devices}, {"failed_plans", failed_plans}};
     fake::state().kernel_spans = kernel_spans;

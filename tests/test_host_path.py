@@ -40,7 +40,7 @@ def check(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["tables", "uploaded", "retry", "order", "turns", "first_calls", "captured",
-                                      "tuner_file", "one_shot_calls", "errors", "levels", "random_levels",
+                                      "tuner_file", "one_shot_calls", "images", "errors", "levels", "random_levels",
                                       "long_plans", "devices", "failed_plans"])
 def test_host_path(check, scenario):
     r = subprocess.run([check, scenario], capture_output=True, text=True, timeout=120)
